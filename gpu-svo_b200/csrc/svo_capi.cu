@@ -177,7 +177,7 @@ struct MeshHost {
     const int32_t *d_tris = nullptr;
     bool tris_on_device = false;
     Pyramid py;
-    uint64_t bits_off = 0, cnt_off = 0;  // into the batch's bitmap / count buffers
+    uint64_t bits_off = 0, pre_off = 0, base_off = 0;  // into the batch's bitmap / rank buffers
     uint32_t cta0 = 0;                   // first pyramid CTA (level-0 region) in the batch
     int status = SVO_OK;
     std::string error;
@@ -233,12 +233,11 @@ struct svo_batch {
     std::vector<int> live;                  // meshes with device work
     std::vector<void *> allocs;             // phase A buffers (pool)
     uint64_t *bits = nullptr;
-    uint32_t *cnt = nullptr, *pre = nullptr;
+    uint32_t *pre = nullptr, *base = nullptr;  // block ranks, region prefixes (RankDev)
     uint8_t *rflag = nullptr;               // level-0 regions that triangles reach (one byte per pyramid CTA)
     unsigned char *meta = nullptr;
     MeshDev *d_mesh = nullptr;
     std::vector<MeshDev> h_mesh;
-    uint64_t total_blocks = 0;
     float timings_a[5] = {};                // total, bbox, voxelize, pyramid, scan
     bool timed = false;
 };
@@ -357,46 +356,46 @@ int batch_phase_a(svo_batch *b) {
     b->meta = batch_alloc<unsigned char>(b, ml.bytes, err);
     if (!b->meta) return cuda_fail(err, "alloc meta");
     // ---- layout ----
-    uint64_t words = 0, blocks = 0, tris = 0;
-    uint32_t ctas = 0, bblocks = 0;
+    uint64_t words = 0, blocks = 0, bases = 0, tris = 0;
+    uint32_t ctas = 0, max_ctas = 0, bblocks = 0;
     std::vector<uint64_t> tri_off(n + 1);
     std::vector<uint32_t> cta_off(n + 1), bbox_off(n + 1);
     for (int k = 0; k < n; ++k) {
         MeshHost &mh = b->m[b->live[k]];
         mh.py = make_pyramid(mh.res[0], mh.res[1], mh.res[2]);
         mh.bits_off = words;
-        mh.cnt_off = blocks;
+        mh.pre_off = blocks;
+        mh.base_off = bases;
         words += (mh.py.total_words + 31) / 32 * 32;
         blocks += mh.py.total_blocks;
+        bases += 4 * (uint64_t)((mh.py.ctas + 3) & ~3u);
         tri_off[k] = tris;
         cta_off[k] = ctas;
         mh.cta0 = ctas;
         bbox_off[k] = bblocks;
         tris += (uint64_t)mh.n_tris;
         ctas += mh.py.ctas;
+        max_ctas = std::max(max_ctas, mh.py.ctas);
         bblocks += bbox_blocks(mh.n_pts);
     }
     tri_off[n] = tris;
     cta_off[n] = ctas;
     bbox_off[n] = bblocks;
-    b->total_blocks = blocks;
     // the batch's scratch arrays and its mesh tables: one block, one upload
     uint32_t big_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(2 * tris, 1 << 16), 0x7FFFFFFFu);
     HostPack tables;  // mesh table, triangle / CTA / bbox-block offsets (filled below)
     auto a16 = [](size_t x) { return (x + 15) / 16 * 16; };
     const size_t t_bytes = a16(sizeof(MeshDev) * n) + a16(8 * (size_t)(n + 1)) + a16(4 * (size_t)(n + 1)) + 4 * (size_t)(n + 1);
     Layout lay;
-    const size_t o_bits = lay.add<uint64_t>(words), o_cnt = lay.add<uint32_t>(blocks),
-                 o_pre = lay.add<uint32_t>(blocks + 1), o_scan = lay.add<unsigned long long>(scan_scratch_words(blocks)),
+    const size_t o_bits = lay.add<uint64_t>(words), o_pre = lay.add<uint32_t>(blocks), o_base = lay.add<uint32_t>(bases),
                  o_big = lay.add<uint4>(big_cap), o_small = lay.add<uint64_t>(std::max<uint64_t>(tris, 1)),
                  o_rflag = lay.add<uint8_t>(std::max<uint32_t>(ctas, 1));
     const size_t o_tables = lay.add<unsigned char>(t_bytes);
     unsigned char *blk = batch_alloc<unsigned char>(b, lay.bytes, err);
     if (err != cudaSuccess || !blk) return cuda_fail(err, "batch scratch");
     b->bits = reinterpret_cast<uint64_t *>(blk + o_bits);
-    b->cnt = reinterpret_cast<uint32_t *>(blk + o_cnt);
     b->pre = reinterpret_cast<uint32_t *>(blk + o_pre);
-    unsigned long long *scan = reinterpret_cast<unsigned long long *>(blk + o_scan);
+    b->base = reinterpret_cast<uint32_t *>(blk + o_base);
     uint4 *big = reinterpret_cast<uint4 *>(blk + o_big);
     uint64_t *small = reinterpret_cast<uint64_t *>(blk + o_small);
     uint8_t *rflag = b->rflag = blk + o_rflag;
@@ -417,8 +416,9 @@ int batch_phase_a(svo_batch *b) {
         d.gp = gp + k;
         d.mm = mm + 8 * k;
         d.bits = b->bits + mh.bits_off;
-        d.cnt = b->cnt + mh.cnt_off;
-        d.pre = b->pre + mh.cnt_off;
+        d.pre = b->pre + mh.pre_off;
+        d.base = b->base + mh.base_off;
+        d.bstride = (mh.py.ctas + 3) & ~3u;
         d.totals = totals + kMaxLevels * k;
         d.done = done + k;
         d.py = mh.py;
@@ -443,22 +443,18 @@ int batch_phase_a(svo_batch *b) {
         SVO_TRY(launch_bbox(bd, bblocks, st), "bbox");
         tm.mark(StageTimer::kBbox, st);
         SVO_TRY(cudaMemsetAsync(rflag, 0, std::max<uint32_t>(ctas, 1), st), "memset regions");
-        SVO_TRY(cudaMemsetAsync(b->cnt, 0, blocks * 4, st), "memset counts");
         SVO_TRY(launch_regions(bd, (int64_t)tris, ctas, ctx->num_sms, st), "zero bitmaps");
         SVO_TRY(launch_voxelize(bd, (int64_t)tris, strict, b->tune, big, big_cap, counters, ctx->num_sms, st,
                                 small),
                 "voxelize");
         tm.mark(StageTimer::kVox, st);
-        SVO_TRY(launch_pyramid(bd, ctas, ctx->num_sms, st), "pyramid");
+        SVO_TRY(launch_pyramid(bd, ctas, max_ctas, ctx->num_sms, st), "pyramid");
         tm.mark(StageTimer::kPyr, st);
-        SVO_TRY(launch_scan(b->cnt, b->pre, blocks, scan, counters + 2, st), "scan");
-        SVO_TRY(launch_level_totals(bd, st), "totals");
         tm.mark(StageTimer::kScan, st);
         std::vector<unsigned char> h(ml.imm);
         SVO_TRY(cudaMemcpyAsync(h.data(), b->meta, ml.imm, cudaMemcpyDeviceToHost, st), "read meta");
         SVO_TRY(cudaStreamSynchronize(st), "count phase");
         const uint32_t *hc = reinterpret_cast<const uint32_t *>(h.data() + ml.counters);
-        if (hc[2] & kStatusScanTimeout) return fail(SVO_ERR_DEVICE_TIMEOUT, "scan look-back timed out");
         if (hc[0] > big_cap) {  // more big-triangle entries than the queue holds: grow it, redo
             big_cap = hc[0];
             big = batch_alloc<uint4>(b, big_cap, err);
@@ -771,7 +767,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 // compaction jobs: levels 1..T into K, level 0 into the keys
                 CompactJob job{};
                 job.bits = md.bits;
-                job.pre = md.pre;
+                job.rank = RankDev{md.pre, md.base, md.bstride};
                 job.py = mh.py;
                 job.l0 = 1;
                 job.l1 = mh.T + 1;
@@ -794,7 +790,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 word_off.push_back(word_off.back() + mh.py.woff[mh.T] + mh.py.words[mh.T] - mh.py.woff[job.l0]);
                 if (want_keys && mh.T >= 3) {
                     // the level-3 code list is the list of non-empty level-0 blocks
-                    kjobs.push_back(KeyJob{md.bits, md.pre, job.out + job.koff[3], r->keys});
+                    kjobs.push_back(KeyJob{md.bits, job.rank, job.out + job.koff[3], r->keys});
                     blk_off.push_back(blk_off.back() + mh.totals[3]);
                 } else if (want_keys) {
                     CompactJob k0 = job;
@@ -819,12 +815,10 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                     P.lv[l].K1 = job.out + (l < mh.T ? job.koff[l + 1] : job.koff[mh.T]);
                     P.lv[l].bits = md.bits + mh.py.woff[l];
                     P.lv[l].wpre = l >= 1 ? job.wpre + (mh.py.woff[l] - mh.py.woff[1]) : nullptr;
-                    P.lv[l].coff = mh.py.coff[l];
                     P.lv[l].side = std::max<uint32_t>(1u, R >> l);
                     P.lv[l].width = w;
                     w = w * 2.0f;
                 }
-                P.pre = md.pre;
                 P.gp = md.gp;
                 P.nodes = r->nodes;
                 P.verts = ve ? r->verts : nullptr;

@@ -26,20 +26,29 @@ struct VoxTuning {
 
 // Occupancy bitmap pyramid: level 0 is the voxel grid (one bit per Morton
 // code), level l+1 bit j = OR of level-l bits 8j..8j+7.  Every level is stored
-// as u64 words padded to whole 512-bit blocks; cnt holds one popcount per
-// 512-bit block of every level, pre its exclusive prefix sum.
+// as u64 words padded to whole 512-bit blocks, ranked by RankDev.
 struct Pyramid {
     int levels = 0;                      // stored levels (>= 5)
     int grid_levels = 0;                 // log2(R) + 1 levels of the real grid
     uint64_t woff[kMaxLevels] = {};      // u64 word offset of level l
     uint64_t words[kMaxLevels] = {};     // u64 words of level l
-    uint64_t coff[kMaxLevels + 1] = {};  // block-count offset of level l
+    uint64_t coff[kMaxLevels + 1] = {};  // 512-bit block offset of level l
     uint64_t total_words = 0;
     uint64_t total_blocks = 0;
     uint32_t ctas = 0;                   // pyramid CTAs (level-0 chunks of 2048 words)
 };
 
 Pyramid make_pyramid(int rx, int ry, int rz);
+
+// Ranks of a mesh's 512-bit blocks.  Levels 0..2: the set bits before the
+// block in its level-0 region (pre, at coff[l]) on top of the region's prefix
+// (base, level l at l * bstride); level 3, half a block per region: the
+// region's prefix; levels 4..: pre alone.
+struct RankDev {
+    const uint32_t *pre;
+    const uint32_t *base;
+    uint32_t bstride;  // regions of the mesh rounded up to 4
+};
 
 // One mesh of a batch, as the kernels see it (an array in device memory).
 // A single build is a batch of one.
@@ -53,10 +62,11 @@ struct MeshDev {
     GridParams *gp;
     uint32_t *mm;            // bbox scratch (6 u32)
     uint64_t *bits;          // this mesh's pyramid (level l at bits + py.woff[l])
-    uint32_t *cnt;           // this mesh's block counts (level l at cnt + py.coff[l])
-    uint32_t *pre;           // exclusive prefix at this mesh's first block
+    uint32_t *pre;           // block ranks (RankDev)
+    uint32_t *base;          // region sums, then their prefixes (RankDev)
+    uint32_t bstride;
     uint32_t *totals;        // set bits per level (kMaxLevels)
-    uint32_t *done;          // pyramid CTAs finished
+    uint32_t *done;          // pyramid regions finished
     Pyramid py;
 };
 
@@ -81,7 +91,6 @@ struct EmitLevel {
     const uint64_t *K1;    // sorted codes of level l+1 (the level's groups); level T: its own code
     const uint64_t *bits;  // bitmap of level l
     const uint32_t *wpre;  // rank at each non-empty word of level l (l >= 1)
-    uint64_t coff;         // block-count offset of level l
     uint32_t side;         // grid side at this level (R >> l)
     float width;           // node width
 };
@@ -92,7 +101,6 @@ struct EmitParams {
     uint32_t N;             // total nodes
     uint32_t flags;
     EmitLevel lv[kMaxLevels];
-    const uint32_t *pre;    // exclusive prefix of the block counts (this mesh's base)
     const GridParams *gp;
     svo_node *nodes;
     svo_vertex *verts;      // may be null (SVO_FLAG_NO_VERT_EDGE)
@@ -114,7 +122,7 @@ struct EmitBatch {
 // index (word_off, n + 1 entries).
 struct CompactJob {
     const uint64_t *bits;
-    const uint32_t *pre;
+    RankDev rank;
     Pyramid py;
     int l0, l1;
     uint64_t *out;
@@ -131,7 +139,7 @@ struct CompactBatch {
 // (= its level-3 code list).
 struct KeyJob {
     const uint64_t *bits;    // level-0 bitmap
-    const uint32_t *pre;     // the mesh's scanned block counts (level 0 first)
+    RankDev rank;
     const uint64_t *blocks;  // sorted non-empty block indices
     uint64_t *out;
 };
@@ -171,8 +179,9 @@ cudaError_t launch_index_ranges(const IndexJob *jobs, int n, const uint32_t *blo
 cudaError_t launch_voxelize(const BatchDev &b, int64_t total_tris, bool strict, const VoxTuning &tune,
                             uint4 *big, uint32_t big_cap, uint32_t *counters, int num_sms, cudaStream_t st,
                             uint64_t *small = nullptr);
-// Builds levels 1.. of every mesh's pyramid and the per-block counts.
-cudaError_t launch_pyramid(const BatchDev &b, uint32_t total_ctas, int num_sms, cudaStream_t st);
+// Builds levels 1.. of every mesh's pyramid, the block ranks and the level
+// totals; max_ctas: the most regions of any mesh (py.ctas).  done must be zero.
+cudaError_t launch_pyramid(const BatchDev &b, uint32_t total_ctas, uint32_t max_ctas, int num_sms, cudaStream_t st);
 // Flags the level-0 regions that triangles of region-mode meshes reach, then
 // zeroes level 0 where needed (every region of other meshes, the flagged ones
 // of region-mode meshes) and each mesh's levels >= 3.  Replaces a memset of
@@ -196,8 +205,6 @@ cudaError_t launch_scan_stalled(const uint32_t *in, uint32_t *out, uint64_t n, u
 // Stream-ordered allocation from one of a context's pools: the one place a
 // build allocates device memory (svo_debug_fail_alloc injects failures here).
 cudaError_t pool_malloc(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t st);
-// totals of every (mesh, level).
-cudaError_t launch_level_totals(const BatchDev &b, cudaStream_t st);
 cudaError_t launch_compact(const CompactBatch &c, uint64_t total_words, cudaStream_t st);
 cudaError_t launch_compact_keys(const KeyBatch &k, uint64_t total_blocks, cudaStream_t st);
 // Levels 1 and 2 of a region-mode job (job.rflag set), one block per level-0 region.

@@ -131,9 +131,9 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
     CompactJob *d_job = c.take<CompactJob>(1);
     uint64_t *d_word_off = c.take<uint64_t>(2);
     uint64_t *bits = c.take<uint64_t>(py.total_words);
-    uint32_t *cnt = c.take<uint32_t>(py.total_blocks);
-    uint32_t *pre = c.take<uint32_t>(py.total_blocks + 1);
-    unsigned long long *scan = c.take<unsigned long long>(scan_scratch_words(py.total_blocks));
+    uint32_t *pre = c.take<uint32_t>(py.total_blocks);
+    const uint32_t bstride = (py.ctas + 3) & ~3u;
+    uint32_t *region_base = c.take<uint32_t>(4 * (size_t)bstride);
     if (c.used > kNoAllocScratchBytes) return noalloc_fail(SVO_ERR_UNSUPPORTED, "scratch layout exceeds 3 MiB");
 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -158,8 +158,9 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
     md.gp = gp;
     md.mm = mm;
     md.bits = bits;
-    md.cnt = cnt;
     md.pre = pre;
+    md.base = region_base;
+    md.bstride = bstride;
     md.totals = totals;
     md.done = done;
     md.py = py;
@@ -181,20 +182,17 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
     if ((rc = cuda(launch_voxelize(bd, nt, (flags & SVO_FLAG_STRICT_FP) != 0, tune, nullptr, 0, counters,
                                    num_sms, st))))
         return rc;
-    if ((rc = cuda(launch_pyramid(bd, py.ctas, num_sms, st)))) return rc;
-    if ((rc = cuda(launch_scan(cnt, pre, py.total_blocks, scan, &gp->status, st)))) return rc;
-    if ((rc = cuda(launch_level_totals(bd, st)))) return rc;
+    if ((rc = cuda(launch_pyramid(bd, py.ctas, py.ctas, num_sms, st)))) return rc;
     uint32_t h_tot = 0, h_status = 0;
     if ((rc = cuda(cudaMemcpyAsync(&h_tot, totals, 4, cudaMemcpyDeviceToHost, st)))) return rc;
     if ((rc = cuda(cudaMemcpyAsync(&h_status, &gp->status, 4, cudaMemcpyDeviceToHost, st)))) return rc;
     if ((rc = cuda(cudaStreamSynchronize(st)))) return rc;
     if (h_status & kStatusNonFinite) return noalloc_fail(SVO_ERR_INVALID_ARGUMENT, "non-finite vertex coordinate");
-    if (h_status & kStatusScanTimeout) return noalloc_fail(SVO_ERR_DEVICE_TIMEOUT, "scan look-back timed out");
     *n_keys = h_tot;
     if ((int64_t)h_tot > keys_cap) return noalloc_fail(SVO_ERR_INVALID_ARGUMENT, "keys buffer too small (see *n_keys)");
     CompactJob job{};
     job.bits = bits;
-    job.pre = pre;
+    job.rank = RankDev{pre, region_base, bstride};
     job.py = py;
     job.l0 = 0;
     job.l1 = 1;

@@ -6,8 +6,9 @@
 // children.  Here every level comes out of one occupancy-bitmap pyramid:
 //   * level l+1 bit j is the OR of level-l bits 8j..8j+7 (a byte test), so
 //     one streaming pass builds all levels (k_pyramid);
-//   * one popcount per 512-bit block and a single exclusive scan give O(1)
-//     rank queries on every level (k_scan);
+//   * the same pass leaves each 512-bit block's rank within its 2048-word
+//     region and each region's sums, whose scan gives O(1) rank queries on
+//     every level;
 //   * the node at local index 8g+k of level l has code 8*K[l+1][g] + k, where
 //     K[l+1] is the sorted list of set bits of level l+1 (k_compact); its
 //     children start at 8*rank_l(code) in level l-1, its parent sits at
@@ -65,32 +66,185 @@ __device__ __forceinline__ uint32_t nz_bytes(uint64_t v) {
     return (uint32_t)((m * 0x0102040810204080ull) >> 56);
 }
 
+// Exclusive prefix of v over the NT threads of the block, and the block's sum.
+// All threads call; s_warp holds NT / 32 words.
+template <int NT>
+__device__ __forceinline__ uint32_t block_exscan(uint32_t v, uint32_t *s_warp, uint32_t &total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= d) incl += o;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    const uint32_t w = lane < NT / 32 ? s_warp[lane] : 0u;
+    total = __reduce_add_sync(0xFFFFFFFFu, w);
+    const uint32_t before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? w : 0u);
+    __syncthreads();  // s_warp may be rewritten
+    return before + incl - v;
+}
+
+// The region sums of one of levels 0..3 (base + level * bstride) become their
+// exclusive prefixes in place; the sum goes to totals[level].  Padding past
+// the mesh's regions (up to the 16-byte stride) is treated as zero.
+template <int NT, int ITEMS>
+__device__ __forceinline__ void scan_regions(const MeshDev &md, int level, uint32_t *s_warp) {
+    uint32_t *a = md.base + (uint64_t)level * md.bstride;
+    const uint32_t n = md.py.ctas;
+    uint32_t carry = 0;
+    for (uint32_t i0 = 0; i0 < n; i0 += NT * ITEMS) {
+        const uint32_t i = i0 + threadIdx.x * ITEMS;
+        uint32_t v[ITEMS];
+        uint32_t sum = 0;
+#pragma unroll
+        for (int q = 0; q < ITEMS / 4; ++q) {
+            uint4 x = make_uint4(0, 0, 0, 0);
+            if (i + 4 * q < n) x = __ldcg(reinterpret_cast<const uint4 *>(a + i) + q);
+            v[4 * q] = x.x;
+            v[4 * q + 1] = x.y;
+            v[4 * q + 2] = x.z;
+            v[4 * q + 3] = x.w;
+        }
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            if (i + k >= n) v[k] = 0;
+            sum += v[k];
+        }
+        uint32_t tot;
+        uint32_t run = carry + block_exscan<NT>(sum, s_warp, tot);
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const uint32_t x = v[k];
+            v[k] = run;
+            run += x;
+        }
+#pragma unroll
+        for (int q = 0; q < ITEMS / 4; ++q)
+            if (i + 4 * q < n)
+                reinterpret_cast<uint4 *>(a + i)[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        carry += tot;
+    }
+    if (threadIdx.x == 0) md.totals[level] = carry;
+}
+
+// scan_regions of the four levels at once for a mesh of at most 4 NT regions:
+// one round trip for all loads.
+template <int NT>
+__device__ __forceinline__ void scan_regions_all(const MeshDev &md, uint32_t *s_warp) {
+    const uint32_t n = md.py.ctas, i = threadIdx.x * 4;
+    uint4 v[4];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        v[l] = make_uint4(0, 0, 0, 0);
+        if (i < n) v[l] = __ldcg(reinterpret_cast<const uint4 *>(md.base + (uint64_t)l * md.bstride + i));
+        if (i + 1 >= n) v[l].y = 0;  // padding
+        if (i + 2 >= n) v[l].z = 0;
+        if (i + 3 >= n) v[l].w = 0;
+    }
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        uint32_t tot;
+        const uint32_t a = block_exscan<NT>(v[l].x + v[l].y + v[l].z + v[l].w, s_warp, tot);
+        const uint32_t b = a + v[l].x, c = b + v[l].y, d = c + v[l].z;
+        if (i < n) *reinterpret_cast<uint4 *>(md.base + (uint64_t)l * md.bstride + i) = make_uint4(a, b, c, d);
+        if (threadIdx.x == 0) md.totals[l] = tot;
+    }
+}
+
+// Levels 5.. of a mesh from its level 4, with the scanned block counts and the
+// totals of levels 4..  Levels of at most kTopWords words stay in shared
+// memory between the steps, so only the first step waits on global loads.
+constexpr uint32_t kTopWords = 512;
+
+template <int NT>
+__device__ __forceinline__ void finish_top(const MeshDev &md, uint64_t (*s_top)[kTopWords], uint32_t *s_warp) {
+    const Pyramid &py = md.py;
+    bool held = false;  // level l is in s_top[l & 1]
+    for (int l = 4; l < py.levels; ++l) {
+        const uint64_t *in = md.bits + py.woff[l];
+        const uint32_t nblk = (uint32_t)(py.words[l] / 8);
+        const bool has_next = l + 1 < py.levels;
+        uint64_t *out = has_next ? md.bits + py.woff[l + 1] : nullptr;
+        const bool hold = has_next && py.words[l + 1] <= kTopWords;
+        if (hold)
+            for (uint32_t j = nblk + threadIdx.x; j < py.words[l + 1]; j += NT) s_top[(l + 1) & 1][j] = 0;  // padding
+        uint32_t carry = 0;
+        for (uint32_t j0 = 0; j0 < nblk; j0 += NT) {
+            const uint32_t j = j0 + threadIdx.x;
+            uint64_t w = 0;
+            uint32_t c = 0;
+            if (j < nblk) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    ulonglong2 v;
+                    if (held) v = reinterpret_cast<const ulonglong2 *>(s_top[l & 1] + 8 * j)[q];
+                    else v = __ldcg(reinterpret_cast<const ulonglong2 *>(in + 8 * (uint64_t)j) + q);
+                    c += __popcll(v.x) + __popcll(v.y);
+                    w |= (uint64_t)nz_bytes(v.x) << (16 * q);
+                    w |= (uint64_t)nz_bytes(v.y) << (16 * q + 8);
+                }
+            }
+            uint32_t tot;
+            const uint32_t ex = carry + block_exscan<NT>(c, s_warp, tot);
+            if (j < nblk) {
+                md.pre[py.coff[l] + j] = ex;
+                if (has_next) out[j] = w;
+                if (hold) s_top[(l + 1) & 1][j] = w;
+            }
+            carry += tot;
+        }
+        if (threadIdx.x == 0) md.totals[l] = carry;
+        held = hold;
+        __syncthreads();  // level l + 1 is complete (in shared memory, or in global memory for this block)
+    }
+}
+
 // Levels 1..4 of 2048-word chunks of level 0 (regions), a persistent grid
 // taking them in turn (one 512-bit block of level 0 per thread, 16-byte
-// streaming loads); the levels above 4 come from k_pyramid_top.  A
-// region-mode mesh's region that no triangle reaches is empty and is not read
-// (its level-0 words are not zeroed in memory): its words of levels 1..4 are
-// written as zeros and its counts stay at their memset zero.
-__global__ void __launch_bounds__(256, 8) k_pyramid(BatchDev bd, uint32_t total) {
+// streaming loads).  The same pass ranks: every 512-bit block of levels 0..2
+// gets the set bits before it in its region (md.pre), and every region its
+// set bits of levels 0..3 (md.base), whose prefix over the regions completes
+// the rank -- there is no scan over the blocks (19.2M of them at res 2048:
+// that scan and the memset before it took 60 us, this scan of 4 x 65,536
+// region sums takes 7).  A region-mode mesh's region that no triangle reaches
+// is empty and is not read (its level-0 words are not zeroed in memory): its
+// words of levels 1..4 and its sums are written as zeros.
+//
+// FUSE: the CTA that finishes a mesh's last region scans the sums and builds
+// the levels above 4 as well, which saves a launch (about 5 us of the 213 us
+// of a 20k-triangle build at res 128).  One CTA of 256 threads takes 4 region
+// sums per thread and level in one step up to kFuseRegions; meshes with more
+// regions (res 1024 and up) are finished by k_pyramid_finish, whose five
+// 1024-thread CTAs per mesh work side by side, and so are batches with more
+// than 8 regions per SM, where the fused variant's 56 registers (4 CTAs per SM
+// instead of 8) cost the streaming pass more than the launch saves.
+constexpr uint32_t kFuseRegions = 1024;
+
+template <bool FUSE>
+__global__ void __launch_bounds__(256, FUSE ? 4 : 8) k_pyramid(BatchDev bd, uint32_t total) {
     __shared__ uint64_t s1[256];
     __shared__ uint64_t s2[32];
     __shared__ uint64_t s3[4];
-    const uint32_t t = threadIdx.x;
+    __shared__ uint32_t s_warp[8];
+    __shared__ uint32_t s_last;
+    __shared__ __align__(16) uint64_t s_top[FUSE ? 2 : 1][kTopWords];
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     for (uint32_t g = blockIdx.x; g < total; g += gridDim.x) {
         const int m = find_segment(bd.cta_off, bd.n, g);
         const MeshDev &md = bd.mesh[m];
         const Pyramid &py = md.py;
         uint64_t *__restrict__ bits = md.bits;
-        uint32_t *__restrict__ cnt = md.cnt;
+        uint32_t *__restrict__ pre = md.pre;
         const uint32_t b = g - bd.cta_off[m];
         if (md.regions && !bd.rflag[g]) {  // the same for the whole CTA
             bits[py.woff[1] + (uint64_t)b * 256 + t] = 0;
             if (t < 32) bits[py.woff[2] + (uint64_t)b * 32 + t] = 0;
             if (t < 4) bits[py.woff[3] + (uint64_t)b * 4 + t] = 0;
+            if (t < 4) md.base[(uint64_t)t * md.bstride + b] = 0;
             if (t == 0) reinterpret_cast<uint32_t *>(bits + py.woff[4])[b] = 0;
-            continue;
-        }
-        {
+        } else {
             const uint4 *src = reinterpret_cast<const uint4 *>(bits + py.woff[0] + (uint64_t)b * 2048 + t * 8);
             uint64_t w1 = 0;
             uint32_t c0 = 0;
@@ -102,79 +256,91 @@ __global__ void __launch_bounds__(256, 8) k_pyramid(BatchDev bd, uint32_t total)
                 w1 |= (uint64_t)nz_bytes(a) << (16 * q);
                 w1 |= (uint64_t)nz_bytes(c) << (16 * q + 8);
             }
-            cnt[py.coff[0] + (uint64_t)b * 256 + t] = c0;
             bits[py.woff[1] + (uint64_t)b * 256 + t] = w1;
             s1[t] = w1;
-        }
-        __syncthreads();
-        if (t < 32) {
-            uint64_t w = 0;
-            uint32_t c = 0;
+            uint32_t sum0;
+            pre[py.coff[0] + (uint64_t)b * 256 + t] = block_exscan<256>(c0, s_warp, sum0);  // s1 is complete after it
+            if (warp == 0) {  // levels 2..4 of the region: one warp
+                uint64_t w = 0;
+                uint32_t c = 0;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const uint64_t v = s1[8 * t + k];
-                c += __popcll(v);
-                w |= (uint64_t)nz_bytes(v) << (8 * k);
-            }
-            cnt[py.coff[1] + (uint64_t)b * 32 + t] = c;
-            bits[py.woff[2] + (uint64_t)b * 32 + t] = w;
-            s2[t] = w;
-        }
-        __syncthreads();
-        if (t < 4) {
-            uint64_t w = 0;
-            uint32_t c = 0;
+                for (int k = 0; k < 8; ++k) {
+                    const uint64_t v = s1[8 * t + k];
+                    c += __popcll(v);
+                    w |= (uint64_t)nz_bytes(v) << (8 * k);
+                }
+                uint32_t incl = c;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const uint64_t v = s2[8 * t + k];
-                c += __popcll(v);
-                w |= (uint64_t)nz_bytes(v) << (8 * k);
-            }
-            cnt[py.coff[2] + (uint64_t)b * 4 + t] = c;
-            bits[py.woff[3] + (uint64_t)b * 4 + t] = w;
-            s3[t] = w;
-        }
-        __syncthreads();
-        if (t == 0) {
-            uint32_t w = 0, c = 0;
+                for (int d = 1; d < 32; d <<= 1) {
+                    const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                    if (lane >= d) incl += o;
+                }
+                const uint32_t sum1 = __shfl_sync(0xFFFFFFFFu, incl, 31);
+                pre[py.coff[1] + (uint64_t)b * 32 + t] = incl - c;
+                bits[py.woff[2] + (uint64_t)b * 32 + t] = w;
+                s2[t] = w;
+                __syncwarp();
+                w = 0;
+                c = 0;
+                if (t < 4) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                c += __popcll(s3[k]);
-                w |= nz_bytes(s3[k]) << (8 * k);
+                    for (int k = 0; k < 8; ++k) {
+                        const uint64_t v = s2[8 * t + k];
+                        c += __popcll(v);
+                        w |= (uint64_t)nz_bytes(v) << (8 * k);
+                    }
+                    bits[py.woff[3] + (uint64_t)b * 4 + t] = w;
+                    s3[t] = w;
+                }
+                incl = c;
+#pragma unroll
+                for (int d = 1; d < 4; d <<= 1) {
+                    const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                    if (lane >= d) incl += o;
+                }
+                const uint32_t sum2 = __shfl_sync(0xFFFFFFFFu, incl, 3);
+                if (t < 4) pre[py.coff[2] + (uint64_t)b * 4 + t] = incl - c;
+                __syncwarp();
+                if (t == 0) {
+                    uint32_t w4 = 0, sum3 = 0;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        sum3 += __popcll(s3[k]);
+                        w4 |= nz_bytes(s3[k]) << (8 * k);
+                    }
+                    uint32_t *base = md.base + b;
+                    base[0] = sum0;
+                    base[md.bstride] = sum1;
+                    base[2 * (uint64_t)md.bstride] = sum2;
+                    base[3 * (uint64_t)md.bstride] = sum3;
+                    reinterpret_cast<uint32_t *>(bits + py.woff[4])[b] = w4;
+                }
             }
-            if (c) atomicAdd(cnt + py.coff[3] + b / 2, c);
-            reinterpret_cast<uint32_t *>(bits + py.woff[4])[b] = w;
         }
-        __syncthreads();  // s1..s3 are rewritten by the next region
+        __syncthreads();  // s1 is rewritten by the next region; the region's stores come before its arrival
+        if (FUSE) {
+            if (t == 0) {
+                __threadfence();
+                s_last = atomicAdd(md.done, 1u) == py.ctas - 1 ? 1u : 0u;
+                __threadfence();
+            }
+            __syncthreads();
+            if (s_last) {
+                scan_regions_all<256>(md, s_warp);
+                finish_top<256>(md, s_top, s_warp);
+            }
+        }
     }
 }
 
-// Levels 5.. and the counts of levels 4.. of every mesh: one CTA per mesh.
-__global__ void __launch_bounds__(256) k_pyramid_top(BatchDev bd) {
-    const MeshDev &md = bd.mesh[blockIdx.x];
-    const Pyramid &py = md.py;
-    uint64_t *__restrict__ bits = md.bits;
-    uint32_t *__restrict__ cnt = md.cnt;
-    const uint32_t t = threadIdx.x;
-    for (int l = 4; l < py.levels; ++l) {
-        const uint64_t *in = bits + py.woff[l];
-        const uint64_t nblk = py.words[l] / 8;
-        const bool has_next = l + 1 < py.levels;
-        uint64_t *out = has_next ? bits + py.woff[l + 1] : nullptr;
-        for (uint64_t j = t; j < nblk; j += blockDim.x) {
-            uint64_t w = 0;
-            uint32_t c = 0;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const uint64_t v = in[8 * j + k];
-                c += __popcll(v);
-                w |= (uint64_t)nz_bytes(v) << (8 * k);
-            }
-            cnt[py.coff[l] + j] = c;
-            if (has_next) out[j] = w;
-        }
-        __syncthreads();
-    }
+// The region sums' prefixes (CTAs 0..3 of a mesh, one level each) and levels
+// 5.. (CTA 4) of every mesh.
+__global__ void __launch_bounds__(1024) k_pyramid_finish(BatchDev bd) {
+    __shared__ __align__(16) uint64_t s_top[2][kTopWords];
+    __shared__ uint32_t s_warp[32];
+    const MeshDev &md = bd.mesh[blockIdx.y];
+    if (blockIdx.x < 4) scan_regions<1024, 16>(md, (int)blockIdx.x, s_warp);
+    else finish_top<1024>(md, s_top, s_warp);
 }
 
 // ---------------------------------------------------------------------------
@@ -393,12 +559,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const uint32_t *__re
     }
 }
 
-__global__ void k_level_totals(BatchDev bd) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int m = i / kMaxLevels, l = i % kMaxLevels;
-    if (m >= bd.n) return;
-    const MeshDev &md = bd.mesh[m];
-    if (l < md.py.levels) md.totals[l] = md.pre[md.py.coff[l + 1]] - md.pre[md.py.coff[l]];
+// Set bits of level l before its 512-bit block `blk`.
+__device__ __forceinline__ uint32_t block_rank(const RankDev &r, const Pyramid &py, int l, uint64_t blk) {
+    if (l >= 4) return r.pre[py.coff[l] + blk];
+    if (l == 3) return r.base[3 * (uint64_t)r.bstride + 2 * blk];  // a level-3 block spans two regions
+    return r.base[(uint64_t)l * r.bstride + (blk >> (8 - 3 * l))] + r.pre[py.coff[l] + blk];
 }
 
 // One thread per 64-bit word of every job's levels: its first rank is the
@@ -439,7 +604,7 @@ __device__ __forceinline__ void warp_codes(uint64_t *out, uint32_t o, uint32_t p
 // positions.  All 32 lanes of the warp call (8 aligned lanes per block).
 __device__ __forceinline__ void compact_word(const CompactJob &job, int l, uint64_t w, uint64_t v) {
     const int sub = threadIdx.x & 7;
-    const uint32_t r0 = v ? job.pre[job.py.coff[l] + (w >> 3)] - job.pre[job.py.coff[l]] : 0u;
+    const uint32_t r0 = v ? block_rank(job.rank, job.py, l, w >> 3) : 0u;
     const uint32_t pc = __popcll(v);
     uint32_t x = pc;
 #pragma unroll
@@ -509,7 +674,7 @@ __global__ void __launch_bounds__(256) k_compact_keys(KeyBatch kb, uint64_t tota
         const KeyJob &job = kb.job[j];
         blk = job.blocks[item - kb.blk_off[j]];
         v = job.bits[blk * 8 + sub];
-        r = job.pre[blk] - job.pre[0];
+        r = job.rank.base[blk >> 8] + job.rank.pre[blk];
     }
     const uint32_t pc = __popcll(v);
     uint32_t x = pc;
@@ -975,10 +1140,15 @@ cudaError_t unique_impl(const T *in, uint64_t n, T *out, uint32_t *tile_counts, 
 
 }  // namespace
 
-cudaError_t launch_pyramid(const BatchDev &b, uint32_t total_ctas, int num_sms, cudaStream_t st) {
+cudaError_t launch_pyramid(const BatchDev &b, uint32_t total_ctas, uint32_t max_ctas, int num_sms, cudaStream_t st) {
     if (total_ctas == 0) return cudaSuccess;
-    k_pyramid<<<std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 8), 256, 0, st>>>(b, total_ctas);
-    k_pyramid_top<<<b.n, 256, 0, st>>>(b);
+    if (max_ctas <= kFuseRegions && total_ctas <= (uint32_t)num_sms * 8) {
+        k_pyramid<true><<<std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 4), 256, 0, st>>>(b, total_ctas);
+        count_launches(1);
+        return cudaGetLastError();
+    }
+    k_pyramid<false><<<std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 8), 256, 0, st>>>(b, total_ctas);
+    k_pyramid_finish<<<dim3(5, b.n), 1024, 0, st>>>(b);
     count_launches(2);
     return cudaGetLastError();
 }
@@ -1019,13 +1189,6 @@ cudaError_t launch_scan_stalled(const uint32_t *in, uint32_t *out, uint64_t n, u
     if ((e = cudaMemcpyAsync(scratch, &one, sizeof(one), cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
     k_scan<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, scratch, status, spin_limit);
-    count_launches(1);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_level_totals(const BatchDev &b, cudaStream_t st) {
-    const int n = b.n * kMaxLevels;
-    k_level_totals<<<(n + 127) / 128, 128, 0, st>>>(b);
     count_launches(1);
     return cudaGetLastError();
 }
