@@ -207,15 +207,6 @@ struct MetaLayout {
     }
 };
 
-__global__ void k_meta_init(uint32_t *mm, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    for (int a = 0; a < 3; ++a) {
-        mm[8 * i + a] = 0xFFFFFFFFu;
-        mm[8 * i + 3 + a] = 0u;
-    }
-}
-
 // top_codes[i] = *ptrs[i] (the single code of each mesh's top level)
 __global__ void k_gather_top(const uint64_t *const *ptrs, int n, uint64_t *out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -404,6 +395,7 @@ int batch_phase_a(svo_batch *b) {
     uint32_t *mm = reinterpret_cast<uint32_t *>(b->meta + ml.mm);
     uint32_t *done = reinterpret_cast<uint32_t *>(b->meta + ml.done);
     uint32_t *counters = reinterpret_cast<uint32_t *>(b->meta + ml.counters);
+    bool any_regions = false;
     b->h_mesh.assign(n, MeshDev{});
     for (int k = 0; k < n; ++k) {
         const MeshHost &mh = b->m[b->live[k]];
@@ -423,6 +415,7 @@ int batch_phase_a(svo_batch *b) {
         d.done = done + k;
         d.py = mh.py;
         d.regions = mh.py.words[0] >= kRegionWords ? 1 : 0;
+        any_regions |= d.regions != 0;
     }
     const size_t p_mesh = tables.add(b->h_mesh), p_tri = tables.add(tri_off), p_cta = tables.add(cta_off),
                  p_bbox = tables.add(bbox_off);
@@ -431,19 +424,18 @@ int batch_phase_a(svo_batch *b) {
     const uint64_t *d_tri_off = reinterpret_cast<const uint64_t *>(dt + p_tri);
     const uint32_t *d_cta_off = reinterpret_cast<const uint32_t *>(dt + p_cta);
     const uint32_t *d_bbox_off = reinterpret_cast<const uint32_t *>(dt + p_bbox);
-    SVO_TRY(cudaMemcpyAsync(dt, tables.buf.data(), tables.buf.size(), cudaMemcpyHostToDevice, st), "upload meshes");
+    if (n > 1)  // a lone mesh's table goes with the first kernel
+        SVO_TRY(cudaMemcpyAsync(dt, tables.buf.data(), tables.buf.size(), cudaMemcpyHostToDevice, st), "upload meshes");
     const BatchDev bd{b->d_mesh, n, d_tri_off, d_cta_off, d_bbox_off, rflag};
     const bool strict = (b->flags & SVO_FLAG_STRICT_FP) != 0;
     StageTimer tm((b->flags & SVO_FLAG_TIMINGS) != 0);
     for (int attempt = 0; attempt < 2; ++attempt) {
         tm.mark(StageTimer::kStart, st);
         SVO_TRY(cudaMemsetAsync(b->meta, 0, ml.imm, st), "memset meta");
-        k_meta_init<<<(n + 127) / 128, 128, 0, st>>>(mm, n);
-        count_launches(1);
-        SVO_TRY(launch_bbox(bd, bblocks, st), "bbox");
+        SVO_TRY(launch_front(bd, n == 1 ? &b->h_mesh[0] : nullptr, bblocks, ctas, any_regions, ctx->num_sms, st),
+                "bounding cube");
         tm.mark(StageTimer::kBbox, st);
-        SVO_TRY(cudaMemsetAsync(rflag, 0, std::max<uint32_t>(ctas, 1), st), "memset regions");
-        SVO_TRY(launch_regions(bd, (int64_t)tris, ctas, ctx->num_sms, st), "zero bitmaps");
+        if (any_regions) SVO_TRY(launch_regions(bd, (int64_t)tris, ctas, ctx->num_sms, st), "zero regions");
         SVO_TRY(launch_voxelize(bd, (int64_t)tris, strict, b->tune, big, big_cap, counters, ctx->num_sms, st,
                                 small),
                 "voxelize");

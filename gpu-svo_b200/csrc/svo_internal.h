@@ -60,7 +60,7 @@ struct MeshDev {
     int res[3];
     int regions;             // 1: level 0 is zeroed and read only in the regions triangles reach
     GridParams *gp;
-    uint32_t *mm;            // bbox scratch (6 u32)
+    uint32_t *mm;            // bbox scratch (8 u32: 6 extremes, blocks finished), zero at the start
     uint64_t *bits;          // this mesh's pyramid (level l at bits + py.woff[l])
     uint32_t *pre;           // block ranks (RankDev)
     uint32_t *base;          // region sums, then their prefixes (RankDev)
@@ -160,7 +160,14 @@ __host__ __device__ __forceinline__ int find_segment(const T *off, int n, T x) {
     return lo;
 }
 
-cudaError_t launch_bbox(const BatchDev &b, uint32_t total_blocks, cudaStream_t st);
+// Bounding cube and grid of every mesh (bbox_blocks: bbox_off[n]), beside the
+// clearing of the bitmaps of total_ctas regions (0: they are clear already)
+// and, with any_regions, of the region flags (padded to whole words).  one:
+// the host copy of a one-mesh batch's table, which the kernel stores in b
+// (mesh, tri_off, cta_off), or null when b's tables are filled in.  Every mm
+// and gp->status must be zero.
+cudaError_t launch_front(const BatchDev &b, const MeshDev *one, uint32_t bbox_blocks, uint32_t total_ctas,
+                         bool any_regions, int num_sms, cudaStream_t st);
 // mm[0] = min, mm[1] = max of n int32 indices.
 cudaError_t launch_index_range(const int32_t *idx, int64_t n, int32_t *mm, cudaStream_t st);
 // The same for a table of n index arrays in one launch: job k gets
@@ -173,7 +180,7 @@ struct IndexJob {
 uint32_t index_blocks(int64_t n);
 cudaError_t launch_index_ranges(const IndexJob *jobs, int n, const uint32_t *block_off, uint32_t total_blocks,
                                 int32_t *mm, cudaStream_t st);
-// counters: 4 u32 (queue entries, queue cursor, -, small-list length); small:
+// counters: 4 zeroed u32 (queue entries, queue cursor, -, small-list length); small:
 // room for one u64 per triangle, or null (then no in-warp tier unless big is
 // null too, which walks every large triangle in the warp that set it up).
 cudaError_t launch_voxelize(const BatchDev &b, int64_t total_tris, bool strict, const VoxTuning &tune,
@@ -182,10 +189,8 @@ cudaError_t launch_voxelize(const BatchDev &b, int64_t total_tris, bool strict, 
 // Builds levels 1.. of every mesh's pyramid, the block ranks and the level
 // totals; max_ctas: the most regions of any mesh (py.ctas).  done must be zero.
 cudaError_t launch_pyramid(const BatchDev &b, uint32_t total_ctas, uint32_t max_ctas, int num_sms, cudaStream_t st);
-// Flags the level-0 regions that triangles of region-mode meshes reach, then
-// zeroes level 0 where needed (every region of other meshes, the flagged ones
-// of region-mode meshes) and each mesh's levels >= 3.  Replaces a memset of
-// the whole pyramid; rflag must be zeroed (total_ctas bytes).
+// For batches with a region-mode mesh: flags the level-0 regions that its
+// triangles reach (rflag zeroed by launch_front), then zeroes those.
 cudaError_t launch_regions(const BatchDev &b, int64_t total_tris, uint32_t total_ctas, int num_sms, cudaStream_t st);
 // Exclusive scan of n u32 values; out has n + 1 entries (out[n] = total).
 // scratch: >= scan_scratch_words(n) u64 words, zeroed by the call.

@@ -127,7 +127,6 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
     MeshDev *d_mesh = c.take<MeshDev>(1);
     uint64_t *d_tri_off = c.take<uint64_t>(2);
     uint32_t *d_cta_off = c.take<uint32_t>(2);
-    uint32_t *d_bbox_off = c.take<uint32_t>(2);
     CompactJob *d_job = c.take<CompactJob>(1);
     uint64_t *d_word_off = c.take<uint64_t>(2);
     uint64_t *bits = c.take<uint64_t>(py.total_words);
@@ -146,7 +145,7 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
         if ((rc = cuda(cudaStreamSynchronize(st)))) return rc;
         if (h[0] < 0 || h[1] >= n_points) return noalloc_fail(SVO_ERR_INVALID_ARGUMENT, "triangle index out of range");
     }
-    // the one-mesh tables, copied from the host stack (no device allocation)
+    // the one-mesh table, passed by value to the first kernel
     MeshDev md{};
     md.pts = points;
     md.tris = tris;
@@ -164,19 +163,10 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
     md.totals = totals;
     md.done = done;
     md.py = py;
-    const uint64_t h_tri_off[2] = {0, (uint64_t)nt};
-    const uint32_t h_cta_off[2] = {0, py.ctas};
-    const uint32_t h_bbox_off[2] = {0, bbox_blocks(n_points)};
     // everything that must start at zero (the array keeps the last call's data)
     if ((rc = cuda(cudaMemsetAsync(base, 0, c.used, st)))) return rc;
-    const uint32_t mm_init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
-    if ((rc = cuda(cudaMemcpyAsync(mm, mm_init, sizeof(mm_init), cudaMemcpyHostToDevice, st)))) return rc;
-    if ((rc = cuda(cudaMemcpyAsync(d_mesh, &md, sizeof(md), cudaMemcpyHostToDevice, st)))) return rc;
-    if ((rc = cuda(cudaMemcpyAsync(d_tri_off, h_tri_off, sizeof(h_tri_off), cudaMemcpyHostToDevice, st)))) return rc;
-    if ((rc = cuda(cudaMemcpyAsync(d_cta_off, h_cta_off, sizeof(h_cta_off), cudaMemcpyHostToDevice, st)))) return rc;
-    if ((rc = cuda(cudaMemcpyAsync(d_bbox_off, h_bbox_off, sizeof(h_bbox_off), cudaMemcpyHostToDevice, st)))) return rc;
-    const BatchDev bd{d_mesh, 1, d_tri_off, d_cta_off, d_bbox_off};
-    if ((rc = cuda(launch_bbox(bd, h_bbox_off[1], st)))) return rc;
+    const BatchDev bd{d_mesh, 1, d_tri_off, d_cta_off, nullptr};
+    if ((rc = cuda(launch_front(bd, &md, bbox_blocks(n_points), 0, false, num_sms, st)))) return rc;
     VoxTuning tune;
     tune.warp_max = 0xFFFFFFFFu;  // no big-triangle queue: warps take every large triangle
     if ((rc = cuda(launch_voxelize(bd, nt, (flags & SVO_FLAG_STRICT_FP) != 0, tune, nullptr, 0, counters,

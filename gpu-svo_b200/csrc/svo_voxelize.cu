@@ -49,18 +49,18 @@ __device__ __forceinline__ void bbox_take(float v, int a, uint32_t lo[3], uint32
     hi[a] = max(hi[a], o);
 }
 
-// Block b belongs to mesh m = the segment of bbox_off holding b.  When the
-// mesh's points are 16-byte aligned, 4 points (12 floats, 3 float4) per step;
-// the component of float k is k % 3, the same in every 12-float group.
-__global__ void k_bbox_reduce(BatchDev bd) {
-    const int m = find_segment(bd.bbox_off, bd.n, (uint32_t)blockIdx.x);
-    const MeshDev &md = bd.mesh[m];
+// Block `blk` of the `nb` blocks of mesh md's reduction.  When the mesh's
+// points are 16-byte aligned, 4 points (12 floats, 3 float4) per step; the
+// component of float k is k % 3, the same in every 12-float group.  md.mm
+// holds the mesh's largest ~key (0..2: the smallest keys) and largest key
+// (3..5) so far, so that zero is the start value of all six; returns true in
+// every thread of the mesh's last block, with md.mm complete.
+__device__ __forceinline__ bool bbox_block(const MeshDev &md, uint32_t blk, uint32_t nb) {
     const float *__restrict__ pts = md.pts;
     const int64_t n = md.n_pts;
     uint32_t lo[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, hi[3] = {0u, 0u, 0u};
     bool bad = false;
-    const uint32_t nb = bd.bbox_off[m + 1] - bd.bbox_off[m];
-    const int64_t tid = (blockIdx.x - bd.bbox_off[m]) * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t tid = blk * (int64_t)blockDim.x + threadIdx.x;
     const int64_t nth = (int64_t)nb * blockDim.x;
     int64_t done = 0;
     if ((reinterpret_cast<uintptr_t>(pts) & 15) == 0) {
@@ -87,49 +87,54 @@ __global__ void k_bbox_reduce(BatchDev bd) {
     // the block's extremes, then one atomic per value and block (the 6 words
     // are shared by every block of the mesh)
     __shared__ uint32_t wmm[32][6];
+    __shared__ uint32_t s_last;
     const int warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     if ((threadIdx.x & 31) == 0) {
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            wmm[warp][a] = lo[a];
+            wmm[warp][a] = ~lo[a];
             wmm[warp][3 + a] = hi[a];
         }
     }
     __syncthreads();
     if (threadIdx.x < 6) {
         uint32_t v = wmm[0][threadIdx.x];
-        for (int w = 1; w < nwarp; ++w) v = threadIdx.x < 3 ? min(v, wmm[w][threadIdx.x]) : max(v, wmm[w][threadIdx.x]);
-        if (threadIdx.x < 3) atomicMin(md.mm + threadIdx.x, v);
-        else atomicMax(md.mm + threadIdx.x, v);
+        for (int w = 1; w < nwarp; ++w) v = max(v, wmm[w][threadIdx.x]);
+        atomicMax(md.mm + threadIdx.x, v);
+        __threadfence();
     }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(md.mm + 6, 1u) == nb - 1 ? 1u : 0u;
+        __threadfence();
+    }
+    __syncthreads();
+    return s_last != 0;
 }
 
 // createMeshBBCube (src/BaseModel.h:24-49) and unitVoxelSize
-// (src/SVO.cu:348-350).  Host code in the reference: no contraction there, so
-// every operation is an explicitly rounded intrinsic.
-__global__ void k_grid_setup(BatchDev bd) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= bd.n) return;
-    const MeshDev &md = bd.mesh[m];
-    const uint32_t *mm = md.mm;
+// (src/SVO.cu:348-350), one thread.  Host code in the reference: no
+// contraction there, so every operation is an explicitly rounded intrinsic.
+__device__ __forceinline__ void grid_setup(const MeshDev &md) {
     GridParams *gp = md.gp;
-    const int rx = md.res[0], ry = md.res[1], rz = md.res[2];
     float mn[3], mx[3], len[3], amin[3], amax[3];
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-        mn[a] = ord2f(mm[a]);
-        mx[a] = ord2f(mm[3 + a]);
+        mn[a] = ord2f(~__ldcg(md.mm + a));
+        mx[a] = ord2f(__ldcg(md.mm + 3 + a));
         len[a] = __fsub_rn(mx[a], mn[a]);
         amin[a] = mn[a];
         amax[a] = mx[a];
     }
     const float maxlen = cmaxf(len[0], cmaxf(len[1], len[2]));
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
         if (maxlen == len[a]) continue;
         const float half = __fdiv_rn(__fsub_rn(maxlen, len[a]), 2.0f);
         amin[a] = __fsub_rn(mn[a], half);
         amax[a] = __fadd_rn(mx[a], half);
     }
-    const int res[3] = {rx, ry, rz};
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
         const float eps = __fdiv_rn(__fsub_rn(amax[a], amin[a]), 10001.0f);
         amin[a] = __fsub_rn(amin[a], eps);
@@ -139,7 +144,61 @@ __global__ void k_grid_setup(BatchDev bd) {
         gp->bbox[3 + a] = amax[a];
         gp->bbox[6 + a] = w;
         gp->origin[a] = amin[a];
-        gp->unit[a] = __fdiv_rn(w, (float)res[a]);
+        gp->unit[a] = __fdiv_rn(w, (float)md.res[a]);
+    }
+}
+
+// The first kernel of a build, two independent jobs side by side:
+//   * blocks [0, bbox_blocks): the bounding cube of every mesh (block b
+//     belongs to the mesh whose segment of bbox_off holds b); a mesh's last
+//     block sets up its grid;
+//   * the other blocks clear the bitmaps: level 0 of the meshes that are not
+//     in region mode (those clear their flagged regions later), the level-0
+//     region flags, and the words the pyramid does not write whole (level-3
+//     padding, level 4, which it writes as 32-bit halves, and levels >= 5).
+// A lone mesh's table travels by value (`one`) and is stored for the later
+// kernels here, which saves its upload.  (One kernel instead of the five
+// launches it replaces: a launch costs about 4 us in a small build, where the
+// host's launches are the critical path.)
+__global__ void __launch_bounds__(256) k_front(BatchDev bd, const __grid_constant__ MeshDev one, int by_value,
+                                               uint32_t bbox_blocks, uint32_t regions, uint32_t flag_words) {
+    if (blockIdx.x < bbox_blocks) {
+        const int m = by_value ? 0 : find_segment(bd.bbox_off, bd.n, (uint32_t)blockIdx.x);
+        if (by_value && blockIdx.x == 0 && threadIdx.x == 0) {
+            *const_cast<MeshDev *>(bd.mesh) = one;
+            auto *tri = const_cast<uint64_t *>(bd.tri_off);
+            auto *cta = const_cast<uint32_t *>(bd.cta_off);
+            tri[0] = 0;
+            tri[1] = (uint64_t)one.n_tris;
+            cta[0] = 0;
+            cta[1] = one.py.ctas;
+        }
+        const uint32_t b0 = by_value ? 0u : bd.bbox_off[m];
+        const uint32_t nb = by_value ? bbox_blocks : bd.bbox_off[m + 1] - b0;
+        // (two calls: the by-value table is read from the constant bank)
+        if (by_value) {
+            if (bbox_block(one, blockIdx.x - b0, nb) && threadIdx.x == 0) grid_setup(one);
+        } else {
+            const MeshDev &md = bd.mesh[m];
+            if (bbox_block(md, blockIdx.x - b0, nb) && threadIdx.x == 0) grid_setup(md);
+        }
+        return;
+    }
+    const uint32_t zb = blockIdx.x - bbox_blocks, nz = gridDim.x - bbox_blocks;
+    for (uint32_t i = zb * blockDim.x + threadIdx.x; i < flag_words; i += nz * blockDim.x)
+        reinterpret_cast<uint32_t *>(bd.rflag)[i] = 0;
+    for (uint32_t g = zb; g < regions; g += nz) {
+        const int m = by_value ? 0 : find_segment(bd.cta_off, bd.n, g);
+        const MeshDev &md = by_value ? one : bd.mesh[m];
+        const uint32_t r = by_value ? g : g - bd.cta_off[m];
+        if (!md.regions) {
+            uint4 *w = reinterpret_cast<uint4 *>(md.bits + md.py.woff[0] + (uint64_t)r * 2048);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) w[threadIdx.x + 256 * q] = make_uint4(0, 0, 0, 0);
+        }
+        const uint64_t z0 = md.py.woff[3] + 4ull * md.py.ctas;
+        for (uint64_t i = z0 + (uint64_t)r * 256 + threadIdx.x; i < md.py.total_words; i += (uint64_t)md.py.ctas * 256)
+            md.bits[i] = 0;
     }
 }
 
@@ -876,10 +935,12 @@ cudaError_t launch_index_ranges(const IndexJob *jobs, int n, const uint32_t *blo
     return cudaGetLastError();
 }
 
-cudaError_t launch_bbox(const BatchDev &b, uint32_t total_blocks, cudaStream_t st) {
-    k_bbox_reduce<<<total_blocks, 256, 0, st>>>(b);
-    k_grid_setup<<<(b.n + 127) / 128, 128, 0, st>>>(b);
-    count_launches(2);
+cudaError_t launch_front(const BatchDev &b, const MeshDev *one, uint32_t bbox_blocks, uint32_t total_ctas,
+                         bool any_regions, int num_sms, cudaStream_t st) {
+    const uint32_t zblocks = std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 8);
+    k_front<<<bbox_blocks + zblocks, 256, 0, st>>>(b, one ? *one : MeshDev{}, one ? 1 : 0, bbox_blocks, total_ctas,
+                                                   any_regions ? (total_ctas + 3) / 4 : 0);
+    count_launches(1);
     return cudaGetLastError();
 }
 
@@ -972,24 +1033,16 @@ __global__ void __launch_bounds__(256) k_region_mark(BatchDev bd, int64_t total)
     }
 }
 
-// Level-0 regions, a persistent grid taking them in turn: zeroes each unless
-// it is a region-mode mesh's unflagged region.  The pyramid writes every word of levels 1 and 2 and the
-// first 4 * ctas of level 3; the words after those (level-3 padding, level 4,
-// which the pyramid writes as 32-bit halves, and levels >= 5) are zeroed
-// here, spread over the mesh's CTAs.
+// Zeroes the flagged level-0 regions of the region-mode meshes, a persistent
+// grid taking the regions in turn.
 __global__ void __launch_bounds__(256) k_region_zero(BatchDev bd, uint32_t total) {
     for (uint32_t g = blockIdx.x; g < total; g += gridDim.x) {
+        if (!bd.rflag[g]) continue;
         const int m = find_segment(bd.cta_off, bd.n, g);
         const MeshDev &md = bd.mesh[m];
-        const uint32_t r = g - bd.cta_off[m];
-        if (!md.regions || bd.rflag[g]) {
-            uint4 *w = reinterpret_cast<uint4 *>(md.bits + md.py.woff[0] + (uint64_t)r * 2048);
+        uint4 *w = reinterpret_cast<uint4 *>(md.bits + md.py.woff[0] + (uint64_t)(g - bd.cta_off[m]) * 2048);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) w[threadIdx.x + 256 * q] = make_uint4(0, 0, 0, 0);
-        }
-        const uint64_t z0 = md.py.woff[3] + 4ull * md.py.ctas;
-        for (uint64_t i = z0 + (uint64_t)r * 256 + threadIdx.x; i < md.py.total_words; i += (uint64_t)md.py.ctas * 256)
-            md.bits[i] = 0;
+        for (int q = 0; q < 4; ++q) w[threadIdx.x + 256 * q] = make_uint4(0, 0, 0, 0);
     }
 }
 
@@ -1002,19 +1055,14 @@ cudaError_t launch_regions(const BatchDev &b, int64_t total_tris, uint32_t total
         k_region_mark<<<blocks, 256, 0, st>>>(b, total_tris);
         count_launches(1);
     }
-    if (total_ctas > 0) {
-        k_region_zero<<<std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 8), 256, 0, st>>>(b, total_ctas);
-        count_launches(1);
-    }
+    k_region_zero<<<std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 8), 256, 0, st>>>(b, total_ctas);
+    count_launches(1);
     return cudaGetLastError();
 }
 
 cudaError_t launch_voxelize(const BatchDev &b, int64_t total, bool strict, const VoxTuning &tune, uint4 *big,
                             uint32_t big_cap, uint32_t *counters, int num_sms, cudaStream_t st, uint64_t *small) {
     // counters[0] = queue entries, counters[1] = queue cursor, counters[3] = small-list length
-    cudaError_t e = cudaMemsetAsync(counters, 0, 2 * sizeof(uint32_t), st);
-    if (e == cudaSuccess && small) e = cudaMemsetAsync(counters + 3, 0, sizeof(uint32_t), st);
-    if (e != cudaSuccess) return e;
     if (total > 0) {
         const int64_t want = (total + 255) / 256;
         const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)num_sms * 16));

@@ -337,7 +337,8 @@ int svo_result_copy_edges(const svo_result *r, svo_edge *dst, int64_t cap);
 int svo_result_copy_keys(const svo_result *r, uint64_t *dst, int64_t cap);
 /* Per-stage device times in ms of a build made with SVO_FLAG_TIMINGS, from
  * CUDA events on the build stream: [0] first to last event (includes the
- * host round trip that sizes the outputs), [1] bounding cube, [2] voxelize,
+ * host round trip that sizes the outputs), [1] bounding cube and clearing of
+ * the bitmaps, [2] voxelize,
  * [3] bitmap pyramid with its block ranks, [4] 0 (a rank scan of its own in
  * earlier versions), [5] level code lists,
  * [6] node/vertex/edge emission, [7] duplicate removal, [8] dedup keys (on a
