@@ -1,10 +1,11 @@
 // svo_capi.cu -- C ABI: context, build orchestration, results.
 //
 // One build = (host->device copy of the mesh) -> bounding cube -> voxelize
-// into the level-0 bitmap -> pyramid + block counts -> one scan -> one small
-// device->host read of the level totals (the only mid-build sync, to size the
+// into the level-0 bitmap -> pyramid + block ranks, whose last kernel writes
+// the level totals to pinned host memory (the only mid-build sync, to size the
 // outputs) -> per-level code lists -> one emission pass writing nodes,
-// vertices and edges -> one small read of the duplicate counters.
+// vertices and edges, which raises a flag in pinned host memory when it meets
+// duplicates.
 // The reference's equivalent (src/SVO.cu:341-735) synchronises with the host
 // at least six times per level and reallocates its node array per level.
 #include <atomic>
@@ -38,6 +39,13 @@ struct svo_ctx {
     std::mutex tune_mu;
     std::mutex aux_mu;                 // builds on other threads take sets of their own
     std::vector<AuxStreams *> aux_free, aux_all;
+    // Pinned host blocks for the reports of batches in flight (one batch each).
+    struct Pinned {
+        void *p;
+        size_t bytes;
+    };
+    std::mutex pinned_mu;
+    std::vector<Pinned> pinned_free;
 };
 
 // One device block that holds the output arrays of several results (a wave of
@@ -186,12 +194,14 @@ struct MeshHost {
     int T = -1;
     uint64_t n_l[kMaxLevels] = {}, off[kMaxLevels + 1] = {};
     uint64_t N = 0;
+    uint64_t top = 0;  // the code of the single level-T node
     bool emitted = false;
 };
 
-// Layout of the small per-batch meta block (device), read back after phase A.
+// Layout of a batch's small device block that starts zeroed: counters, grid
+// parameters, bounding-box scratch, duplicate counts.
 struct MetaLayout {
-    size_t counters = 0, gp = 0, totals = 0, mm = 0, done = 0, imm = 0, bytes = 0;
+    size_t counters = 0, gp = 0, any = 0, mm = 0, done = 0, dups = 0, bytes = 0;
     explicit MetaLayout(int n) {
         auto take = [&](size_t b) {
             const size_t o = (bytes + 255) / 256 * 256;
@@ -200,18 +210,12 @@ struct MetaLayout {
         };
         counters = take(4 * sizeof(uint32_t));
         gp = take(sizeof(GridParams) * n);
-        totals = take(sizeof(uint32_t) * kMaxLevels * n);
+        any = take(sizeof(uint64_t) * n);
         mm = take(sizeof(uint32_t) * 8 * n);
         done = take(sizeof(uint32_t) * n);
-        imm = take(sizeof(int32_t) * 2 * n);
+        dups = take(sizeof(unsigned long long) * 2 * n);
     }
 };
-
-// top_codes[i] = *ptrs[i] (the single code of each mesh's top level)
-__global__ void k_gather_top(const uint64_t *const *ptrs, int n, uint64_t *out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = *ptrs[i];
-}
 
 }  // namespace
 
@@ -226,9 +230,12 @@ struct svo_batch {
     uint64_t *bits = nullptr;
     uint32_t *pre = nullptr, *base = nullptr;  // block ranks, region prefixes (RankDev)
     uint8_t *rflag = nullptr;               // level-0 regions that triangles reach (one byte per pyramid CTA)
-    unsigned char *meta = nullptr;
+    unsigned long long *dups = nullptr;     // 2 per live mesh (device, zeroed by phase A)
+    svo_ctx::Pinned box{nullptr, 0};        // pinned host memory: a MeshOut per live mesh
+    MeshOut *out = nullptr;
     MeshDev *d_mesh = nullptr;
     std::vector<MeshDev> h_mesh;
+    bool pending = false;                   // the stream may still hold work of this batch
     float timings_a[5] = {};                // total, bbox, voxelize, pyramid, scan
     bool timed = false;
 };
@@ -242,9 +249,45 @@ T *batch_alloc(svo_batch *b, size_t count, cudaError_t &err) {
     return p;
 }
 
+// A pinned host block of at least `bytes` (kept blocks first); p is null when
+// there is none to be had.  Blocks of up to 1 MiB are kept for later batches,
+// at most 16 of them; the context frees them.
+svo_ctx::Pinned pinned_acquire(svo_ctx *ctx, size_t bytes) {
+    {
+        std::lock_guard<std::mutex> lk(ctx->pinned_mu);
+        for (size_t i = 0; i < ctx->pinned_free.size(); ++i)
+            if (ctx->pinned_free[i].bytes >= bytes) {
+                const svo_ctx::Pinned b = ctx->pinned_free[i];
+                ctx->pinned_free.erase(ctx->pinned_free.begin() + (long)i);
+                return b;
+            }
+    }
+    svo_ctx::Pinned b{nullptr, std::max<size_t>(bytes, 1 << 14)};
+    if (cudaHostAlloc(&b.p, b.bytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        b.p = nullptr;
+    }
+    return b;
+}
+
+void pinned_release(svo_ctx *ctx, svo_ctx::Pinned b) {
+    if (!b.p) return;
+    {
+        std::lock_guard<std::mutex> lk(ctx->pinned_mu);
+        if (b.bytes <= (1u << 20) && ctx->pinned_free.size() < 16) {
+            ctx->pinned_free.push_back(b);
+            return;
+        }
+    }
+    cudaFreeHost(b.p);
+}
+
+// The batch's stream must have finished (its kernels write to the report).
 void batch_release(svo_batch *b) {
     for (void *p : b->allocs) cudaFreeAsync(p, b->st);
     b->allocs.clear();
+    pinned_release(b->ctx, b->box);
+    b->box = svo_ctx::Pinned{nullptr, 0};
 }
 
 int mesh_error(MeshHost &mh, int code, const char *msg) {
@@ -293,6 +336,7 @@ int batch_phase_a(svo_batch *b) {
     cudaStream_t st = b->st;
     SVO_TRY(cudaSetDevice(ctx->device), "cudaSetDevice");
     cudaError_t err = cudaSuccess;
+    b->pending = true;
     // ---- validation and mesh data on the device ----
     for (int i = 0; i < (int)b->m.size(); ++i) {
         MeshHost &mh = b->m[i];
@@ -344,8 +388,10 @@ int batch_phase_a(svo_batch *b) {
     const int n = (int)b->live.size();
     if (n == 0) return SVO_OK;
     const MetaLayout ml(n);
-    b->meta = batch_alloc<unsigned char>(b, ml.bytes, err);
-    if (!b->meta) return cuda_fail(err, "alloc meta");
+    b->box = pinned_acquire(ctx, sizeof(MeshOut) * (size_t)n);
+    if (!b->box.p) return fail(SVO_ERR_OUT_OF_MEMORY, "pinned host memory");
+    b->out = static_cast<MeshOut *>(b->box.p);
+    std::memset(b->box.p, 0, sizeof(MeshOut) * (size_t)n);
     // ---- layout ----
     uint64_t words = 0, blocks = 0, bases = 0, tris = 0;
     uint32_t ctas = 0, max_ctas = 0, bblocks = 0;
@@ -378,6 +424,7 @@ int batch_phase_a(svo_batch *b) {
     auto a16 = [](size_t x) { return (x + 15) / 16 * 16; };
     const size_t t_bytes = a16(sizeof(MeshDev) * n) + a16(8 * (size_t)(n + 1)) + a16(4 * (size_t)(n + 1)) + 4 * (size_t)(n + 1);
     Layout lay;
+    const size_t o_meta = lay.add<unsigned char>(ml.bytes);
     const size_t o_bits = lay.add<uint64_t>(words), o_pre = lay.add<uint32_t>(blocks), o_base = lay.add<uint32_t>(bases),
                  o_big = lay.add<uint4>(big_cap), o_small = lay.add<uint64_t>(std::max<uint64_t>(tris, 1)),
                  o_rflag = lay.add<uint8_t>(std::max<uint32_t>(ctas, 1));
@@ -390,11 +437,13 @@ int batch_phase_a(svo_batch *b) {
     uint4 *big = reinterpret_cast<uint4 *>(blk + o_big);
     uint64_t *small = reinterpret_cast<uint64_t *>(blk + o_small);
     uint8_t *rflag = b->rflag = blk + o_rflag;
-    GridParams *gp = reinterpret_cast<GridParams *>(b->meta + ml.gp);
-    uint32_t *totals = reinterpret_cast<uint32_t *>(b->meta + ml.totals);
-    uint32_t *mm = reinterpret_cast<uint32_t *>(b->meta + ml.mm);
-    uint32_t *done = reinterpret_cast<uint32_t *>(b->meta + ml.done);
-    uint32_t *counters = reinterpret_cast<uint32_t *>(b->meta + ml.counters);
+    unsigned char *meta = blk + o_meta;
+    GridParams *gp = reinterpret_cast<GridParams *>(meta + ml.gp);
+    uint64_t *any = reinterpret_cast<uint64_t *>(meta + ml.any);
+    uint32_t *mm = reinterpret_cast<uint32_t *>(meta + ml.mm);
+    uint32_t *done = reinterpret_cast<uint32_t *>(meta + ml.done);
+    uint32_t *counters = reinterpret_cast<uint32_t *>(meta + ml.counters);
+    b->dups = reinterpret_cast<unsigned long long *>(meta + ml.dups);
     bool any_regions = false;
     b->h_mesh.assign(n, MeshDev{});
     for (int k = 0; k < n; ++k) {
@@ -411,7 +460,9 @@ int batch_phase_a(svo_batch *b) {
         d.pre = b->pre + mh.pre_off;
         d.base = b->base + mh.base_off;
         d.bstride = (mh.py.ctas + 3) & ~3u;
-        d.totals = totals + kMaxLevels * k;
+        d.any = any + k;
+        d.queue = counters;
+        d.out = b->out + k;
         d.done = done + k;
         d.py = mh.py;
         d.regions = mh.py.words[0] >= kRegionWords ? 1 : 0;
@@ -431,7 +482,7 @@ int batch_phase_a(svo_batch *b) {
     StageTimer tm((b->flags & SVO_FLAG_TIMINGS) != 0);
     for (int attempt = 0; attempt < 2; ++attempt) {
         tm.mark(StageTimer::kStart, st);
-        SVO_TRY(cudaMemsetAsync(b->meta, 0, ml.imm, st), "memset meta");
+        SVO_TRY(cudaMemsetAsync(meta, 0, ml.bytes, st), "memset meta");
         SVO_TRY(launch_front(bd, n == 1 ? &b->h_mesh[0] : nullptr, bblocks, ctas, any_regions, ctx->num_sms, st),
                 "bounding cube");
         tm.mark(StageTimer::kBbox, st);
@@ -443,20 +494,20 @@ int batch_phase_a(svo_batch *b) {
         SVO_TRY(launch_pyramid(bd, ctas, max_ctas, ctx->num_sms, st), "pyramid");
         tm.mark(StageTimer::kPyr, st);
         tm.mark(StageTimer::kScan, st);
-        std::vector<unsigned char> h(ml.imm);
-        SVO_TRY(cudaMemcpyAsync(h.data(), b->meta, ml.imm, cudaMemcpyDeviceToHost, st), "read meta");
         SVO_TRY(cudaStreamSynchronize(st), "count phase");
-        const uint32_t *hc = reinterpret_cast<const uint32_t *>(h.data() + ml.counters);
-        if (hc[0] > big_cap) {  // more big-triangle entries than the queue holds: grow it, redo
-            big_cap = hc[0];
+        b->pending = false;
+        if (b->out[0].queue > big_cap) {  // more big-triangle entries than the queue holds: grow it, redo
+            big_cap = b->out[0].queue;
             big = batch_alloc<uint4>(b, big_cap, err);
             if (!big) return cuda_fail(err, "big-triangle queue");
+            b->pending = true;
             continue;
         }
         for (int k = 0; k < n; ++k) {
             MeshHost &mh = b->m[b->live[k]];
-            std::memcpy(&mh.gp, h.data() + ml.gp + sizeof(GridParams) * k, sizeof(GridParams));
-            std::memcpy(mh.totals, h.data() + ml.totals + sizeof(uint32_t) * kMaxLevels * k, sizeof(mh.totals));
+            mh.gp = b->out[k].gp;
+            std::memcpy(mh.totals, b->out[k].totals, sizeof(mh.totals));
+            mh.top = b->out[k].any;
         }
         break;
     }
@@ -498,6 +549,7 @@ int batch_phase_a(svo_batch *b) {
             mesh_error(mh, SVO_ERR_CUDA, "octree levels did not converge");
             continue;
         }
+        mh.top >>= 3 * mh.T;  // every surface voxel lies under the top node
         for (int l = 0; l <= mh.T; ++l) {
             mh.n_l[l] = l < mh.T ? 8ull * mh.totals[l + 1] : 1ull;
             mh.off[l + 1] = mh.off[l] + mh.n_l[l];
@@ -568,6 +620,12 @@ T *arena_take(unsigned char *&at, uint64_t count) {
 #endif
 constexpr uint64_t kOwnEmitNodes = SVO_OWN_EMIT_NODES;
 
+// Meshes of up to this many level-0 words (res 256) have their surface-voxel
+// keys listed by the launch that lists the other levels; above, a launch of its
+// own visits the non-empty level-0 blocks only (k_compact_keys: at res 512 the
+// 2.1M words cost 12 us to look through, the launch 5 us).
+constexpr uint64_t kDirectKeyWords = 1ull << 18;
+
 // Phase B for meshes [first, first + count).
 int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *status_out) {
     svo::host::TraceRange trace("svo: emission wave (codes, nodes, vertices, edges, dedup)");
@@ -602,6 +660,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
         }
     };
     if (n > 0) {
+        b->pending = true;
         // The wave body: an error return from it still reaches the per-mesh
         // status loop below, which marks every mesh of the wave as failed.
         const int wave_rc = [&]() -> int {
@@ -675,7 +734,6 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
             std::vector<KeyJob> kjobs;
             std::vector<uint64_t> blk_off(1, 0);
             std::vector<EmitParams> ep(n);
-            std::vector<const uint64_t *> top_ptr(n);
             uint64_t ktot = 0;
             std::vector<uint64_t> kbase(n);
             for (int j = 0; j < n; ++j) {
@@ -691,17 +749,13 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 wbase[j] = wtot;
                 wtot += mh.py.woff[mh.T] + mh.py.words[mh.T] - mh.py.woff[1];
             }
-            // code lists, word ranks, duplicate counts, top codes: one block
+            // code lists, word ranks: one block
             Layout wl;
-            const size_t o_K = wl.add<uint64_t>(ktot + 1), o_WP = wl.add<uint32_t>(wtot + 1),
-                         o_dups = wl.add<unsigned long long>(2 * (size_t)n), o_top = wl.add<uint64_t>(n);
+            const size_t o_K = wl.add<uint64_t>(ktot + 1), o_WP = wl.add<uint32_t>(wtot + 1);
             unsigned char *wblk = S.get<unsigned char>(wl.bytes);
             if (!wblk) return cuda_fail(S.err, "wave scratch");
             uint64_t *K = reinterpret_cast<uint64_t *>(wblk + o_K);
             uint32_t *WP = reinterpret_cast<uint32_t *>(wblk + o_WP);
-            unsigned long long *dups = reinterpret_cast<unsigned long long *>(wblk + o_dups);
-            uint64_t *top = reinterpret_cast<uint64_t *>(wblk + o_top);
-            check(cudaMemsetAsync(dups, 0, 16 * (size_t)n, st), "memset");
             // one block for the output arrays of the whole wave
             size_t arena_bytes = 0;
             for (int j = 0; j < n; ++j) {
@@ -776,23 +830,27 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                     job.rflag = b->rflag + mh.cta0;
                     region_jobs.push_back(job);
                     region_counts.push_back(mh.py.ctas);
-                    job.l0 = 3;
                 }
-                jobs.push_back(job);
-                word_off.push_back(word_off.back() + mh.py.woff[mh.T] + mh.py.words[mh.T] - mh.py.woff[job.l0]);
-                if (want_keys && mh.T >= 3) {
+                if (want_keys && (mh.T < 3 || mh.py.words[0] <= kDirectKeyWords)) {
+                    job.l0 = 0;
+                    job.keys = r->keys;
+                } else if (want_keys) {
                     // the level-3 code list is the list of non-empty level-0 blocks
                     kjobs.push_back(KeyJob{md.bits, job.rank, job.out + job.koff[3], r->keys});
                     blk_off.push_back(blk_off.back() + mh.totals[3]);
-                } else if (want_keys) {
-                    CompactJob k0 = job;
-                    k0.l0 = 0;
-                    k0.l1 = 1;
-                    k0.out = r->keys;
-                    k0.wpre = nullptr;
-                    std::memset(k0.koff, 0, sizeof(k0.koff));
-                    jobs.push_back(k0);
-                    word_off.push_back(word_off.back() + mh.py.words[0]);
+                }
+                auto add_job = [&](int l0, int l1) {
+                    if (l0 >= l1) return;
+                    job.l0 = l0;
+                    job.l1 = l1;
+                    jobs.push_back(job);
+                    word_off.push_back(word_off.back() + mh.py.woff[l1 - 1] + mh.py.words[l1 - 1] - mh.py.woff[l0]);
+                };
+                if (job.rflag) {  // levels 1-2 have a launch of their own (region_jobs)
+                    if (job.l0 == 0) add_job(0, 1);
+                    add_job(3, mh.T + 1);
+                } else {
+                    add_job(job.l0, mh.T + 1);
                 }
                 // emission parameters
                 EmitParams &P = ep[j];
@@ -815,32 +873,49 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 P.nodes = r->nodes;
                 P.verts = ve ? r->verts : nullptr;
                 P.edges = ve ? r->edges : nullptr;
-                P.dups = dups + 2 * j;
-                top_ptr[j] = job.out + job.koff[mh.T];
+                P.dups = b->dups + 2 * dev_k[j];
+                P.dup_flag = &b->out[dev_k[j]].dup;
             }
             if (err != cudaSuccess) {
                 free_results();
                 drop_arena();
                 return cuda_fail(err, "output allocation");
             }
-            // the wave's job tables: one block, one upload
+            // Large meshes' emission launches of their own (parameters in the kernel's
+            // constant space); the rest share one launch over the mesh table.
+            std::vector<EmitParams> ep_small;
+            std::vector<uint64_t> off_small(1, 0);
+            int n_own = 0;
+            for (int j = 0; j < n; ++j) {
+                if (n == 1 || ep[j].N >= kOwnEmitNodes) {
+                    ++n_own;
+                } else {
+                    ep_small.push_back(ep[j]);
+                    off_small.push_back(off_small.back() + (ep[j].N + 31) / 32 * 32);
+                }
+            }
+            // the wave's tables: one block, one upload; what one kernel takes by
+            // value (a lone mesh's compaction job and emission) needs none
+            const bool lone_job = jobs.size() == 1;
             HostPack wt;
-            const size_t p_jobs = wt.add(jobs), p_woff = wt.add(word_off), p_kjobs = wt.add(kjobs),
-                         p_boff = wt.add(blk_off), p_top = wt.add(top_ptr);
-            unsigned char *dwt = S.get<unsigned char>(wt.buf.size());
-            CompactJob *d_jobs = dwt ? reinterpret_cast<CompactJob *>(dwt + p_jobs) : nullptr;
-            uint64_t *d_word_off = dwt ? reinterpret_cast<uint64_t *>(dwt + p_woff) : nullptr;
-            KeyJob *d_kjobs = (dwt && !kjobs.empty()) ? reinterpret_cast<KeyJob *>(dwt + p_kjobs) : nullptr;
-            uint64_t *d_blk_off = (dwt && !kjobs.empty()) ? reinterpret_cast<uint64_t *>(dwt + p_boff) : nullptr;
-            const uint64_t **d_top_ptr = dwt ? reinterpret_cast<const uint64_t **>(dwt + p_top) : nullptr;
+            const size_t p_jobs = lone_job ? 0 : wt.add(jobs), p_woff = lone_job ? 0 : wt.add(word_off),
+                         p_kjobs = wt.add(kjobs), p_boff = kjobs.empty() ? 0 : wt.add(blk_off),
+                         p_eps = wt.add(ep_small), p_offs = ep_small.empty() ? 0 : wt.add(off_small);
+            unsigned char *dwt = wt.buf.empty() ? nullptr : S.get<unsigned char>(wt.buf.size());
             if (S.err != cudaSuccess) {
                 free_results();
                 drop_arena();
                 return cuda_fail(S.err, "wave tables");
             }
-            check(cudaMemcpyAsync(dwt, wt.buf.data(), wt.buf.size(), cudaMemcpyHostToDevice, st), "upload");
+            const CompactJob *d_jobs = reinterpret_cast<const CompactJob *>(dwt + p_jobs);
+            const uint64_t *d_word_off = reinterpret_cast<const uint64_t *>(dwt + p_woff);
+            const KeyJob *d_kjobs = reinterpret_cast<const KeyJob *>(dwt + p_kjobs);
+            const uint64_t *d_blk_off = reinterpret_cast<const uint64_t *>(dwt + p_boff);
+            if (dwt) check(cudaMemcpyAsync(dwt, wt.buf.data(), wt.buf.size(), cudaMemcpyHostToDevice, st), "upload");
             tm.mark(StageTimer::kCompact0, st);
-            check(launch_compact(CompactBatch{d_jobs, (int)jobs.size(), d_word_off}, word_off.back(), st), "compact");
+            check(launch_compact(CompactBatch{d_jobs, (int)jobs.size(), d_word_off}, lone_job ? &jobs[0] : nullptr,
+                                 word_off.back(), st),
+                  "compact");
             for (size_t i = 0; i < region_jobs.size(); ++i)
                 check(launch_compact_regions(region_jobs[i], region_counts[i], ctx->num_sms, st), "compact");
             if (!kjobs.empty())
@@ -853,14 +928,8 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 check(cudaEventRecord(dset->fork, st), "fork");
                 check(cudaStreamWaitEvent(ds, dset->fork, 0), "fork");
             }
-            // Large meshes get launches of their own (parameters in the kernel's
-            // constant space); the rest share one launch over the mesh table.
-            // With two or more of them, they spread round-robin over the build
-            // stream and three more, so that one kernel's tail overlaps the next.
-            std::vector<EmitParams> ep_small;
-            std::vector<uint64_t> off_small(1, 0);
-            int n_own = 0;
-            for (int j = 0; j < n; ++j) n_own += (n == 1 || ep[j].N >= kOwnEmitNodes) ? 1 : 0;
+            // With two or more emission launches of their own, they spread round-robin
+            // over the build stream and three more, so that one kernel's tail overlaps the next.
             AuxStreams *aux = n_own >= 2 ? aux_acquire(ctx) : nullptr;
             if (aux) {
                 check(cudaEventRecord(aux->fork, st), "fork");
@@ -873,9 +942,6 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                     cudaStream_t es = lane == 0 ? st : aux->s[lane - 1];
                     ++k_own;
                     check(launch_emit(EmitBatch{nullptr, 1, nullptr}, &ep[j], ep[j].N, flags, ctx->num_sms, es), "emit");
-                } else {
-                    ep_small.push_back(ep[j]);
-                    off_small.push_back(off_small.back() + (ep[j].N + 31) / 32 * 32);
                 }
             }
             if (aux) {
@@ -885,25 +951,12 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 }
                 aux_release(ctx, aux);
             }
-            if (!ep_small.empty()) {
-                EmitParams *d_eps = S.get<EmitParams>(ep_small.size());
-                uint64_t *d_offs = S.get<uint64_t>(off_small.size());
-                if (S.err != cudaSuccess) {
-                    join_dedup();
-                    free_results();
-                    drop_arena();
-                    return cuda_fail(S.err, "wave tables");
-                }
-                check(upload(d_eps, ep_small, st), "upload");
-                check(upload(d_offs, off_small, st), "upload");
-                check(launch_emit(EmitBatch{d_eps, (int)ep_small.size(), d_offs}, nullptr, off_small.back(), flags,
-                                  ctx->num_sms, st),
+            if (!ep_small.empty())
+                check(launch_emit(EmitBatch{reinterpret_cast<const EmitParams *>(dwt + p_eps), (int)ep_small.size(),
+                                            reinterpret_cast<const uint64_t *>(dwt + p_offs)},
+                                  nullptr, off_small.back(), flags, ctx->num_sms, st),
                       "emit");
-            }
             tm.mark(StageTimer::kEmit, st);
-            // the top codes, gathered after the emission
-            k_gather_top<<<(n + 127) / 128, 128, 0, st>>>(d_top_ptr, n, top);
-            count_launches(1);
             // Dedup of every mesh on the forked stream (its host-side waits
             // overlap the emission running on the GPU); statuses are applied
             // after the emission's own checks.
@@ -918,22 +971,25 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 }
                 tm.mark(StageTimer::kDedup, ds);
             }
-            // read back the top codes and duplicate counts (pageable copies:
-            // these wait for the emission, so they come after the dedup launches)
-            std::vector<uint64_t> h_top(n);
-            std::vector<unsigned long long> h_dups(2 * n);
-            check(cudaMemcpyAsync(h_top.data(), top, 8 * (size_t)n, cudaMemcpyDeviceToHost, st), "read top");
-            check(cudaMemcpyAsync(h_dups.data(), dups, 16 * (size_t)n, cudaMemcpyDeviceToHost, st), "read dups");
+            join_dedup();
             check(cudaStreamSynchronize(st), "emit phase");
+            bool more = false;  // work launched after this wait
             for (int j = 0; j < n && rc == SVO_OK; ++j) {
                 MeshHost &mh = b->m[wave[j]];
                 svo_result *r = res[j];
-                if (mh.T == 0 || (h_top[j] & 7) != 0) {
+                if (mh.T == 0 || (mh.top & 7) != 0) {
                     mesh_error(mh, SVO_ERR_DEGENERATE,
                                "single top-level node with a non-zero octant: undefined in the reference");
                     continue;
                 }
-                if (ve && (h_dups[2 * j] || h_dups[2 * j + 1])) {
+                unsigned long long h_dups[2] = {0, 0};
+                if (ve && b->out[dev_k[j]].dup) {
+                    check(cudaMemcpyAsync(h_dups, b->dups + 2 * dev_k[j], sizeof(h_dups), cudaMemcpyDeviceToHost, st),
+                          "read dups");
+                    check(cudaStreamSynchronize(st), "read dups");
+                    more = true;
+                }
+                if (h_dups[0] || h_dups[1]) {
                     // consecutive duplicates (degenerate widths or absorbed
                     // coordinates): compact both arrays as thrust::unique does
                     const uint64_t nv = mh.N * 8, ne = mh.N * 12;
@@ -942,8 +998,8 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                     uint32_t *tc = U.get<uint32_t>(tiles), *tp = U.get<uint32_t>(tiles + 1);
                     unsigned long long *ss = U.get<unsigned long long>(scan_scratch_words(tiles));
                     uint32_t *ustat = U.get<uint32_t>(1);
-                    svo_vertex *v2 = h_dups[2 * j] ? pool_alloc<svo_vertex>(ctx->out_pool, st, nv, err) : nullptr;
-                    svo_edge *e2 = h_dups[2 * j + 1] ? pool_alloc<svo_edge>(ctx->out_pool, st, ne, err) : nullptr;
+                    svo_vertex *v2 = h_dups[0] ? pool_alloc<svo_vertex>(ctx->out_pool, st, nv, err) : nullptr;
+                    svo_edge *e2 = h_dups[1] ? pool_alloc<svo_edge>(ctx->out_pool, st, ne, err) : nullptr;
                     if (U.err != cudaSuccess || err != cudaSuccess) {
                         rc = cuda_fail(U.err != cudaSuccess ? U.err : err, "unique scratch");
                         break;
@@ -977,7 +1033,8 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 }
             }
             tm.mark(StageTimer::kUnique, st);
-            join_dedup();
+            if (more) check(cudaStreamSynchronize(st), "unique phase");
+            b->pending = rc != SVO_OK;
             for (int j = 0; j < n; ++j) {
                 MeshHost &mh = b->m[wave[j]];
                 if (mh.status == SVO_OK && drc[j] != SVO_OK) mesh_error(mh, drc[j], dmsg[j].c_str());
@@ -1027,6 +1084,14 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
     return first_err;
 }
 
+void batch_destroy(svo_batch *b) {
+    if (!b) return;
+    cudaSetDevice(b->ctx->device);
+    if (b->pending) cudaStreamSynchronize(b->st);
+    batch_release(b);  // stream-ordered frees
+    delete b;
+}
+
 // tune: the voxelizer split to use (null: the context's, read once here).
 int batch_create(svo_ctx *ctx, const svo_mesh_desc *descs, int n, uint32_t flags, cudaStream_t st,
                  svo_batch **out, const VoxTuning *tune = nullptr) {
@@ -1051,21 +1116,13 @@ int batch_create(svo_ctx *ctx, const svo_mesh_desc *descs, int n, uint32_t flags
     }
     const int rc = batch_phase_a(b);
     if (rc != SVO_OK) {
-        batch_release(b);
-        cudaStreamSynchronize(st);
-        delete b;
+        const std::string msg = g_err;
+        batch_destroy(b);
+        g_err = msg;
         return rc;
     }
     *out = b;
     return SVO_OK;
-}
-
-void batch_destroy(svo_batch *b) {
-    if (!b) return;
-    cudaSetDevice(b->ctx->device);
-    batch_release(b);
-    cudaStreamSynchronize(b->st);
-    delete b;
 }
 
 }  // namespace
@@ -1145,6 +1202,7 @@ void svo_ctx_destroy(svo_ctx *ctx) {
         cudaEventDestroy(a->fork);
         delete a;
     }
+    for (svo_ctx::Pinned &b : ctx->pinned_free) cudaFreeHost(b.p);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     if (ctx->out_pool) cudaMemPoolDestroy(ctx->out_pool);
     delete ctx;

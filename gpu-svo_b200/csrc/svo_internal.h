@@ -50,6 +50,17 @@ struct RankDev {
     uint32_t bstride;  // regions of the mesh rounded up to 4
 };
 
+// What the counting phase reports about one mesh, in pinned host memory that
+// the kernels write directly (no copy after the last kernel); dup is raised by
+// the emission.
+struct MeshOut {
+    GridParams gp;
+    uint32_t totals[kMaxLevels];  // set bits per level
+    uint64_t any;                 // the code of one surface voxel
+    uint32_t queue;               // entries the big-triangle queue needed (the same for all meshes of a batch)
+    uint32_t dup;                 // the emission met consecutive duplicates
+};
+
 // One mesh of a batch, as the kernels see it (an array in device memory).
 // A single build is a batch of one.
 struct MeshDev {
@@ -65,7 +76,9 @@ struct MeshDev {
     uint32_t *pre;           // block ranks (RankDev)
     uint32_t *base;          // region sums, then their prefixes (RankDev)
     uint32_t bstride;
-    uint32_t *totals;        // set bits per level (kMaxLevels)
+    uint64_t *any;           // the code of one surface voxel
+    const uint32_t *queue;   // big-triangle queue entries of the batch
+    MeshOut *out;            // pinned host memory (or device memory of a caller that copies it)
     uint32_t *done;          // pyramid regions finished
     Pyramid py;
 };
@@ -106,6 +119,7 @@ struct EmitParams {
     svo_vertex *verts;      // may be null (SVO_FLAG_NO_VERT_EDGE)
     svo_edge *edges;
     unsigned long long *dups;  // [0] vertex, [1] edge consecutive duplicates
+    uint32_t *dup_flag;        // pinned host memory: set to 1 with the first of them
 };
 
 // The meshes of one emission pass: mesh i owns global node slots
@@ -117,16 +131,17 @@ struct EmitBatch {
     const uint64_t *node_off;  // n + 1 entries
 };
 
-// One compaction job: the set bits of levels [l0, l1) of one mesh, level l
-// written to out + koff[l]; jobs own consecutive ranges of a global word
-// index (word_off, n + 1 entries).
+// One compaction job: the set bits of levels [l0, l1) of one mesh, level 0
+// written to keys, level l >= 1 to out + koff[l]; jobs own consecutive ranges
+// of a global word index (word_off, n + 1 entries).
 struct CompactJob {
     const uint64_t *bits;
     RankDev rank;
     Pyramid py;
     int l0, l1;
     uint64_t *out;
-    uint32_t *wpre;  // optional: rank at each non-empty word of levels >= 1 (indexed from woff[1])
+    uint64_t *keys;
+    uint32_t *wpre;  // rank at each non-empty word of levels >= 1 (indexed from woff[1])
     uint64_t koff[kMaxLevels];
     const uint8_t *rflag;  // region-mode mesh: its level-0 region flags (unflagged regions read as empty)
 };
@@ -210,7 +225,8 @@ cudaError_t launch_scan_stalled(const uint32_t *in, uint32_t *out, uint64_t n, u
 // Stream-ordered allocation from one of a context's pools: the one place a
 // build allocates device memory (svo_debug_fail_alloc injects failures here).
 cudaError_t pool_malloc(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t st);
-cudaError_t launch_compact(const CompactBatch &c, uint64_t total_words, cudaStream_t st);
+// one: the job of a one-job batch (host copy, passed by value), or null.
+cudaError_t launch_compact(const CompactBatch &c, const CompactJob *one, uint64_t total_words, cudaStream_t st);
 cudaError_t launch_compact_keys(const KeyBatch &k, uint64_t total_blocks, cudaStream_t st);
 // Levels 1 and 2 of a region-mode job (job.rflag set), one block per level-0 region.
 cudaError_t launch_compact_regions(const CompactJob &job, uint32_t regions, int num_sms, cudaStream_t st);

@@ -121,14 +121,13 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
     GridParams *gp = c.take<GridParams>(1);
     uint32_t *mm = c.take<uint32_t>(8);
     int32_t *imm = c.take<int32_t>(2);
-    uint32_t *totals = c.take<uint32_t>(kMaxLevels);
+    uint64_t *any = c.take<uint64_t>(1);
+    MeshOut *report = c.take<MeshOut>(1);
     uint32_t *counters = c.take<uint32_t>(4);
     uint32_t *done = c.take<uint32_t>(1);
     MeshDev *d_mesh = c.take<MeshDev>(1);
     uint64_t *d_tri_off = c.take<uint64_t>(2);
     uint32_t *d_cta_off = c.take<uint32_t>(2);
-    CompactJob *d_job = c.take<CompactJob>(1);
-    uint64_t *d_word_off = c.take<uint64_t>(2);
     uint64_t *bits = c.take<uint64_t>(py.total_words);
     uint32_t *pre = c.take<uint32_t>(py.total_blocks);
     const uint32_t bstride = (py.ctas + 3) & ~3u;
@@ -160,7 +159,9 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
     md.pre = pre;
     md.base = region_base;
     md.bstride = bstride;
-    md.totals = totals;
+    md.any = any;
+    md.queue = counters;
+    md.out = report;  // in the scratch array, copied below
     md.done = done;
     md.py = py;
     // everything that must start at zero (the array keeps the last call's data)
@@ -173,10 +174,10 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
                                    num_sms, st))))
         return rc;
     if ((rc = cuda(launch_pyramid(bd, py.ctas, py.ctas, num_sms, st)))) return rc;
-    uint32_t h_tot = 0, h_status = 0;
-    if ((rc = cuda(cudaMemcpyAsync(&h_tot, totals, 4, cudaMemcpyDeviceToHost, st)))) return rc;
-    if ((rc = cuda(cudaMemcpyAsync(&h_status, &gp->status, 4, cudaMemcpyDeviceToHost, st)))) return rc;
+    MeshOut h{};
+    if ((rc = cuda(cudaMemcpyAsync(&h, report, sizeof(h), cudaMemcpyDeviceToHost, st)))) return rc;
     if ((rc = cuda(cudaStreamSynchronize(st)))) return rc;
+    const uint32_t h_tot = h.totals[0], h_status = h.gp.status;
     if (h_status & kStatusNonFinite) return noalloc_fail(SVO_ERR_INVALID_ARGUMENT, "non-finite vertex coordinate");
     *n_keys = h_tot;
     if ((int64_t)h_tot > keys_cap) return noalloc_fail(SVO_ERR_INVALID_ARGUMENT, "keys buffer too small (see *n_keys)");
@@ -186,10 +187,7 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
     job.py = py;
     job.l0 = 0;
     job.l1 = 1;
-    job.out = keys;
-    const uint64_t h_word_off[2] = {0, py.words[0]};
-    if ((rc = cuda(cudaMemcpyAsync(d_job, &job, sizeof(job), cudaMemcpyHostToDevice, st)))) return rc;
-    if ((rc = cuda(cudaMemcpyAsync(d_word_off, h_word_off, sizeof(h_word_off), cudaMemcpyHostToDevice, st)))) return rc;
-    if ((rc = cuda(launch_compact(CompactBatch{d_job, 1, d_word_off}, py.words[0], st)))) return rc;
+    job.keys = keys;
+    if ((rc = cuda(launch_compact(CompactBatch{}, &job, py.words[0], st)))) return rc;
     return cuda(cudaStreamSynchronize(st));
 }

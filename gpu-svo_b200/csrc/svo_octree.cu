@@ -87,7 +87,7 @@ __device__ __forceinline__ uint32_t block_exscan(uint32_t v, uint32_t *s_warp, u
 }
 
 // The region sums of one of levels 0..3 (base + level * bstride) become their
-// exclusive prefixes in place; the sum goes to totals[level].  Padding past
+// exclusive prefixes in place; the sum goes to out->totals[level].  Padding past
 // the mesh's regions (up to the 16-byte stride) is treated as zero.
 template <int NT, int ITEMS>
 __device__ __forceinline__ void scan_regions(const MeshDev &md, int level, uint32_t *s_warp) {
@@ -126,7 +126,7 @@ __device__ __forceinline__ void scan_regions(const MeshDev &md, int level, uint3
                 reinterpret_cast<uint4 *>(a + i)[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
         carry += tot;
     }
-    if (threadIdx.x == 0) md.totals[level] = carry;
+    if (threadIdx.x == 0) md.out->totals[level] = carry;
 }
 
 // scan_regions of the four levels at once for a mesh of at most 4 NT regions:
@@ -149,18 +149,25 @@ __device__ __forceinline__ void scan_regions_all(const MeshDev &md, uint32_t *s_
         const uint32_t a = block_exscan<NT>(v[l].x + v[l].y + v[l].z + v[l].w, s_warp, tot);
         const uint32_t b = a + v[l].x, c = b + v[l].y, d = c + v[l].z;
         if (i < n) *reinterpret_cast<uint4 *>(md.base + (uint64_t)l * md.bstride + i) = make_uint4(a, b, c, d);
-        if (threadIdx.x == 0) md.totals[l] = tot;
+        if (threadIdx.x == 0) md.out->totals[l] = tot;
     }
 }
 
 // Levels 5.. of a mesh from its level 4, with the scanned block counts and the
-// totals of levels 4..  Levels of at most kTopWords words stay in shared
+// totals of levels 4.., and the rest of the mesh's report.  Levels of at most kTopWords words stay in shared
 // memory between the steps, so only the first step waits on global loads.
 constexpr uint32_t kTopWords = 512;
 
 template <int NT>
 __device__ __forceinline__ void finish_top(const MeshDev &md, uint64_t (*s_top)[kTopWords], uint32_t *s_warp) {
     const Pyramid &py = md.py;
+    if (threadIdx.x < sizeof(GridParams) / 4)  // every earlier kernel has left its status bits
+        reinterpret_cast<uint32_t *>(&md.out->gp)[threadIdx.x] =
+            __ldcg(reinterpret_cast<const uint32_t *>(md.gp) + threadIdx.x);
+    if (threadIdx.x == 32) {
+        md.out->any = __ldcg(reinterpret_cast<const unsigned long long *>(md.any));
+        md.out->queue = __ldcg(md.queue);
+    }
     bool held = false;  // level l is in s_top[l & 1]
     for (int l = 4; l < py.levels; ++l) {
         const uint64_t *in = md.bits + py.woff[l];
@@ -195,7 +202,7 @@ __device__ __forceinline__ void finish_top(const MeshDev &md, uint64_t (*s_top)[
             }
             carry += tot;
         }
-        if (threadIdx.x == 0) md.totals[l] = carry;
+        if (threadIdx.x == 0) md.out->totals[l] = carry;
         held = hold;
         __syncthreads();  // level l + 1 is complete (in shared memory, or in global memory for this block)
     }
@@ -247,17 +254,22 @@ __global__ void __launch_bounds__(256, FUSE ? 4 : 8) k_pyramid(BatchDev bd, uint
         } else {
             const uint4 *src = reinterpret_cast<const uint4 *>(bits + py.woff[0] + (uint64_t)b * 2048 + t * 8);
             uint64_t w1 = 0;
-            uint32_t c0 = 0;
+            uint32_t c0 = 0, first = 0;  // first: bit of the block
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const uint4 v = __ldcs(src + q);
                 const uint64_t a = ((uint64_t)v.y << 32) | v.x, c = ((uint64_t)v.w << 32) | v.z;
+                if (a) first = 128 * q + __ffsll((long long)a) - 1;
+                else if (c) first = 128 * q + 64 + __ffsll((long long)c) - 1;
                 c0 += __popcll(a) + __popcll(c);
                 w1 |= (uint64_t)nz_bytes(a) << (16 * q);
                 w1 |= (uint64_t)nz_bytes(c) << (16 * q + 8);
             }
             bits[py.woff[1] + (uint64_t)b * 256 + t] = w1;
             s1[t] = w1;
+            // one surface voxel of the mesh (any: the last store wins)
+            const uint32_t some = __ballot_sync(0xFFFFFFFFu, c0 != 0);
+            if (some && lane == __ffs(some) - 1) *md.any = ((uint64_t)b * 256 + t) * 512 + first;
             uint32_t sum0;
             pre[py.coff[0] + (uint64_t)b * 256 + t] = block_exscan<256>(c0, s_warp, sum0);  // s1 is complete after it
             if (warp == 0) {  // levels 2..4 of the region: one warp
@@ -571,8 +583,8 @@ __device__ __forceinline__ uint32_t block_rank(const RankDev &r, const Pyramid &
 // One thread per bitmap word; the 8 lanes of a 512-bit block are 8 aligned
 // lanes of a warp (every level and job starts on a block boundary), so a
 // word's rank in its level is the block's scanned base plus an 8-lane prefix
-// of popcounts.  Writes the sorted set-bit positions and, for levels >= 1
-// when wpre is given, the rank at each non-empty word (rank_of's table).
+// of popcounts.  Writes the sorted set-bit positions and, for levels >= 1,
+// the rank at each non-empty word (rank_of's table).
 // In a region-mode mesh a word of levels 0-3 lies inside one level-0 region
 // (level-l word w covers level-0 words w * 8^l ..): an unflagged one is
 // empty and is not read.
@@ -614,8 +626,8 @@ __device__ __forceinline__ void compact_word(const CompactJob &job, int l, uint6
     }
     const uint32_t r = r0 + x - pc;
     if (!v) return;
-    if (job.wpre && l >= 1) job.wpre[job.py.woff[l] - job.py.woff[1] + w] = r;
-    uint64_t *o = job.out + job.koff[l] + r;
+    if (l >= 1) job.wpre[job.py.woff[l] - job.py.woff[1] + w] = r;
+    uint64_t *o = (l == 0 ? job.keys : job.out + job.koff[l]) + r;
     const uint64_t b64 = w * 64;
     while (v) {
         *o++ = b64 + __ffsll((long long)v) - 1;
@@ -623,22 +635,25 @@ __device__ __forceinline__ void compact_word(const CompactJob &job, int l, uint6
     }
 }
 
-__global__ void __launch_bounds__(256) k_compact(CompactBatch cb, uint64_t total) {
+// ONE: a single job, passed by value (no upload of its table).
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_compact(CompactBatch cb, const __grid_constant__ CompactJob one,
+                                                 uint64_t total) {
     const uint64_t gi = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (gi >= ((total + 31) & ~31ull)) return;  // whole warps stay for the shuffles
     uint64_t v = 0, w = 0;
     int l = 0, j = 0;
     if (gi < total) {
-        j = find_segment(cb.word_off, cb.n, gi);
-        const CompactJob &job = cb.job[j];
+        if (!ONE) j = find_segment(cb.word_off, cb.n, gi);
+        const CompactJob &job = ONE ? one : cb.job[j];
         const Pyramid &py = job.py;
-        const uint64_t gw = py.woff[job.l0] + (gi - cb.word_off[j]);
+        const uint64_t gw = py.woff[job.l0] + (ONE ? gi : gi - cb.word_off[j]);
         l = job.l0;
         while (l + 1 < job.l1 && gw >= py.woff[l + 1]) ++l;
         w = gw - py.woff[l];
         v = (l <= 3 && job.rflag && !job.rflag[w >> (11 - 3 * l)]) ? 0ull : job.bits[gw];
     }
-    compact_word(cb.job[j], l, w, v);
+    compact_word(ONE ? one : cb.job[j], l, w, v);
 }
 
 // Levels 1 and 2 of a region-mode mesh, region by region (a block takes
@@ -650,7 +665,7 @@ __global__ void __launch_bounds__(256) k_compact_regions(const __grid_constant__
         if (!job.rflag[rg]) continue;
         const uint64_t w1 = (uint64_t)rg * 256 + threadIdx.x;
         compact_word(job, 1, w1, job.bits[job.py.woff[1] + w1]);
-        if (threadIdx.x < 32) {
+        if (threadIdx.x < 32 && job.l1 > 2) {  // a two-voxel octree's top is level 1
             const uint64_t w2 = (uint64_t)rg * 32 + threadIdx.x;
             compact_word(job, 2, w2, job.bits[job.py.woff[2] + w2]);
         }
@@ -1066,8 +1081,9 @@ __global__ void __launch_bounds__(kEmitWarps * 32, (FULL || ONE) ? 5 : 1)
             vdup += __shfl_xor_sync(0xFFFFFFFFu, vdup, d);
             edup += __shfl_xor_sync(0xFFFFFFFFu, edup, d);
         }
-        if (lane == 0 && vdup) atomicAdd(P.dups, vdup);
-        if (lane == 0 && edup) atomicAdd(P.dups + 1, edup);
+        // the first of them raises the host's flag: only then are the counters read back
+        if (lane == 0 && vdup && atomicAdd(P.dups, vdup) == 0) *P.dup_flag = 1;
+        if (lane == 0 && edup && atomicAdd(P.dups + 1, edup) == 0) *P.dup_flag = 1;
     }
 }
 
@@ -1193,9 +1209,11 @@ cudaError_t launch_scan_stalled(const uint32_t *in, uint32_t *out, uint64_t n, u
     return cudaGetLastError();
 }
 
-cudaError_t launch_compact(const CompactBatch &c, uint64_t total_words, cudaStream_t st) {
+cudaError_t launch_compact(const CompactBatch &c, const CompactJob *one, uint64_t total_words, cudaStream_t st) {
     if (total_words == 0) return cudaSuccess;
-    k_compact<<<(unsigned)((total_words + 255) / 256), 256, 0, st>>>(c, total_words);
+    const unsigned blocks = (unsigned)((total_words + 255) / 256);
+    if (one) k_compact<true><<<blocks, 256, 0, st>>>(c, *one, total_words);
+    else k_compact<false><<<blocks, 256, 0, st>>>(c, CompactJob{}, total_words);
     count_launches(1);
     return cudaGetLastError();
 }
