@@ -426,7 +426,7 @@ int batch_phase_a(svo_batch *b) {
     Layout lay;
     const size_t o_meta = lay.add<unsigned char>(ml.bytes);
     const size_t o_bits = lay.add<uint64_t>(words), o_pre = lay.add<uint32_t>(blocks), o_base = lay.add<uint32_t>(bases),
-                 o_big = lay.add<uint4>(big_cap), o_small = lay.add<uint64_t>(std::max<uint64_t>(tris, 1)),
+                 o_big = lay.add<uint4>(big_cap),
                  o_rflag = lay.add<uint8_t>(std::max<uint32_t>(ctas, 1));
     const size_t o_tables = lay.add<unsigned char>(t_bytes);
     unsigned char *blk = batch_alloc<unsigned char>(b, lay.bytes, err);
@@ -435,7 +435,6 @@ int batch_phase_a(svo_batch *b) {
     b->pre = reinterpret_cast<uint32_t *>(blk + o_pre);
     b->base = reinterpret_cast<uint32_t *>(blk + o_base);
     uint4 *big = reinterpret_cast<uint4 *>(blk + o_big);
-    uint64_t *small = reinterpret_cast<uint64_t *>(blk + o_small);
     uint8_t *rflag = b->rflag = blk + o_rflag;
     unsigned char *meta = blk + o_meta;
     GridParams *gp = reinterpret_cast<GridParams *>(meta + ml.gp);
@@ -487,8 +486,7 @@ int batch_phase_a(svo_batch *b) {
                 "bounding cube");
         tm.mark(StageTimer::kBbox, st);
         if (any_regions) SVO_TRY(launch_regions(bd, (int64_t)tris, ctas, ctx->num_sms, st), "zero regions");
-        SVO_TRY(launch_voxelize(bd, (int64_t)tris, strict, b->tune, big, big_cap, counters, ctx->num_sms, st,
-                                small),
+        SVO_TRY(launch_voxelize(bd, (int64_t)tris, strict, b->tune, big, big_cap, counters, ctx->num_sms, st),
                 "voxelize");
         tm.mark(StageTimer::kVox, st);
         SVO_TRY(launch_pyramid(bd, ctas, max_ctas, ctx->num_sms, st), "pyramid");
@@ -1376,19 +1374,14 @@ int svo_ctx_autotune(svo_ctx *ctx, const svo_mesh_desc *descs, int n, uint32_t f
         }
         return SVO_OK;
     };
-    VoxTuning cur = saved, win = saved;
-    cur.split = 0;
+    VoxTuning win = saved;
     float best_ms = 1e30f;
     int rc = SVO_OK;
-    // stage 1: the serial / small-triangle thresholds and the serial tier's
-    // layout; stage 2: queue entry size
-    for (uint32_t sm : {32u, 64u, 128u, 256u}) {
-        for (uint32_t cand = 0; cand < 6; ++cand) {
-            VoxTuning t = cur;
+    for (uint32_t sm : {16u, 32u, 64u, 128u}) {
+        for (uint32_t wm : {64u, 128u, 256u, 512u, 1024u}) {
+            VoxTuning t = saved;
             t.serial_max = sm;
-            t.inplace_max = cand % 3 == 0 ? 16u : cand % 3 == 1 ? 32u : 64u;
-            t.serial_packed = cand / 3;
-            t.warp_max = 256;
+            t.warp_max = wm;
             float ms = 0.0f;
             if ((rc = measure(t, ms)) != SVO_OK) break;
             if (ms < best_ms) {
@@ -1397,17 +1390,6 @@ int svo_ctx_autotune(svo_ctx *ctx, const svo_mesh_desc *descs, int n, uint32_t f
             }
         }
         if (rc != SVO_OK) break;
-    }
-    for (uint32_t wm : {64u, 128u, 512u, 1024u}) {
-        if (rc != SVO_OK) break;
-        VoxTuning t = win;
-        t.warp_max = wm;
-        float ms = 0.0f;
-        if ((rc = measure(t, ms)) != SVO_OK) break;
-        if (ms < best_ms) {
-            best_ms = ms;
-            win = t;
-        }
     }
     if (rc != SVO_OK) return rc;
     {

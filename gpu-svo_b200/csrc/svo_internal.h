@@ -15,13 +15,14 @@ void count_launches(int n);
 constexpr int kMaxLevels = 24;
 constexpr int kMaxRes = 2048;
 
-// Voxelizer work split.
+// Voxelizer work split (svo_tuning; split, inplace_max and serial_packed have
+// no effect).
 struct VoxTuning {
-    uint32_t serial_max = 64;    // grid-bbox voxels tested by one thread, row by row
-    uint32_t warp_max = 256;     // 4x4x4 bricks per queue entry (one warp walks one entry)
-    uint32_t split = 0;          // cull 2x2x2 sub-bricks of surviving bricks too
-    uint32_t inplace_max = 32;   // bricks of a triangle walked by the warp that set it up
-    uint32_t serial_packed = 0;  // serial tier: rows packed across the warp's lanes (else one triangle per lane)
+    uint32_t serial_max = 64;  // most grid-bbox voxels of a triangle tested by one thread
+    uint32_t warp_max = 256;   // queue entries hold a sixteenth as many brick columns
+    uint32_t split = 0;
+    uint32_t inplace_max = 32;
+    uint32_t serial_packed = 0;
 };
 
 // Occupancy bitmap pyramid: level 0 is the voxel grid (one bit per Morton
@@ -195,12 +196,11 @@ struct IndexJob {
 uint32_t index_blocks(int64_t n);
 cudaError_t launch_index_ranges(const IndexJob *jobs, int n, const uint32_t *block_off, uint32_t total_blocks,
                                 int32_t *mm, cudaStream_t st);
-// counters: 4 zeroed u32 (queue entries, queue cursor, -, small-list length); small:
-// room for one u64 per triangle, or null (then no in-warp tier unless big is
-// null too, which walks every large triangle in the warp that set it up).
+// counters: 2 zeroed u32 (queue entries, queue cursor); big: the queue of
+// large triangles, or null: every large triangle is walked by the warp that
+// set it up.
 cudaError_t launch_voxelize(const BatchDev &b, int64_t total_tris, bool strict, const VoxTuning &tune,
-                            uint4 *big, uint32_t big_cap, uint32_t *counters, int num_sms, cudaStream_t st,
-                            uint64_t *small = nullptr);
+                            uint4 *big, uint32_t big_cap, uint32_t *counters, int num_sms, cudaStream_t st);
 // Builds levels 1.. of every mesh's pyramid, the block ranks and the level
 // totals; max_ctas: the most regions of any mesh (py.ctas).  done must be zero.
 cudaError_t launch_pyramid(const BatchDev &b, uint32_t total_ctas, uint32_t max_ctas, int num_sms, cudaStream_t st);

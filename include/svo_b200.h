@@ -102,19 +102,18 @@ int svo_ctx_reserve(svo_ctx *ctx, uint64_t result_bytes, uint64_t scratch_bytes,
  * reference. */
 int svo_ctx_memory(const svo_ctx *ctx, uint64_t *scratch_used, uint64_t *result_used);
 
-/* Voxelizer work split: triangles whose grid bbox has at most serial_max
- * (<= 65536) voxels are tested row by row without culling, the rows of a
- * warp's such triangles handed out one row per lane per round
- * (serial_packed = 1) or one triangle per lane (0, the default); triangles of at most inplace_max 4x4x4
- * bricks are walked by the warp that set them up, packed 32 bricks per round
- * across the warp's triangles; larger ones are cut into queue entries of at
- * most warp_max bricks, one warp per entry.  Results do not depend on these
- * values, only the speed.  No counterpart in the reference (one thread per
- * triangle there, src/SVO.cu:37-188). */
+/* Voxelizer work split: a triangle whose grid bbox has at most serial_max
+ * (<= 65536) voxels, and at most 4 x 4 x 8 of them, is tested whole by one
+ * thread; a larger one is cut into queue entries of at most warp_max / 16
+ * columns of 4x4x4 bricks, which warps take several at a time.  split,
+ * inplace_max and serial_packed (0 or 1) are accepted and have no effect: they
+ * chose between layouts that are gone.  Results do not depend on these values,
+ * only the speed.  No counterpart in the reference (one thread per triangle
+ * there, src/SVO.cu:37-188). */
 typedef struct svo_tuning {
     uint32_t serial_max;
     uint32_t warp_max;
-    uint32_t split; /* also cull the 2x2x2 sub-bricks of surviving bricks (queue tier) */
+    uint32_t split;
     uint32_t inplace_max;
     uint32_t serial_packed;
 } svo_tuning;
@@ -179,7 +178,7 @@ int svo_build_batch(svo_ctx *ctx, const svo_mesh_desc *descs, int n, void *strea
                     svo_result **out, int *status_out);
 
 /* Autotuner for the work split: runs the counting phase of the sample meshes
- * (a batch, as svo_batch_create) for a grid of candidate splits, times the
+ * (a batch, as svo_batch_create) for a grid of serial_max and warp_max values, times the
  * voxelizer stage on the device, installs the fastest split in the context
  * and returns it in *best (may be null).  Results do not depend on the split.
  * Builds that other threads run on the context meanwhile keep its previous
