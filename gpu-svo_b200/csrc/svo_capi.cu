@@ -693,7 +693,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                     bits[l] = md.bits + mh.py.woff[l];
                     sides[l] = std::max<uint32_t>(1u, R >> l);
                 }
-                drc[j] = dedup_begin(ctx->pool, ds, mh.T, bits, sides, ctx->num_sms, &druns[j]);
+                drc[j] = dedup_begin(ctx->pool, ds, mh.T, bits, sides, ctx->num_sms, b->out[dev_k[j]].dedup, &druns[j]);
                 if (drc[j] != SVO_OK) dmsg[j] = svo_last_error();
             };
             struct DedupGuard {  // on every exit: unfinished runs freed, the dedup stream joined

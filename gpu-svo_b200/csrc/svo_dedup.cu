@@ -17,7 +17,8 @@
 //      lattice points 2Q + r): the corners of the nodes of levels >= 1 --
 //      every level-0 corner is also a corner of a level-1 node.  The
 //      level-1 corners come word by word from the level-2 bitmap
-//      (k_dedup_build), the coarser levels' by marking their node groups;
+//      (k_dedup_build), the coarser levels' by marking their node groups
+//      (k_dedup_mark);
 //   2. walk D's words in order and derive, per Q, what its 8 points need
 //      from the parent bitmaps (coarser levels only for r = 0), for the 64 Q
 //      of a word at once by shifts of whole bitmap words; pack it into one
@@ -53,96 +54,64 @@ struct DedupParams {
     int T;                      // top level
     const uint64_t *root;       // device: the root's code
     DedupLevel lv[kMaxLevels];
-    uint32_t gstart[kMaxLevels + 1];  // marking threads of levels 1..T-1 (prefix of groups)
+    uint32_t gstart[kMaxLevels + 1];  // first marked group of levels 2..T-1 (prefix of groups)
     uint32_t *D;                // candidate bitmap over Q (u32 view)
     uint32_t *G;                // one bit per chunk of D
     uint64_t chunks;
     const uint32_t *list;       // the touched chunks (a set bit in G), in order
     uint64_t ntouched;
-    unsigned long long *nq;     // set bits of D (counted while marking)
-    uint32_t *qn;               // [ntouched] set bits per touched chunk
-    const uint32_t *qpre;       // [ntouched + 1] their prefix: the first state of each chunk
+    const uint32_t *qpre;       // [ntouched] the first state of each touched chunk
     uint64_t *qs;               // one state per set bit of D, in order
     uint64_t ntiles;            // tiles of 32 consecutive states
     uint32_t *tcnt;             // [3][ntiles] keys per tile and kind
-    const uint32_t *tpre;       // [3][ntiles + 1] their prefixes
+    const uint32_t *tpre;       // [3 ntiles + 1] their prefix over all kinds
     uint64_t *out[3];
-    const struct DedupTables *tables;  // built once per dedup by k_dedup_tables
 };
 
-// Adds the block's sum of v (each thread's share) to *dst with one atomic.
-// All threads of the block call.
-__device__ __forceinline__ void block_add(unsigned long long *dst, uint32_t v) {
-    __shared__ uint32_t part[32];
-    v = __reduce_add_sync(0xFFFFFFFFu, v);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        uint32_t s = threadIdx.x < (blockDim.x >> 5) ? part[threadIdx.x] : 0u;
-        s = __reduce_add_sync(0xFFFFFFFFu, s);
-        if (threadIdx.x == 0 && s) atomicAdd(dst, (unsigned long long)s);
-    }
-}
-
-__device__ __forceinline__ void mark_chunk(const DedupParams &p, uint64_t bit) {
+// Sets bit `bit` of D and its chunk's bit of G.  Most corners are shared by
+// several groups: a look first spares the atomic (a stale look only costs it).
+__device__ __forceinline__ void mark_bit(const DedupParams &p, uint64_t bit) {
+    uint32_t *w = p.D + (bit >> 5);
+    const uint32_t m = 1u << (bit & 31);
+    if (*(volatile uint32_t *)w & m) return;
+    atomicOr(w, m);
     const uint64_t ch = bit >> 11;
     uint32_t *g = p.G + (ch >> 5);
-    const uint32_t m = 1u << (ch & 31);
-    if (!(*(volatile uint32_t *)g & m)) atomicOr(g, m);
+    const uint32_t gm = 1u << (ch & 31);
+    if (!(*(volatile uint32_t *)g & gm)) atomicOr(g, gm);
 }
 
-// Returns 1 when the bit was not set before.
-__device__ __forceinline__ uint32_t mark_bit(const DedupParams &p, uint64_t bit) {
-    const uint32_t m = 1u << (bit & 31);
-    const uint32_t old = atomicOr(p.D + (bit >> 5), m);
-    mark_chunk(p, bit);
-    return (old & m) ? 0u : 1u;
-}
-
-// Marks the Q of every corner of every node at levels >= 1.
-//   level 1, group g (a level-2 code): nodes 2g + {0,1}^3, corners
-//     Q = 2g + {0,1,2}^3, i.e. for each e in {0,1}^3 the byte morton(g + e)
-//     of D gets the sub-points k' with k'_i = 0 wherever e_i = 1;
-//   level l >= 2: Q = (2g + {0,1,2}^3) << (l - 1), one bit each;
-//   the root (level T): Q = (root + {0,1}^3) << (T - 1).
-//   Also counts the bits it sets first (*p.nq: the set bits of D).  Threads
-//   from `first` on (first = gstart[2] when k_dedup_build did level 1).
-__global__ void k_dedup_mark(const __grid_constant__ DedupParams p, uint32_t first, uint32_t total) {
-    uint32_t fresh = 0;
-    for (uint32_t t = first + blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        if (t == total - 1) {
-            const uint64_t rc = *p.root;
-            const uint32_t r[3] = {compact3(rc), compact3(rc >> 1), compact3(rc >> 2)};
-            const int sh = p.T - 1;
-            for (int d = 0; d < 8; ++d)
-                fresh += mark_bit(p, morton3((r[0] + (d & 1)) << sh, (r[1] + ((d >> 1) & 1)) << sh,
-                                             (r[2] + ((d >> 2) & 1)) << sh));
-            continue;
-        }
-        int l = 1;
-        while (l + 1 < p.T && t >= p.gstart[l + 1]) ++l;
-        const uint64_t gc = p.lv[l].K1[t - p.gstart[l]];
-        const uint32_t g[3] = {compact3(gc), compact3(gc >> 1), compact3(gc >> 2)};
-        if (l == 1) {
-            for (int e = 0; e < 8; ++e) {
-                const uint64_t byte = morton3(g[0] + (e & 1), g[1] + ((e >> 1) & 1), g[2] + ((e >> 2) & 1));
-                uint32_t m = 0xFFu;
-                if (e & 1) m &= 0x55u;
-                if (e & 2) m &= 0x33u;
-                if (e & 4) m &= 0x0Fu;
-                m <<= 8 * (byte & 3);
-                fresh += __popc(m & ~atomicOr(p.D + (byte >> 2), m));
-                mark_chunk(p, byte << 3);
-            }
-        } else {
-            const int sh = l - 1;
-            for (int k = 0; k < 27; ++k) {
-                const uint32_t kx = k % 3, ky = (k / 3) % 3, kz = k / 9;
-                fresh += mark_bit(p, morton3((2 * g[0] + kx) << sh, (2 * g[1] + ky) << sh, (2 * g[2] + kz) << sh));
-            }
-        }
+// Marks the Q of every corner of the nodes at levels >= 2, a corner per
+// thread:
+//   level l, group g (a level l + 1 code): nodes 2g + {0,1}^3, corners
+//     Q = (2g + {0,1,2}^3) << (l - 1): 27 threads;
+//   the root (level T): Q = (root + {0,1}^3) << (T - 1): 8 threads.
+// (One thread per group, its 27 marks one after another, took 45 us for the
+// 21,000 groups of an 80k-triangle icosphere at res 200: a chain of 27 atomic
+// round trips.)
+__global__ void __launch_bounds__(256) k_dedup_mark(const __grid_constant__ DedupParams p, uint32_t groups) {
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 27ull * groups + 8) return;
+    if (t >= 27ull * groups) {
+        const uint32_t d = (uint32_t)(t - 27ull * groups);
+        const uint64_t rc = *p.root;
+        mark_bit(p, morton3(compact3(rc) + (d & 1), compact3(rc >> 1) + ((d >> 1) & 1), compact3(rc >> 2) + ((d >> 2) & 1))
+                        << (3 * (p.T - 1)));
+        return;
     }
-    block_add(p.nq, fresh);
+    const uint32_t i = (uint32_t)(t / 27), k = (uint32_t)(t - 27ull * i);
+    int l = 2;
+    while (l + 1 < p.T && i >= p.gstart[l + 1]) ++l;
+    const uint64_t gc = p.lv[l].K1[i - p.gstart[l]];
+    const uint32_t kk[3] = {k % 3, (k / 3) % 3, k / 9};
+    const uint64_t mask[3] = {kDilX, kDilY, kDilZ};
+    uint64_t q = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {  // dilated 2g, 2g + 1 or 2g + 2
+        const uint64_t g = gc & mask[a];
+        q |= ((kk[a] == 2 ? dil_inc(g, mask[a]) : g) << 3) | (kk[a] == 1 ? 1ull << a : 0ull);
+    }
+    mark_bit(p, q << (3 * (l - 1)));
 }
 
 // Bit e of the result: cell v - e exists at the level whose occupancy bitmap
@@ -195,50 +164,52 @@ struct alignas(16) DedupTables {
     uint32_t e0[256], f0[256];
 };
 
-__device__ void init_tables(DedupTables &t) {
-    for (int i = threadIdx.x; i < 2048; i += blockDim.x) {
+constexpr uint32_t bits_of(uint32_t v) {
+    uint32_t n = 0;
+    for (; v; v &= v - 1) ++n;
+    return n;
+}
+
+constexpr DedupTables make_tables() {
+    DedupTables t{};
+    for (uint32_t i = 0; i < 2048; ++i) {
         const uint32_t E = i >> 3, s = i & 7;
         uint32_t ex = 0;
-        for (int d = 0; d < 8; ++d) ex |= ((E >> (d & ~s & 7)) & 1u) << d;
+        for (uint32_t d = 0; d < 8; ++d) ex |= ((E >> (d & ~s & 7)) & 1u) << d;
         t.around[i] = (uint8_t)ex;
     }
-    for (int ex = threadIdx.x; ex < 256; ex += blockDim.x) {
+    for (uint32_t ex = 0; ex < 256; ++ex) {
         uint32_t k = ex != 0;
         k |= (uint32_t)((ex & 0x55) != 0) << 1 | (uint32_t)((ex & 0x33) != 0) << 2 | (uint32_t)((ex & 0x0F) != 0) << 3;
         k |= (uint32_t)((ex & 0x03) != 0) << 4 | (uint32_t)((ex & 0x05) != 0) << 5 | (uint32_t)((ex & 0x11) != 0) << 6;
         t.kinds[ex] = (uint8_t)k;
     }
-    __syncthreads();
-    for (int E = threadIdx.x; E < 256; E += blockDim.x) {
-        uint32_t v = 0, e = 0, f = 0;
-        for (int r = 0; r < 8; ++r) {
+    for (uint32_t E = 0; E < 256; ++E) {
+        uint32_t v = 0, e = 0, f = 0, vm = 0, em = 0, fm = 0;
+        for (uint32_t r = 0; r < 8; ++r) {
             const uint32_t k = t.kinds[t.around[E * 8 + r]];
+            const uint32_t at = r == 0 ? 0 : 9 + 3 * (r - 1);
             v += k & 1;
-            e += __popc((k >> 1) & 7);
-            f += __popc((k >> 4) & 7);
-        }
-        t.cnt0[E] = v | e << 8 | f << 16;
-        uint32_t vm = 0, em = 0, fm = 0;
-        for (int r = 0; r < 8; ++r) {
-            const uint32_t k = t.kinds[t.around[E * 8 + r]];
-            const int at = r == 0 ? 0 : 9 + 3 * (r - 1);
+            e += bits_of((k >> 1) & 7);
+            f += bits_of((k >> 4) & 7);
             vm |= (k & 1u) << r;
             em |= ((k >> 1) & 7u) << at;
             fm |= ((k >> 4) & 7u) << at;
         }
+        t.cnt0[E] = v | e << 8 | f << 16;
         t.v0[E] = (uint8_t)vm;
         t.e0[E] = em;
         t.f0[E] = fm;
     }
-    __syncthreads();
+    return t;
 }
 
-// The tables of one dedup, built by one block into global memory; the state
-// and write passes copy them into shared memory.
-__global__ void __launch_bounds__(256) k_dedup_tables(DedupTables *t) { init_tables(*t); }
+// Computed at compile time; the state and write passes copy them into shared
+// memory.
+__device__ const DedupTables kTables = make_tables();
 
-__device__ __forceinline__ void load_tables(DedupTables &sh, const DedupTables *g) {
-    const uint4 *src = reinterpret_cast<const uint4 *>(g);
+__device__ __forceinline__ void load_tables(DedupTables &sh) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(&kTables);
     uint4 *dst = reinterpret_cast<uint4 *>(&sh);
     for (int i = threadIdx.x; i < (int)(sizeof(DedupTables) / 16); i += blockDim.x) dst[i] = src[i];
     __syncthreads();
@@ -391,7 +362,7 @@ __global__ void __launch_bounds__(kStateWarps * 32) k_dedup_state(const __grid_c
     __shared__ uint32_t wdeep[kStateWarps][kChunkWords];  // E2 | deep key counts of Q_0 (packed as below)
     __shared__ uint64_t sx[kMaxLevels];  // dilated side of each level
     if (threadIdx.x < kMaxLevels) sx[threadIdx.x] = (int)threadIdx.x <= p.T ? spread3(p.lv[threadIdx.x].side) : 0;
-    load_tables(tb, p.tables);
+    load_tables(tb);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t nwarps = (uint64_t)gridDim.x * kStateWarps;
     const uint64_t root = *p.root;
@@ -569,7 +540,7 @@ __global__ void __launch_bounds__(kDedupWarps * 32) k_dedup_write(const __grid_c
     __shared__ uint16_t stage[kDedupWarps][kStageKeys];
     __shared__ uint64_t sx[kMaxLevels];
     if (threadIdx.x < kMaxLevels) sx[threadIdx.x] = (int)threadIdx.x <= p.T ? spread3(p.lv[threadIdx.x].side) : 0;
-    load_tables(tb, p.tables);
+    load_tables(tb);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t nwarps = (uint64_t)gridDim.x * kDedupWarps;
     const uint64_t root = *p.root;
@@ -591,60 +562,42 @@ __global__ void __launch_bounds__(kDedupWarps * 32) k_dedup_write(const __grid_c
             if (lane >= d) x += y;
         }
         const uint32_t tot = __shfl_sync(0xFFFFFFFFu, x, 31), ex = x - c;
+        // (the prefix runs through all kinds; differences are exact modulo 2^32)
         emit_kind<0>(p.out[0], p.tpre[t], m.v, 0u, qc, stg, lane, ex & 0x1FFu, tot & 0x1FFu);
-        emit_kind<1>(p.out[1], p.tpre[(p.ntiles + 1) + t], m.el, m.eh, qc, stg, lane, (ex >> 9) & 0x7FFu,
+        emit_kind<1>(p.out[1], p.tpre[p.ntiles + t] - p.tpre[p.ntiles], m.el, m.eh, qc, stg, lane, (ex >> 9) & 0x7FFu,
                      (tot >> 9) & 0x7FFu);
-        emit_kind<2>(p.out[2], p.tpre[2 * (p.ntiles + 1) + t], m.fl, m.fh, qc, stg, lane, ex >> 20, tot >> 20);
+        emit_kind<2>(p.out[2], p.tpre[2 * p.ntiles + t] - p.tpre[2 * p.ntiles], m.fl, m.fh, qc, stg, lane, ex >> 20,
+                     tot >> 20);
     }
 }
 
-// Set bits per touched chunk (one warp per chunk).
-__global__ void k_chunk_bits(const __grid_constant__ DedupParams p) {
-    const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= p.ntouched) return;
-    const uint64_t *D64 = reinterpret_cast<const uint64_t *>(p.D);
-    const uint32_t n = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)__popcll(D64[(uint64_t)p.list[w] * kChunkWords + lane]));
-    if (lane == 0) p.qn[w] = n;
-}
-
-// Zeroes the 2048-word regions of D that can hold a candidate: every lattice
-// cell Q has coordinates <= side / 2 (corners of the grid's cells), and a
-// region -- an aligned box of 64 x 64 x 32 Q -- holds one iff its lowest
-// corner does.  At side 2048 that is 9,537 of 65,536 regions; only the
-// touched chunks of D are read later, all inside these.
-__global__ void __launch_bounds__(256) k_dedup_zero(uint64_t *__restrict__ D, uint64_t regions, uint32_t half) {
-    for (uint64_t b = blockIdx.x; b < regions; b += gridDim.x) {
-        const uint64_t c = b << 17;
-        if (compact3(c) > half || compact3(c >> 1) > half || compact3(c >> 2) > half) continue;
-        uint4 *w = reinterpret_cast<uint4 *>(D + b * 2048);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) w[threadIdx.x + 256 * q] = make_uint4(0, 0, 0, 0);
-    }
-}
-
-// The level-1 part of D, word by word over the same regions: bit Q is set
-// iff some level-1 node has corner Q, i.e. a level-1 cell Q - d (d in
+// The level-1 part of D, word by word over the regions that can hold a
+// candidate: every lattice cell Q has coordinates <= side / 2 (corners of the
+// grid's cells), and a region of 2048 words -- an aligned box of 64 x 64 x 32
+// Q -- holds one iff its lowest corner does.  At side 2048 that is 9,537 of
+// 65,536 regions; only the touched chunks of D are read later, all inside
+// these.  Bit Q is set iff some level-1 node has corner Q, i.e. a level-1 cell Q - d (d in
 // {0,1}^3) exists -- its level-2 parent is occupied.  The level-2 bytes
 // above the blocks b - d, upsampled to level-1 cells, dilated by one cell
 // along each axis (separable: 7 shifts).  Every word of a region is
 // written, zeros included, so D needs no zeroing; G gets every chunk with a
-// set bit and *p.nq the set bits.  Needs T >= 2 (the level-2 bitmap).
+// set bit.  With T < 2 (no level-2 bitmap) the root's corners are all there
+// is: D is only cleared.
 // Most words lie far from every node: a region (64 x 64 x 32 Q) whose
 // level-7 cells c - e (c = its origin >> 6, e in {0,1}^3: they hold every
 // level-2 parent of the cells Q - d it needs) are all empty is only
 // zeroed, and so is a warp's chunk (16 x 16 x 8 Q) whose level-5 cells
 // c - e (c = its origin >> 4) are empty.
-__global__ void __launch_bounds__(256) k_dedup_build(const __grid_constant__ DedupParams p, uint64_t regions,
+__global__ void __launch_bounds__(256) k_dedup_build(const __grid_constant__ DedupParams p, uint64_t words,
                                                      uint32_t half) {
+    const uint64_t regions = (words + 2047) / 2048;  // a grid of side 32 or less has part of one
     const int lane = threadIdx.x & 31;
-    const uint32_t s2 = p.lv[2].side;
+    const int T = p.T;
+    const uint32_t s2 = T >= 2 ? p.lv[2].side : 0u;
     const uint64_t nb2 = spread3((s2 + 1) / 2), valid2 = s2 >= 2 ? 0xFFull : 0x1ull;
     const uint64_t *bits2 = p.lv[2].bits;
-    const int T = p.T;
     const uint64_t sx5 = T >= 5 ? spread3(p.lv[5].side) : 0, sx7 = T >= 7 ? spread3(p.lv[7].side) : 0;
     uint64_t *D64 = reinterpret_cast<uint64_t *>(p.D);
-    uint32_t cnt = 0;
     for (uint64_t r = blockIdx.x; r < regions; r += gridDim.x) {
         const uint64_t c = r << 17;  // the region's first Q
         if (compact3(c) > half || compact3(c >> 1) > half || compact3(c >> 2) > half) continue;
@@ -657,6 +610,7 @@ __global__ void __launch_bounds__(256) k_dedup_build(const __grid_constant__ Ded
         }
         for (int k = 0; k < 8; ++k) {
             const uint64_t bc = r * 2048 + k * 256 + threadIdx.x;  // word = block code
+            if (bc >= words) continue;  // whole warps: words is a multiple of 32
             if (T >= 5) {
                 const uint64_t c5 = ((bc & ~31ull) << 6) >> 12;  // the chunk's origin at level 5
                 const uint32_t near5 = lane < 8 ? cell_bit(p.lv[5].bits, c5, sx5, lane) : 0u;
@@ -687,29 +641,72 @@ __global__ void __launch_bounds__(256) k_dedup_build(const __grid_constant__ Ded
             D64[bc] = w;
             const uint32_t any = __ballot_sync(0xFFFFFFFFu, w != 0);  // the warp's 32 words: one chunk
             if (lane == 0 && any) atomicOr(p.G + (bc >> 10), 1u << ((bc >> 5) & 31));
-            cnt += __popcll(w);
         }
     }
-    block_add(p.nq, cnt);
 }
 
-// The touched chunks in order: per-word popcounts of G, then (after a scan)
-// the chunk index of every set bit.
-__global__ void k_touched_count(const uint32_t *__restrict__ G, uint64_t n, uint32_t *__restrict__ cnt) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < n) cnt[i] = __popc(G[i]);
-}
-
-__global__ void k_touched_list(const uint32_t *__restrict__ G, uint64_t n, const uint32_t *__restrict__ pre,
-                               uint32_t *__restrict__ list) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+// The touched chunks in order, a warp per word of G (32 chunks, one per lane):
+// k_touched_count leaves the set bits of every touched chunk (qn) and, per
+// word, the touched chunks and set bits (cnt[i] and cnt[n + i]); after one scan
+// over both, k_touched_list writes every touched chunk's index and first state
+// and reports the totals (report: touched chunks, states, status).
+__global__ void __launch_bounds__(256) k_touched_count(const uint32_t *__restrict__ G, const uint64_t *__restrict__ D,
+                                                       uint64_t n, uint16_t *__restrict__ qn, uint32_t *__restrict__ cnt) {
+    const uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (i >= n) return;
-    uint32_t g = G[i];
-    uint32_t at = pre[i];
-    while (g) {
-        list[at++] = (uint32_t)(i * 32 + __ffs(g) - 1);
-        g &= g - 1;
+    const uint32_t g = G[i];
+    uint32_t c = 0;
+    if ((g >> lane) & 1u) {
+        const ulonglong2 *w = reinterpret_cast<const ulonglong2 *>(D + (i * 32 + lane) * kChunkWords);
+#pragma unroll 8
+        for (int q = 0; q < (int)kChunkWords / 2; ++q) {
+            const ulonglong2 v = w[q];
+            c += __popcll(v.x) + __popcll(v.y);
+        }
+        qn[i * 32 + lane] = (uint16_t)c;  // at most 2048
     }
+    c = __reduce_add_sync(0xFFFFFFFFu, c);
+    if (lane == 0) {
+        cnt[i] = __popc(g);
+        cnt[n + i] = c;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_touched_list(const uint32_t *__restrict__ G, uint64_t n,
+                                                      const uint16_t *__restrict__ qn, const uint32_t *__restrict__ pre,
+                                                      uint32_t *__restrict__ list, uint32_t *__restrict__ qpre,
+                                                      const uint32_t *__restrict__ status, uint32_t *__restrict__ report) {
+    const uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const uint32_t g = G[i];
+    const bool on = (g >> lane) & 1u;
+    const uint32_t c = on ? qn[i * 32 + lane] : 0u;
+    uint32_t incl = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= d) incl += y;
+    }
+    if (on) {
+        const uint32_t at = pre[i] + __popc(g & ((1u << lane) - 1u));
+        list[at] = (uint32_t)(i * 32 + lane);
+        qpre[at] = pre[n + i] - pre[n] + incl - c;
+    }
+    if (i == n - 1 && lane == 0) {
+        report[0] = pre[n];
+        report[1] = pre[2 * n] - pre[n];
+        report[2] = *status;
+    }
+}
+
+// The key totals of the three kinds and the scan status, for the host.
+__global__ void k_dedup_totals(const uint32_t *__restrict__ tpre, uint64_t ntiles, const uint32_t *__restrict__ status,
+                               uint32_t *__restrict__ report) {
+    const int k = threadIdx.x;
+    if (k < 3) report[k] = tpre[(k + 1) * ntiles] - tpre[k * ntiles];
+    if (k == 3) report[3] = *status;
 }
 
 int dedup_fail(int code, const char *msg) {
@@ -719,19 +716,18 @@ int dedup_fail(int code, const char *msg) {
 
 }  // namespace
 
-// A dedup between dedup_begin (scratch, tables, the candidate bitmap's
-// level-1 part: bitmaps only) and dedup_finish (coarse marks, states, keys:
-// they need the code lists).  Its scratch is freed on its stream.
+// A dedup between dedup_begin (scratch, the candidate bitmap's level-1 part:
+// bitmaps only) and dedup_finish (coarse marks, states, keys: they need the
+// code lists).  Its scratch is freed on its stream.
 struct DedupRun {
     cudaMemPool_t pool;
     cudaStream_t st;
     int num_sms;
     DedupParams p;
-    void *base;    // one pool block holding blk[0..7]
+    uint32_t *report;  // pinned host memory, 4 words
+    void *base;        // one pool block holding blk[0..7]
     void *blk[8];
-    size_t sz[8];
-    uint64_t side, d_words, g_words;
-    bool build1;
+    uint64_t g_words;
 };
 
 void dedup_abort(DedupRun *run) {
@@ -741,7 +737,7 @@ void dedup_abort(DedupRun *run) {
 }
 
 int dedup_begin(cudaMemPool_t pool, cudaStream_t st, int T, const uint64_t *const *bits, const uint32_t *sides,
-                int num_sms, DedupRun **out) {
+                int num_sms, uint32_t *report, DedupRun **out) {
     svo::host::TraceRange trace("svo: dedup candidates");
     *out = nullptr;
     if (T < 1) return dedup_fail(SVO_ERR_DEGENERATE, "dedup needs at least two levels");
@@ -750,6 +746,7 @@ int dedup_begin(cudaMemPool_t pool, cudaStream_t st, int T, const uint64_t *cons
     run->pool = pool;
     run->st = st;
     run->num_sms = num_sms;
+    run->report = report;
     DedupParams &p = run->p;
     p.T = T;
     for (int l = 0; l <= T; ++l) p.lv[l] = DedupLevel{bits[l], nullptr, 0, sides[l]};
@@ -758,17 +755,15 @@ int dedup_begin(cudaMemPool_t pool, cudaStream_t st, int T, const uint64_t *cons
     const uint64_t d_words = std::max<uint64_t>((d_bits + 63) / 64 + kChunkWords - 1, kChunkWords) / kChunkWords * kChunkWords;
     p.chunks = d_words / kChunkWords;
     const uint64_t g_words = (p.chunks + 31) / 32;
-    run->side = side;
-    run->d_words = d_words;
     run->g_words = g_words;
     if (p.chunks > 0xFFFFFFFFull) {
         delete run;
         return dedup_fail(SVO_ERR_UNSUPPORTED, "dedup grid too large");
     }
-    // scratch: D, G, G popcounts + prefix, touched list, scan scratch, status, tables
-    const size_t sz[8] = {d_words * 8, g_words * 4, g_words * 4, (g_words + 1) * 4, p.chunks * 4,
-                          scan_scratch_words(std::max<uint64_t>(p.chunks, g_words)) * 8, 256, sizeof(DedupTables)};
-    std::memcpy(run->sz, sz, sizeof sz);
+    // scratch: D; G and the scan status (cleared together); the two counts per
+    // word of G and their prefix; bits per chunk, touched list, first states; scan scratch
+    const size_t sz[8] = {d_words * 8, g_words * 4 + 4, 2 * g_words * 4, (2 * g_words + 1) * 4, p.chunks * 2,
+                          p.chunks * 4, p.chunks * 4, scan_scratch_words(2 * g_words) * 8};
     size_t at[8], total = 0;
     for (int i = 0; i < 8; ++i) {
         at[i] = total;
@@ -787,30 +782,14 @@ int dedup_begin(cudaMemPool_t pool, cudaStream_t st, int T, const uint64_t *cons
     void **blk = run->blk;
     p.D = static_cast<uint32_t *>(blk[0]);
     p.G = static_cast<uint32_t *>(blk[1]);
-    p.list = static_cast<uint32_t *>(blk[4]);
-    p.nq = reinterpret_cast<unsigned long long *>(static_cast<char *>(blk[6]) + 8);
-    p.tables = static_cast<const DedupTables *>(blk[7]);
-    k_dedup_tables<<<1, 256, 0, st>>>(static_cast<DedupTables *>(blk[7]));
+    p.list = static_cast<uint32_t *>(blk[5]);
+    p.qpre = static_cast<uint32_t *>(blk[6]);
+    if ((e = cudaMemsetAsync(p.G, 0, sz[1], st)) != cudaSuccess) return fail(e, "memset");
+    const uint64_t regions = (d_words + 2047) / 2048;
+    k_dedup_build<<<(unsigned)std::min<uint64_t>(regions, (uint64_t)num_sms * 8), 256, 0, st>>>(p, d_words,
+                                                                                               (uint32_t)(side / 2));
     count_launches(1);
-    // D: in 2048-word regions, level 1 by k_dedup_build (T >= 2), the
-    // coarser levels marked after it; else zeroed and marked at all levels
-    const bool build1 = d_words % 2048 == 0 && T >= 2;
-    run->build1 = build1;
-    if ((e = cudaMemsetAsync(p.G, 0, sz[1], st)) || (e = cudaMemsetAsync(blk[6], 0, 16, st)))
-        return fail(e, "memset");
-    if (d_words % 2048 == 0) {
-        const uint64_t regions = d_words / 2048;
-        const unsigned rb = (unsigned)std::min<uint64_t>(regions, (uint64_t)num_sms * 8);
-        if (build1)
-            k_dedup_build<<<rb, 256, 0, st>>>(p, regions, (uint32_t)(side / 2));
-        else
-            k_dedup_zero<<<rb, 256, 0, st>>>(reinterpret_cast<uint64_t *>(p.D), regions, (uint32_t)(side / 2));
-        count_launches(1);
-        e = cudaGetLastError();
-    } else {
-        e = cudaMemsetAsync(p.D, 0, sz[0], st);
-    }
-    if (e != cudaSuccess) return fail(e, "clear");
+    if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "candidates");
     *out = run;
     return SVO_OK;
 }
@@ -836,21 +815,23 @@ int dedup_finish(DedupRun *run, cudaMemPool_t out_pool, const EmitParams &ep, ui
         p.lv[l].groups = ep.lv[l].n / 8;
     }
     uint32_t g = 0;
-    for (int l = 1; l < T; ++l) {
+    for (int l = 2; l < T; ++l) {
         p.gstart[l] = g;
         g += p.lv[l].groups;
     }
     p.gstart[T] = g;
-    const uint32_t mark_total = g + 1;
     const uint64_t g_words = run->g_words;
     void **blk = run->blk;
-    void *blk2[6] = {};  // sized once the counts are known: states per chunk, the states, keys per tile
+    void *blk2[4] = {};  // sized once the counts are known: the states, keys per tile
     void *base2 = nullptr;  // one pool block holding blk2
     uint32_t *gcnt = static_cast<uint32_t *>(blk[2]);
     uint32_t *gpre = static_cast<uint32_t *>(blk[3]);
-    uint32_t *list = static_cast<uint32_t *>(blk[4]);
-    auto *scan = static_cast<unsigned long long *>(blk[5]);
-    uint32_t *status = static_cast<uint32_t *>(blk[6]);
+    uint16_t *qn = static_cast<uint16_t *>(blk[4]);
+    uint32_t *list = static_cast<uint32_t *>(blk[5]);
+    uint32_t *qpre = static_cast<uint32_t *>(blk[6]);
+    auto *scan = static_cast<unsigned long long *>(blk[7]);
+    uint32_t *status = p.G + g_words;
+    volatile uint32_t *report = run->report;
     cudaError_t e = cudaSuccess;
     auto release = [&]() {
         if (base2) cudaFreeAsync(base2, st);
@@ -862,70 +843,56 @@ int dedup_finish(DedupRun *run, cudaMemPool_t out_pool, const EmitParams &ep, ui
         snprintf(msg, sizeof msg, "dedup %s: %s", what, cudaGetErrorString(err));
         return dedup_fail(err == cudaErrorMemoryAllocation ? SVO_ERR_OUT_OF_MEMORY : SVO_ERR_CUDA, msg);
     };
-    const bool build1 = run->build1;
-    const uint32_t mark_first = build1 ? p.gstart[2] : 0u;
-    k_dedup_mark<<<(mark_total - mark_first + 255) / 256, 256, 0, st>>>(p, mark_first, mark_total);
-    k_touched_count<<<(unsigned)((g_words + 255) / 256), 256, 0, st>>>(p.G, g_words, gcnt);
+    const uint64_t marks = 27ull * g + 8;
+    k_dedup_mark<<<(unsigned)((marks + 255) / 256), 256, 0, st>>>(p, g);
+    const unsigned gblocks = (unsigned)((g_words + 7) / 8);
+    k_touched_count<<<gblocks, 256, 0, st>>>(p.G, reinterpret_cast<const uint64_t *>(p.D), g_words, qn, gcnt);
     count_launches(2);
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "mark");
-    if ((e = launch_scan(gcnt, gpre, g_words, scan, status, st)) != cudaSuccess) return fail(e, "scan");
-    k_touched_list<<<(unsigned)((g_words + 255) / 256), 256, 0, st>>>(p.G, g_words, gpre, list);
+    if ((e = launch_scan(gcnt, gpre, 2 * g_words, scan, status, st)) != cudaSuccess) return fail(e, "scan");
+    k_touched_list<<<gblocks, 256, 0, st>>>(p.G, g_words, qn, gpre, list, qpre, status, run->report);
     count_launches(1);
-    uint32_t h[4] = {0, 0, 0, 0};
-    unsigned long long h_nq = 0;
-    if ((e = cudaMemcpyAsync(h, gpre + g_words, 4, cudaMemcpyDeviceToHost, st)) ||
-        (e = cudaMemcpyAsync(&h_nq, p.nq, 8, cudaMemcpyDeviceToHost, st)) || (e = cudaStreamSynchronize(st)))
-        return fail(e, "touched chunks");
-    p.ntouched = h[0];
-    const uint64_t nt = p.ntouched;
-    if (h_nq > 0xFFFFFFFFull) {
+    if ((e = cudaGetLastError()) || (e = cudaStreamSynchronize(st))) return fail(e, "touched chunks");
+    if (report[2] & kStatusScanTimeout) {
         release();
-        return dedup_fail(SVO_ERR_UNSUPPORTED, "dedup of more than 2^32 lattice cells");
+        return dedup_fail(SVO_ERR_DEVICE_TIMEOUT, "dedup scan look-back timed out");
     }
+    p.ntouched = report[0];
+    const uint64_t nt = p.ntouched, h_nq = report[1];
     const uint64_t ntiles = (h_nq + 31) / 32;
     p.ntiles = ntiles;
-    const size_t sz2[6] = {std::max<uint64_t>(nt, 1) * 4, (nt + 1) * 4, std::max<uint64_t>(h_nq, 1) * 8,
-                           3 * std::max<uint64_t>(ntiles, 1) * 4, 3 * (ntiles + 1) * 4,
-                           scan_scratch_words(std::max<uint64_t>(std::max<uint64_t>(nt, ntiles), 1)) * 8};
-    size_t at2[6], total2 = 0;
-    for (int i = 0; i < 6; ++i) {
+    const size_t sz2[4] = {std::max<uint64_t>(h_nq, 1) * 8, 3 * std::max<uint64_t>(ntiles, 1) * 4,
+                           (3 * std::max<uint64_t>(ntiles, 1) + 1) * 4,
+                           scan_scratch_words(3 * std::max<uint64_t>(ntiles, 1)) * 8};
+    size_t at2[4], total2 = 0;
+    for (int i = 0; i < 4; ++i) {
         at2[i] = total2;
         total2 += (sz2[i] + 255) / 256 * 256;
     }
     if ((e = pool_malloc(&base2, total2, pool, st)) != cudaSuccess) return fail(e, "scratch");
-    for (int i = 0; i < 6; ++i) blk2[i] = static_cast<char *>(base2) + at2[i];
-    p.qn = static_cast<uint32_t *>(blk2[0]);
-    uint32_t *qpre = static_cast<uint32_t *>(blk2[1]);
-    p.qpre = qpre;
-    p.qs = static_cast<uint64_t *>(blk2[2]);
-    p.tcnt = static_cast<uint32_t *>(blk2[3]);
-    uint32_t *tpre = static_cast<uint32_t *>(blk2[4]);
+    for (int i = 0; i < 4; ++i) blk2[i] = static_cast<char *>(base2) + at2[i];
+    p.qs = static_cast<uint64_t *>(blk2[0]);
+    p.tcnt = static_cast<uint32_t *>(blk2[1]);
+    uint32_t *tpre = static_cast<uint32_t *>(blk2[2]);
     p.tpre = tpre;
-    auto *scan2 = static_cast<unsigned long long *>(blk2[5]);
-    if ((e = cudaMemsetAsync(p.tcnt, 0, sz2[3], st)) != cudaSuccess) return fail(e, "memset");
+    auto *scan2 = static_cast<unsigned long long *>(blk2[3]);
+    if ((e = cudaMemsetAsync(p.tcnt, 0, sz2[1], st)) != cudaSuccess) return fail(e, "memset");
     if (nt > 0) {
-        k_chunk_bits<<<(unsigned)((nt + 7) / 8), 256, 0, st>>>(p);
-        count_launches(1);
-        if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "chunk bits");
-        if ((e = launch_scan(p.qn, qpre, nt, scan2, status, st)) != cudaSuccess) return fail(e, "scan");
         const unsigned sblocks =
             (unsigned)std::min<uint64_t>((nt + kStateWarps - 1) / kStateWarps, (uint64_t)num_sms * 32);
         k_dedup_state<<<sblocks, kStateWarps * 32, 0, st>>>(p);
         count_launches(1);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "count");
-    for (int k = 0; k < 3; ++k)
-        if ((e = launch_scan(p.tcnt + k * ntiles, tpre + k * (ntiles + 1), ntiles, scan2, status, st)) != cudaSuccess)
-            return fail(e, "scan");
-    for (int k = 0; k < 3; ++k)
-        if ((e = cudaMemcpyAsync(h + k, tpre + k * (ntiles + 1) + ntiles, 4, cudaMemcpyDeviceToHost, st)))
-            return fail(e, "read totals");
-    if ((e = cudaMemcpyAsync(h + 3, status, 4, cudaMemcpyDeviceToHost, st)) || (e = cudaStreamSynchronize(st)))
-        return fail(e, "read totals");
-    if (h[3] & kStatusScanTimeout) {
+    if ((e = launch_scan(p.tcnt, tpre, 3 * ntiles, scan2, status, st)) != cudaSuccess) return fail(e, "scan");
+    k_dedup_totals<<<1, 32, 0, st>>>(tpre, ntiles, status, run->report);
+    count_launches(1);
+    if ((e = cudaGetLastError()) || (e = cudaStreamSynchronize(st))) return fail(e, "read totals");
+    if (report[3] & kStatusScanTimeout) {
         release();
         return dedup_fail(SVO_ERR_DEVICE_TIMEOUT, "dedup scan look-back timed out");
     }
+    const uint32_t h[3] = {report[0], report[1], report[2]};
     for (int k = 0; k < 3; ++k) {
         if (h[k] == 0) continue;
         void *o = nullptr;

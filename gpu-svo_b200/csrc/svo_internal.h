@@ -60,6 +60,7 @@ struct MeshOut {
     uint64_t any;                 // the code of one surface voxel
     uint32_t queue;               // entries the big-triangle queue needed (the same for all meshes of a batch)
     uint32_t dup;                 // the emission met consecutive duplicates
+    uint32_t dedup[4];            // counts of the dedup (dedup_finish)
 };
 
 // One mesh of a batch, as the kernels see it (an array in device memory).
@@ -249,10 +250,11 @@ constexpr uint32_t kUniqueTile = 4096;
 // side sides[l], l = 0..T): it takes the scratch and builds the level-1 part
 // of the candidate bitmap, so it can run before the code lists exist.
 // dedup_finish (after the code lists, ep) writes the keys and frees the run;
+// report: 4 words of pinned host memory that the kernels leave counts in.
 // dedup_abort frees a run that will not be finished.
 struct DedupRun;
 int dedup_begin(cudaMemPool_t scratch_pool, cudaStream_t st, int T, const uint64_t *const *bits,
-                const uint32_t *sides, int num_sms, DedupRun **run);
+                const uint32_t *sides, int num_sms, uint32_t *report, DedupRun **run);
 int dedup_finish(DedupRun *run, cudaMemPool_t out_pool, const EmitParams &ep, uint64_t n_out[3], uint64_t *out[3]);
 void dedup_abort(DedupRun *run);
 
