@@ -14,9 +14,9 @@
 //     children start at 8*rank_l(code) in level l-1, its parent sits at
 //     8*rank_{l+2}(code >> 6) + ((code >> 3) & 7) in level l+1 -- exactly the
 //     indices the reference's scans produce (src/SVO.cu:221-339);
-//   * k_emit writes node records, vertex and edge arrays in one pass, staged
-//     per warp in shared memory so every global store is a full 512-byte
-//     coalesced streaming write.
+//   * k_emit writes node records, vertex and edge arrays in one pass: records
+//     and edges staged per warp in shared memory and stored by bulk copies,
+//     vertices as full 512-byte coalesced streaming writes.
 #include <cuda/atomic>
 
 #include "svo_internal.h"
@@ -774,59 +774,67 @@ __device__ __forceinline__ void node_info(const EmitParams &P, const float go[3]
 // Full 27-neighbourhood.  The same-level node at offset d exists iff its
 // parent group is a set bit of the next level.  A node with coordinate parity
 // s has its neighbours' parents among 8 groups: its own and, per axis, the
-// one on the side it borders (-1 where s_i = 0, +1 where s_i = 1).  Those 7
-// other groups are ranked once; neighbour d then lies in group b (b_i = 1
-// where d crosses into the bordering group) at child (s ^ [d != 0]).
-__device__ __forceinline__ void full_neighbors(const EmitParams &P, const NodeInfo &ni, uint32_t self,
-                                               uint32_t nb[27]) {
-    nb[13] = self;
-    if (ni.l >= P.T) return;
-    const int l1 = ni.l + 1;
-    const uint64_t pc = ni.code >> 3;
-    const uint32_t s = (uint32_t)(ni.code & 7);
-    const uint64_t sx = spread3(P.lv[l1].side);
-    const uint64_t m[3] = {pc & kDilX, pc & kDilY, pc & kDilZ};
-    const uint64_t lim[3] = {sx, sx << 1, sx << 2};
-    const uint64_t msk[3] = {kDilX, kDilY, kDilZ};
-    uint64_t step[3];
-    bool ok[3];
+// one on the side it borders (-1 where s_i = 0, +1 where s_i = 1); neighbour d
+// then lies in group b (b_i = 1 where d crosses into the bordering group) at
+// child (s ^ [d != 0]).
+// The 8 siblings of a group sit in 8 aligned lanes and need the same 26 groups
+// around theirs: lane k ranks groups k, k + 8, k + 16 and k + 24 and leaves
+// their first nodes in tab (28 words per group in shared memory), where each
+// lane picks its 7.  That is 4 look-ups a lane instead of 7: the emission with
+// full neighbours was held up by their scattered loads (L1 80% busy).
+// All 32 lanes call; on: the lane holds a node below the top level (the same
+// for the 8 lanes of a group).
+__device__ __forceinline__ void full_neighbors(const EmitParams &P, const NodeInfo &ni, uint32_t self, bool on, int lane,
+                                               uint32_t *tab, uint32_t nb[27]) {
+    uint32_t *mine = tab + (lane >> 3) * 28;
+    if (on) {
+        const int l1 = ni.l + 1;
+        const uint64_t pc = ni.pc;
+        const uint64_t sx = spread3(P.lv[l1].side);
+        const uint64_t m[3] = {pc & kDilX, pc & kDilY, pc & kDilZ};
+        const uint64_t lim[3] = {sx, sx << 1, sx << 2};
+        const uint64_t msk[3] = {kDilX, kDilY, kDilZ};
+        uint64_t dn[3], up[3];
+        uint32_t ok = 0;  // bit 3 a + d: step d - 1 along axis a stays in the grid
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if ((s >> a) & 1) {
-            step[a] = dil_inc(m[a], msk[a]);
-            ok[a] = step[a] < lim[a] && step[a] != 0;
-        } else {
-            ok[a] = m[a] != 0;
-            step[a] = dil_dec(m[a], msk[a]);
+        for (int a = 0; a < 3; ++a) {
+            dn[a] = dil_dec(m[a], msk[a]);
+            up[a] = dil_inc(m[a], msk[a]);
+            ok |= ((m[a] != 0 ? 1u : 0u) | 2u | (up[a] < lim[a] && up[a] != 0 ? 4u : 0u)) << (3 * a);
+        }
+        const bool top = l1 >= P.T;  // the root level: rank 0
+        const uint64_t *__restrict__ bits = P.lv[l1].bits;
+        const uint32_t *__restrict__ wpre = P.lv[l1].wpre;
+        uint64_t wd[4];
+        uint32_t wp[4], sh[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {  // all loads first
+            const uint32_t j = (uint32_t)(lane & 7) + 8 * r, d0 = j % 3, d1 = j / 3 % 3, d2 = j / 9;
+            const uint64_t q = (d0 == 0 ? dn[0] : d0 == 1 ? m[0] : up[0]) | (d1 == 0 ? dn[1] : d1 == 1 ? m[1] : up[1]) |
+                               (d2 == 0 ? dn[2] : d2 == 1 ? m[2] : up[2]);
+            const bool in = j < 27 && j != 13 && ((ok >> d0) & (ok >> (3 + d1)) & (ok >> (6 + d2)) & 1u);
+            wd[r] = in ? bits[q >> 6] : 0ull;
+            wp[r] = in && !top ? wpre[q >> 6] : 0u;
+            sh[r] = (uint32_t)(q & 63);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const uint32_t j = (uint32_t)(lane & 7) + 8 * r;
+            const bool ex = (wd[r] >> sh[r]) & 1ull;
+            if (j < 27)
+                mine[j] = ex ? P.lv[ni.l].off + 8u * (wp[r] + (uint32_t)__popcll(wd[r] & ((1ull << sh[r]) - 1ull))) : kNone;
         }
     }
-    const uint32_t own = self - (uint32_t)(ni.code & 7);  // child 0 of the node's own group
-    // the 7 other groups: codes first, then all word loads (in range even for
-    // groups outside the grid, which fall back to the node's own group), then
-    // existence and rank from the loaded words
-    uint64_t q[8];
-    bool in[8];
-#pragma unroll
-    for (int b = 1; b < 8; ++b) {
-        in[b] = !(((b & 1) && !ok[0]) || ((b & 2) && !ok[1]) || ((b & 4) && !ok[2]));
-        q[b] = in[b] ? (((b & 1) ? step[0] : m[0]) | ((b & 2) ? step[1] : m[1]) | ((b & 4) ? step[2] : m[2])) : pc;
-    }
-    uint64_t wd[8];
-    uint32_t wp[8];
-    const bool top = l1 >= P.T;  // the root level: rank 0
-#pragma unroll
-    for (int b = 1; b < 8; ++b) {
-        wd[b] = P.lv[l1].bits[q[b] >> 6];
-        wp[b] = top ? 0u : P.lv[l1].wpre[q[b] >> 6];
-    }
+    __syncwarp();
+    if (!on) return;
+    const uint32_t s = (uint32_t)(ni.code & 7);
+    nb[13] = self;
     uint32_t base[8];
-    base[0] = own;
+    base[0] = self - s;  // child 0 of the node's own group
+    const int ox = (s & 1) ? 1 : -1, oy = (s & 2) ? 3 : -3, oz = (s & 4) ? 9 : -9;
 #pragma unroll
-    for (int b = 1; b < 8; ++b) {
-        const uint32_t sh = (uint32_t)(q[b] & 63);
-        const bool ex = in[b] && ((wd[b] >> sh) & 1ull);
-        base[b] = ex ? P.lv[ni.l].off + 8u * (wp[b] + (uint32_t)__popcll(wd[b] & ((1ull << sh) - 1ull))) : kNone;
-    }
+    for (int b = 1; b < 8; ++b)
+        base[b] = mine[13 + ((b & 1) ? ox : 0) + ((b & 2) ? oy : 0) + ((b & 4) ? oz : 0)];
     // Neighbour d = base[b] | k with, per axis a, (b_a, k_a) = (1, 1), (0, 0),
     // (0, 1) for d_a = -1, 0, +1 when s_a = 0 and (0, 0), (0, 1), (1, 0) when
     // s_a = 1 (every base is a multiple of 8, and kNone | k = kNone): the
@@ -879,25 +887,89 @@ __device__ __forceinline__ void warp_copy_out(const uint4 *src, char *dst, uint3
     }
 }
 
+// The warp's staged bytes (shared memory, written by all lanes) to global
+// memory as one bulk copy: both addresses 16-byte aligned, nbytes a multiple
+// of 16.  The buffer may be rewritten after bulk_wait.
+__device__ __forceinline__ void warp_bulk_out(const uint4 *src, char *dst, uint32_t nbytes, int lane) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the lanes' writes, before the copy reads them
+    __syncwarp();
+    if (lane == 0) {
+        uint64_t first;  // evict first: the outputs are not read again here
+        asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;" ::"l"(dst),
+                     "r"((uint32_t)__cvta_generic_to_shared(src)), "r"(nbytes), "l"(first)
+                     : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+}
+__device__ __forceinline__ void bulk_wait(int lane) {
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    __syncwarp();
+}
+
 __device__ __forceinline__ bool veq(const float *a, const float *b) {
     return a[0] == b[0] && a[1] == b[1] && a[2] == b[2];
 }
 
+// Consecutive duplicates (thrust::unique, src/SVO.cu:679-725) among this node's
+// vertices and edges and between them and the previous node's last ones: the
+// previous node has width pw and origin po; first: there is none.
+__device__ __forceinline__ void count_duplicates(const float *o, float w, const float *po, float pw, bool first,
+                                              uint32_t &vdup, uint32_t &edup) {
+    float vp[8][3], cp[8][3];
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            vp[c][a] = __fmul_rn(w, (float)((c >> a) & 1));
+            cp[c][a] = c == 0 ? o[a] : __fadd_rn(o[a], (c >> a) & 1 ? w : 0.0f);
+        }
+#pragma unroll
+    for (int i = 1; i < 8; ++i) vdup += veq(vp[i], vp[i - 1]);
+#pragma unroll
+    for (int e = 1; e < 12; ++e) {
+        const float *a0 = cp[edge_corner(e - 1, 0)], *a1 = cp[edge_corner(e - 1, 1)];
+        const float *b0 = cp[edge_corner(e, 0)], *b1 = cp[edge_corner(e, 1)];
+        edup += (veq(a0, b0) && veq(a1, b1)) || (veq(a0, b1) && veq(a1, b0));
+    }
+    if (first) return;
+    const float pv7[3] = {__fmul_rn(pw, 1.0f), __fmul_rn(pw, 1.0f), __fmul_rn(pw, 1.0f)};
+    vdup += veq(vp[0], pv7);
+    // previous node's edge 11 = (corner 1, corner 5)
+    const float q1[3] = {__fadd_rn(po[0], pw), __fadd_rn(po[1], 0.0f), __fadd_rn(po[2], 0.0f)};
+    const float q5[3] = {__fadd_rn(po[0], pw), __fadd_rn(po[1], 0.0f), __fadd_rn(po[2], pw)};
+    const float *b0 = cp[0], *b1 = cp[2];
+    edup += (veq(q1, b0) && veq(q5, b1)) || (veq(q1, b1) && veq(q5, b0));
+}
+
 constexpr int kEmitWarps = 4;
-constexpr int kEmitBufBytes = 32 * 336;  // per warp
+constexpr int kEmitBufBytes = 32 * 168;  // per warp: 32 node records, then the edges of 16 nodes at a time
+constexpr int kOwnBytes = 32 * 9 * 4;    // vertex owners (full neighbour tables)
 
 // ONE: a single mesh whose parameters travel in the kernel's parameter space
 // (`one`, read through the constant cache); otherwise each warp looks up its
 // mesh in the batch table (global memory, L1-cached).
+// Node records and edges are staged per warp and leave as bulk copies (the
+// edges 16 nodes at a time, which halves the stage), vertices straight from
+// registers, everything marked to leave L2 first.  The kernel is bound by
+// writes: the SMs' path to L2 is 80% busy (32 bytes per clock and SM) and DRAM
+// 78%.  633 bytes a node: 27.4M nodes in 2,380 us (7.3 TB/s), with full
+// neighbour tables, whose look-ups cost the same memory pipe, in 2,540 to 2,580
+// (2,680 with 7 look-ups per node, plain stores and the whole edge stage at 5
+// CTAs per SM).  6 CTAs per SM: with full tables that spills a few registers
+// that 5 would not, but the dedup's kernels fit beside it (heightfield at res
+// 2048 with dedup 4,150 us for the build, 4,255 with 5, 4,240 before); the
+// vertex and edge arrays alone gain 1% from 6 instead of 8 (torus soup
+// 1,900 us, 1,912), node records alone need 8 (121 us for 3.7M nodes, 139).
+// Without the eviction mark the outputs crowd out the bitmaps (heightfield at
+// res 1024 864 us, 840 with it).
 template <bool S, bool FULL, bool VE, bool ONE>
-// 5 CTAs per SM for the full-neighbour and single-mesh variants (the
-// shared-memory staging allows 5; 102 registers hold them without spills);
-// the batched parity variant measured faster with the compiler's own choice.
-__global__ void __launch_bounds__(kEmitWarps * 32, (FULL || ONE) ? 5 : 1)
+__global__ void __launch_bounds__(kEmitWarps * 32, FULL || VE ? 6 : 8)
     k_emit(EmitBatch eb, const __grid_constant__ EmitParams one, uint64_t total) {
-    extern __shared__ uint4 smem[];
+    extern __shared__ __align__(128) uint4 smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint4 *wbuf = smem + warp * (kEmitBufBytes / 16);
+    constexpr int kWarpBytes = kEmitBufBytes + (VE && FULL ? kOwnBytes : 0);
+    uint4 *wbuf = smem + warp * (kWarpBytes / 16);
     const uint64_t nwarps = (uint64_t)gridDim.x * kEmitWarps;
     for (uint64_t gbase = ((uint64_t)blockIdx.x * kEmitWarps + warp) * 32; gbase < total; gbase += nwarps * 32) {
         const int mj = ONE ? 0 : find_segment(eb.node_off, eb.n, gbase);
@@ -905,21 +977,53 @@ __global__ void __launch_bounds__(kEmitWarps * 32, (FULL || ONE) ? 5 : 1)
         const uint64_t base = ONE ? gbase : gbase - eb.node_off[mj];
         if (base >= P.N) continue;  // padding between meshes
         const float go[3] = {P.gp->origin[0], P.gp->origin[1], P.gp->origin[2]};
-        unsigned long long vdup = 0, edup = 0;
         const uint32_t t = (uint32_t)(base + lane);
         const bool valid = base + lane < P.N;
         const uint32_t cnt = (uint32_t)(P.N - base < 32 ? P.N - base : 32);
         NodeInfo ni;
         if (valid) node_info<S>(P, go, t, ni);
+        if (VE) {
+            // Consecutive duplicates need a corner that coincides with another of the
+            // same node: consecutive edges differ in some corner, and the previous
+            // node's last edge has one y where this node's first has two.  So a node
+            // whose width shows in all three coordinates has none, and the previous
+            // node is looked up only in the rare rest (degenerate widths, coordinates
+            // that absorb the width): that look-up and the 36 comparisons took every
+            // warp a sixth of its instructions.
+            if (__any_sync(0xFFFFFFFFu, valid && (ni.w == 0.0f || __fadd_rn(ni.o[0], ni.w) == ni.o[0] ||
+                                                  __fadd_rn(ni.o[1], ni.w) == ni.o[1] ||
+                                                  __fadd_rn(ni.o[2], ni.w) == ni.o[2]))) {
+                float pw = __shfl_up_sync(0xFFFFFFFFu, valid ? ni.w : 0.0f, 1);
+                float po[3], o[3] = {ni.o[0], ni.o[1], ni.o[2]};
+#pragma unroll
+                for (int a = 0; a < 3; ++a) po[a] = __shfl_up_sync(0xFFFFFFFFu, valid ? ni.o[a] : 0.0f, 1);
+                if (lane == 0 && valid && t > 0) {
+                    NodeInfo pn;
+                    node_info<S>(P, go, t - 1, pn);
+                    pw = pn.w;
+                    po[0] = pn.o[0];
+                    po[1] = pn.o[1];
+                    po[2] = pn.o[2];
+                }
+                uint32_t vdup = 0, edup = 0;
+                if (valid) count_duplicates(o, ni.w, po, pw, t == 0, vdup, edup);
+                vdup = __reduce_add_sync(0xFFFFFFFFu, vdup);
+                edup = __reduce_add_sync(0xFFFFFFFFu, edup);
+                // the first of them raises the host's flag: only then are the counters read back
+                if (lane == 0 && vdup && atomicAdd(P.dups, (unsigned long long)vdup) == 0) *P.dup_flag = 1;
+                if (lane == 0 && edup && atomicAdd(P.dups + 1, (unsigned long long)edup) == 0) *P.dup_flag = 1;
+            }
+        }
         uint32_t nb[27];
 #pragma unroll
         for (int j = 0; j < 27; ++j) nb[j] = kNone;
-        if (valid) {
-            if (FULL) {
-                full_neighbors(P, ni, t, nb);
-            } else if (ni.l == P.T && P.T >= 1) {
-                nb[13] = t;  // root self entry, src/SVO.cu:522-529,556-557
-            }
+        bulk_wait(lane);  // the buffer's last copy has been read
+        if (FULL) {
+            full_neighbors(P, ni, t, valid && ni.l < P.T, lane, reinterpret_cast<uint32_t *>(wbuf), nb);
+            if (valid && ni.l == P.T) nb[13] = t;
+            __syncwarp();  // the table is read before the records take its place
+        } else if (valid && ni.l == P.T && P.T >= 1) {
+            nb[13] = t;  // root self entry, src/SVO.cu:522-529,556-557
         }
         // ---- node records (21 u64 words each) ----
         if (valid) {
@@ -940,151 +1044,123 @@ __global__ void __launch_bounds__(kEmitWarps * 32, (FULL || ONE) ? 5 : 1)
 #pragma unroll
             for (int k = 0; k < 13; ++k) d[8 + k] = pk(nb[1 + 2 * k], nb[2 + 2 * k]);
         }
-        __syncwarp();
-        warp_copy_out(wbuf, reinterpret_cast<char *>(P.nodes) + base * 168, cnt * 168, lane);
-        __syncwarp();
+        if (cnt == 32) {
+            warp_bulk_out(wbuf, reinterpret_cast<char *>(P.nodes) + base * 168, 32 * 168, lane);
+        } else {  // the mesh's last nodes
+            __syncwarp();
+            warp_copy_out(wbuf, reinterpret_cast<char *>(P.nodes) + base * 168, cnt * 168, lane);
+            __syncwarp();
+        }
         if (!VE) continue;
         // ---- vertices: corner i = width * (i&1, i>>1&1, i>>2&1), src/SVO.cu:586-608 ----
-        float vp[8][3];
-        uint32_t vown[8];
-        if (valid) {
+        // Stored in output order straight from registers: lane l writes corner
+        // l & 7 of nodes 4j + (l >> 3).  Only the owners of full neighbour
+        // tables go through shared memory, beside the node records.
+        uint32_t *vown = reinterpret_cast<uint32_t *>(wbuf) + kEmitBufBytes / 4;
+        // Owners with full neighbour tables: the smallest node sharing the vertex (8
+        // nodes) or the edge (4), one axis at a time: pairs along x, then y, then z.
+        // The neighbours come back from the staged record: held in registers across
+        // the staging they spilled (12% of the instructions were local loads and
+        // stores, beside a memory pipe that is the bottleneck here).
+        uint32_t eown[12];
+        if (FULL) {
+            const unsigned long long *rec = reinterpret_cast<const unsigned long long *>(wbuf) + lane * 21;
+            nb[0] = (uint32_t)(rec[7] >> 32);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                vp[i][0] = __fmul_rn(ni.w, (float)(i & 1));
-                vp[i][1] = __fmul_rn(ni.w, (float)((i >> 1) & 1));
-                vp[i][2] = __fmul_rn(ni.w, (float)((i >> 2) & 1));
-                uint32_t own = t;
-                if (FULL) {
-                    const int cx = i & 1, cy = (i >> 1) & 1, cz = (i >> 2) & 1;
-                    uint32_t best = kNone;
+            for (int k = 0; k < 13; ++k) {
+                const unsigned long long v = rec[8 + k];
+                nb[1 + 2 * k] = (uint32_t)v;
+                nb[2 + 2 * k] = (uint32_t)(v >> 32);
+            }
+            uint32_t px[2][3][3], pxy[2][2][3];  // [x pair][y][z], [x pair][y pair][z]
+            uint32_t xe[2][2], ye[2][2], ze[2][2];
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const int s = (cx - 1 + (q & 1) + 1) + 3 * (cy - 1 + ((q >> 1) & 1) + 1) +
-                                      9 * (cz - 1 + ((q >> 2) & 1) + 1);
-                        best = min(best, nb[s]);
-                    }
-                    own = best;
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    xe[i][j] = min(min(nb[1 + 3 * i + 9 * j], nb[4 + 3 * i + 9 * j]),
+                                   min(nb[10 + 3 * i + 9 * j], nb[13 + 3 * i + 9 * j]));
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int y = 0; y < 3; ++y)
+#pragma unroll
+                    for (int z = 0; z < 3; ++z) px[i][y][z] = min(nb[i + 3 * y + 9 * z], nb[i + 1 + 3 * y + 9 * z]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    ye[i][j] = min(px[i][1][j], px[i][1][j + 1]);
+#pragma unroll
+                    for (int z = 0; z < 3; ++z) pxy[i][j][z] = min(px[i][j][z], px[i][j + 1][z]);
+                    ze[i][j] = pxy[i][j][1];
                 }
-                vown[i] = own;
-                wbuf[lane * 8 + (i ^ (lane & 7))] =
-                    make_uint4(__float_as_uint(vp[i][0]), __float_as_uint(vp[i][1]),
-                               __float_as_uint(vp[i][2]), own);
-            }
-        }
-        __syncwarp();
-        {
-            const uint32_t nv = cnt * 8;
-            uint4 *d4 = reinterpret_cast<uint4 *>(P.verts + base * 8);
-            for (uint32_t v = lane; v < nv; v += 32) {
-                const uint32_t node = v >> 3, k = v & 7;
-                __stcs(d4 + v, wbuf[node * 8 + (k ^ (node & 7))]);
-            }
-        }
-        __syncwarp();
-        // ---- edges: 12 per node in the reference's order, src/SVO.cu:629-677 ----
-        float cp[8][3];
-        float pw = 0.0f;
-        float po[3] = {0.0f, 0.0f, 0.0f};
-        {
-            // previous node's width and origin (for the duplicate checks)
-            pw = __shfl_up_sync(0xFFFFFFFFu, valid ? ni.w : 0.0f, 1);
 #pragma unroll
-            for (int a = 0; a < 3; ++a) po[a] = __shfl_up_sync(0xFFFFFFFFu, valid ? ni.o[a] : 0.0f, 1);
-            if (lane == 0 && valid && t > 0) {
-                NodeInfo pn;
-                node_info<S>(P, go, t - 1, pn);
-                pw = pn.w;
-                po[0] = pn.o[0];
-                po[1] = pn.o[1];
-                po[2] = pn.o[2];
-            }
-        }
-        if (valid) {
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                if (c == 0) {
-                    cp[0][0] = ni.o[0];
-                    cp[0][1] = ni.o[1];
-                    cp[0][2] = ni.o[2];
-                } else {
-                    cp[c][0] = __fadd_rn(ni.o[0], (c & 1) ? ni.w : 0.0f);
-                    cp[c][1] = __fadd_rn(ni.o[1], (c & 2) ? ni.w : 0.0f);
-                    cp[c][2] = __fadd_rn(ni.o[2], (c & 4) ? ni.w : 0.0f);
-                }
-            }
-            uint32_t eown[12];
+            for (int c = 0; c < 8; ++c)
+                vown[lane * 9 + c] = min(pxy[c & 1][(c >> 1) & 1][c >> 2], pxy[c & 1][(c >> 1) & 1][(c >> 2) + 1]);
 #pragma unroll
             for (int e = 0; e < 12; ++e) {
-                uint32_t own = t;
-                if (FULL) {
-                    const int a = edge_corner(e, 0), b = edge_corner(e, 1);
-                    uint32_t best = kNone;
+                const int a = edge_corner(e, 0), ax = a ^ edge_corner(e, 1);
+                eown[e] = ax == 1 ? xe[(a >> 1) & 1][a >> 2] : ax == 2 ? ye[a & 1][a >> 2] : ze[a & 1][(a >> 1) & 1];
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 12; ++e) eown[e] = t;
+        }
+        if (FULL) __syncwarp();
+        {
+            uint4 *d4 = reinterpret_cast<uint4 *>(P.verts + base * 8);
+            const float mine = valid ? ni.w : 0.0f;
+            const int k = lane & 7;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint32_t node = 4 * j + (lane >> 3);
+                const float w = __shfl_sync(0xFFFFFFFFu, mine, (int)node);
+                const uint32_t own = FULL ? vown[node * 9 + k] : (uint32_t)base + node;
+                if (node < cnt)
+                    __stcs(d4 + lane + 32 * j, make_uint4(__float_as_uint(__fmul_rn(w, (float)(k & 1))),
+                                                          __float_as_uint(__fmul_rn(w, (float)((k >> 1) & 1))),
+                                                          __float_as_uint(__fmul_rn(w, (float)((k >> 2) & 1))), own));
+            }
+        }
+        // ---- edges: 12 per node in the reference's order, src/SVO.cu:629-677 ----
+        // a corner's coordinates: corner 0 is the origin itself, the others add 0 or the width
+        float oz[3], ow[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            oz[a] = __fadd_rn(ni.o[a], 0.0f);
+            ow[a] = __fadd_rn(ni.o[a], ni.w);
+        }
+        // 16 nodes at a time through the buffer, 84 words per node: edge e = p0 (3), p1 (3), owner
+#pragma unroll 1
+        for (uint32_t h = 0; h < 2; ++h) {
+            bulk_wait(lane);  // the node records, or the first half, have been read
+            if (valid && (uint32_t)(lane >> 4) == h) {
+                uint4 *d = wbuf + (lane & 15) * 21;
+#pragma unroll
+                for (int j = 0; j < 21; ++j) {
+                    uint32_t wv[4];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        int d[3], qq = 0;
-#pragma unroll
-                        for (int ax = 0; ax < 3; ++ax) {
-                            const int ca = (a >> ax) & 1, cb = (b >> ax) & 1;
-                            if (ca != cb) {
-                                d[ax] = 0;
-                            } else {
-                                d[ax] = ca - 1 + ((q >> qq) & 1);
-                                ++qq;
-                            }
-                        }
-                        best = min(best, nb[(d[0] + 1) + 3 * (d[1] + 1) + 9 * (d[2] + 1)]);
+                        const int wi = 4 * j + q, e = wi / 7, f = wi % 7;
+                        const int c = edge_corner(e, f < 3 ? 0 : 1), a = f % 3;
+                        wv[q] = f == 6 ? eown[e] : __float_as_uint(c == 0 ? ni.o[a] : (c >> a) & 1 ? ow[a] : oz[a]);
                     }
-                    own = best;
+                    d[j] = make_uint4(wv[0], wv[1], wv[2], wv[3]);
                 }
-                eown[e] = own;
             }
-            // 84 words per node: edge e = p0 (3), p1 (3), owner
-            uint4 *d = wbuf + lane * 21;
-#pragma unroll
-            for (int j = 0; j < 21; ++j) {
-                uint32_t wv[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int wi = 4 * j + q, e = wi / 7, f = wi % 7;
-                    wv[q] = f < 3   ? __float_as_uint(cp[edge_corner(e, 0)][f])
-                            : f < 6 ? __float_as_uint(cp[edge_corner(e, 1)][f - 3])
-                                    : eown[e];
-                }
-                d[j] = make_uint4(wv[0], wv[1], wv[2], wv[3]);
-            }
-            // consecutive duplicates (thrust::unique, src/SVO.cu:679-725)
-#pragma unroll
-            for (int i = 1; i < 8; ++i) vdup += veq(vp[i], vp[i - 1]);
-            if (t > 0) {
-                const float pv7[3] = {__fmul_rn(pw, 1.0f), __fmul_rn(pw, 1.0f), __fmul_rn(pw, 1.0f)};
-                vdup += veq(vp[0], pv7);
-            }
-#pragma unroll
-            for (int e = 1; e < 12; ++e) {
-                const float *a0 = cp[edge_corner(e - 1, 0)], *a1 = cp[edge_corner(e - 1, 1)];
-                const float *b0 = cp[edge_corner(e, 0)], *b1 = cp[edge_corner(e, 1)];
-                edup += (veq(a0, b0) && veq(a1, b1)) || (veq(a0, b1) && veq(a1, b0));
-            }
-            if (t > 0) {
-                // previous node's edge 11 = (corner 1, corner 5)
-                const float q1[3] = {__fadd_rn(po[0], pw), __fadd_rn(po[1], 0.0f), __fadd_rn(po[2], 0.0f)};
-                const float q5[3] = {__fadd_rn(po[0], pw), __fadd_rn(po[1], 0.0f), __fadd_rn(po[2], pw)};
-                const float *b0 = cp[0], *b1 = cp[2];
-                edup += (veq(q1, b0) && veq(q5, b1)) || (veq(q1, b1) && veq(q5, b0));
+            char *dst = reinterpret_cast<char *>(P.edges) + (base + 16 * h) * 336;
+            if (cnt == 32) {
+                warp_bulk_out(wbuf, dst, 16 * 336, lane);
+            } else {
+                __syncwarp();
+                const uint32_t left = cnt > 16 * h ? (cnt - 16 * h < 16 ? cnt - 16 * h : 16) : 0;
+                warp_copy_out(wbuf, dst, left * 336, lane);
+                __syncwarp();
             }
         }
-        __syncwarp();
-        warp_copy_out(wbuf, reinterpret_cast<char *>(P.edges) + base * 336, cnt * 336, lane);
-        __syncwarp();
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            vdup += __shfl_xor_sync(0xFFFFFFFFu, vdup, d);
-            edup += __shfl_xor_sync(0xFFFFFFFFu, edup, d);
-        }
-        // the first of them raises the host's flag: only then are the counters read back
-        if (lane == 0 && vdup && atomicAdd(P.dups, vdup) == 0) *P.dup_flag = 1;
-        if (lane == 0 && edup && atomicAdd(P.dups + 1, edup) == 0) *P.dup_flag = 1;
     }
+    bulk_wait(lane);  // shared memory is read to the end before the block leaves
 }
 
 // ---------------------------------------------------------------------------
@@ -1238,9 +1314,9 @@ cudaError_t launch_emit(const EmitBatch &b, const EmitParams *one, uint64_t tota
     const uint64_t warps = (total + 31) / 32;
     const unsigned blocks = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>((warps + kEmitWarps - 1) / kEmitWarps, 0x7FFFFFFFull));
-    const size_t shmem = (size_t)kEmitWarps * kEmitBufBytes;
     const bool s = (flags & SVO_FLAG_STRICT_FP) != 0, f = (flags & SVO_FLAG_FULL_NEIGHBORS) != 0,
                ve = (flags & SVO_FLAG_NO_VERT_EDGE) == 0;
+    const size_t shmem = (size_t)kEmitWarps * (kEmitBufBytes + (ve && f ? kOwnBytes : 0));
     const EmitParams p1 = one ? *one : EmitParams{};
 #define SVO_EMIT1(S_, F_, V_)                                                                       \
     do {                                                                                             \
