@@ -13,11 +13,13 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
 #include "svo_internal.h"
 #include "svo_host.h"
+#include "svo_hostcopy.h"
 
 using namespace svo;
 
@@ -46,6 +48,7 @@ struct svo_ctx {
     };
     std::mutex pinned_mu;
     std::vector<Pinned> pinned_free;
+    std::shared_ptr<svo::host::CopyPool> copies;  // staged copies of results, shared with them
 };
 
 // One device block that holds the output arrays of several results (a wave of
@@ -73,6 +76,7 @@ struct svo_result {
     int n_timings = 0;
     float timings[9] = {};
     svo_arena *arena = nullptr;  // holds nodes/verts/edges/keys when set
+    std::shared_ptr<svo::host::CopyPool> copies;
     uint32_t own = 0x7F;         // bit i: array i of {nodes, verts, edges, keys, dedup x3} is freed on its own
 };
 
@@ -110,6 +114,16 @@ bool is_device_ptr(const void *p) {
         return false;
     }
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+}
+
+// Ordinary host memory, unknown to CUDA.
+bool is_pageable_ptr(const void *p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
 }
 
 // Stream-ordered scratch owned by one build; everything is returned to the
@@ -785,6 +799,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 r->device = ctx->device;
                 r->stream = st;
                 r->pool = ctx->pool;
+                r->copies = ctx->copies;
                 r->depth = mh.T + 1;
                 for (int l = 0; l <= mh.T; ++l) r->level_counts.push_back((int64_t)mh.n_l[l]);
                 for (int a = 0; a < 3; ++a) {
@@ -1143,6 +1158,7 @@ int svo_ctx_create(int device, svo_ctx **out) {
     svo_ctx *c = new svo_ctx();
     c->device = device;
     c->num_sms = prop.multiProcessorCount;
+    c->copies = svo::host::copy_pool_create(device);
     // Two pools of its own: per-build scratch, and result arrays (kept apart
     // so scratch never splits their blocks).  Freed blocks stay cached.
     cudaMemPoolProps props{};
@@ -1451,6 +1467,12 @@ static int copy_out(const svo_result *r, void *dst, const void *src, uint64_t n,
     if (n == 0) return SVO_OK;
     if (!src) return fail(SVO_ERR_INVALID_ARGUMENT, "%s were not built", what);
     SVO_TRY(cudaSetDevice(r->device), "cudaSetDevice");
+    cudaError_t staged = cudaSuccess;
+    if (r->copies && is_pageable_ptr(dst) &&
+        svo::host::copy_to_pageable(*r->copies, dst, src, n * esz, r->stream, &staged)) {
+        SVO_TRY(staged, what);
+        return SVO_OK;
+    }
     SVO_TRY(cudaMemcpyAsync(dst, src, n * esz, cudaMemcpyDeviceToHost, r->stream), what);
     SVO_TRY(cudaStreamSynchronize(r->stream), what);
     return SVO_OK;

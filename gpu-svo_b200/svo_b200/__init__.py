@@ -547,7 +547,7 @@ class Result:
         return np.array(list(box.min) + list(box.max) + list(box.width), dtype=np.float32)
 
     def _copy(self, name: str, n: int, dtype) -> np.ndarray:
-        out = np.zeros(n, dtype=dtype)
+        out = np.empty(n, dtype=dtype)  # written whole, or an error is raised
         _check(getattr(lib(), f"svo_result_copy_{name}")(self._h, out.ctypes.data, n))
         return out
 
@@ -571,7 +571,7 @@ class Result:
 
     def dedup(self, kind: int) -> np.ndarray:
         n = lib().svo_result_num_dedup(self._h, kind)
-        out = np.zeros(max(n, 0), dtype=np.uint64)
+        out = np.empty(max(n, 0), dtype=np.uint64)
         _check(lib().svo_result_copy_dedup(self._h, kind, out.ctypes.data, out.shape[0]))
         return out
 

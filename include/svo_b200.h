@@ -328,8 +328,9 @@ const svo_node *svo_result_nodes_device(const svo_result *r);
 const svo_vertex *svo_result_vertices_device(const svo_result *r);
 const svo_edge *svo_result_edges_device(const svo_result *r);
 const uint64_t *svo_result_keys_device(const svo_result *r);
-/* Copies to host memory (cap = capacity in elements; returns SVO_ERR_INVALID_ARGUMENT
- * when too small). */
+/* Copies to host memory (cap = capacity in elements; large copies to pageable
+ * memory go through pinned slots, 16 MiB at most, that the context and its
+ * results share; returns SVO_ERR_INVALID_ARGUMENT when too small). */
 int svo_result_copy_nodes(const svo_result *r, svo_node *dst, int64_t cap);
 int svo_result_copy_vertices(const svo_result *r, svo_vertex *dst, int64_t cap);
 int svo_result_copy_edges(const svo_result *r, svo_edge *dst, int64_t cap);
