@@ -244,6 +244,7 @@ struct svo_batch {
     uint64_t *bits = nullptr;
     uint32_t *pre = nullptr, *base = nullptr;  // block ranks, region prefixes (RankDev)
     uint8_t *rflag = nullptr;               // level-0 regions that triangles reach (one byte per pyramid CTA)
+    uint32_t *rlist = nullptr, *rcount = nullptr;  // the regions to read (BatchDev)
     unsigned long long *dups = nullptr;     // 2 per live mesh (device, zeroed by phase A)
     svo_ctx::Pinned box{nullptr, 0};        // pinned host memory: a MeshOut per live mesh
     MeshOut *out = nullptr;
@@ -409,6 +410,7 @@ int batch_phase_a(svo_batch *b) {
     // ---- layout ----
     uint64_t words = 0, blocks = 0, bases = 0, tris = 0;
     uint32_t ctas = 0, max_ctas = 0, bblocks = 0;
+    bool any_regions = false;
     std::vector<uint64_t> tri_off(n + 1);
     std::vector<uint32_t> cta_off(n + 1), bbox_off(n + 1);
     for (int k = 0; k < n; ++k) {
@@ -427,6 +429,7 @@ int batch_phase_a(svo_batch *b) {
         tris += (uint64_t)mh.n_tris;
         ctas += mh.py.ctas;
         max_ctas = std::max(max_ctas, mh.py.ctas);
+        any_regions |= mh.py.words[0] >= kRegionWords;
         bblocks += bbox_blocks(mh.n_pts);
     }
     tri_off[n] = tris;
@@ -441,7 +444,8 @@ int batch_phase_a(svo_batch *b) {
     const size_t o_meta = lay.add<unsigned char>(ml.bytes);
     const size_t o_bits = lay.add<uint64_t>(words), o_pre = lay.add<uint32_t>(blocks), o_base = lay.add<uint32_t>(bases),
                  o_big = lay.add<uint4>(big_cap),
-                 o_rflag = lay.add<uint8_t>(std::max<uint32_t>(ctas, 1));
+                 o_rflag = lay.add<uint8_t>(std::max<uint32_t>(ctas, 1)),
+                 o_rlist = lay.add<uint32_t>(any_regions ? ctas : 0);
     const size_t o_tables = lay.add<unsigned char>(t_bytes);
     unsigned char *blk = batch_alloc<unsigned char>(b, lay.bytes, err);
     if (err != cudaSuccess || !blk) return cuda_fail(err, "batch scratch");
@@ -450,14 +454,15 @@ int batch_phase_a(svo_batch *b) {
     b->base = reinterpret_cast<uint32_t *>(blk + o_base);
     uint4 *big = reinterpret_cast<uint4 *>(blk + o_big);
     uint8_t *rflag = b->rflag = blk + o_rflag;
+    b->rlist = reinterpret_cast<uint32_t *>(blk + o_rlist);
     unsigned char *meta = blk + o_meta;
     GridParams *gp = reinterpret_cast<GridParams *>(meta + ml.gp);
     uint64_t *any = reinterpret_cast<uint64_t *>(meta + ml.any);
     uint32_t *mm = reinterpret_cast<uint32_t *>(meta + ml.mm);
     uint32_t *done = reinterpret_cast<uint32_t *>(meta + ml.done);
     uint32_t *counters = reinterpret_cast<uint32_t *>(meta + ml.counters);
+    b->rcount = counters + 2;
     b->dups = reinterpret_cast<unsigned long long *>(meta + ml.dups);
-    bool any_regions = false;
     b->h_mesh.assign(n, MeshDev{});
     for (int k = 0; k < n; ++k) {
         const MeshHost &mh = b->m[b->live[k]];
@@ -479,7 +484,6 @@ int batch_phase_a(svo_batch *b) {
         d.done = done + k;
         d.py = mh.py;
         d.regions = mh.py.words[0] >= kRegionWords ? 1 : 0;
-        any_regions |= d.regions != 0;
     }
     const size_t p_mesh = tables.add(b->h_mesh), p_tri = tables.add(tri_off), p_cta = tables.add(cta_off),
                  p_bbox = tables.add(bbox_off);
@@ -490,7 +494,7 @@ int batch_phase_a(svo_batch *b) {
     const uint32_t *d_bbox_off = reinterpret_cast<const uint32_t *>(dt + p_bbox);
     if (n > 1)  // a lone mesh's table goes with the first kernel
         SVO_TRY(cudaMemcpyAsync(dt, tables.buf.data(), tables.buf.size(), cudaMemcpyHostToDevice, st), "upload meshes");
-    const BatchDev bd{b->d_mesh, n, d_tri_off, d_cta_off, d_bbox_off, rflag};
+    const BatchDev bd{b->d_mesh, n, d_tri_off, d_cta_off, d_bbox_off, rflag, any_regions ? b->rlist : nullptr, b->rcount};
     const bool strict = (b->flags & SVO_FLAG_STRICT_FP) != 0;
     StageTimer tm((b->flags & SVO_FLAG_TIMINGS) != 0);
     for (int attempt = 0; attempt < 2; ++attempt) {
@@ -742,7 +746,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
             std::vector<CompactJob> jobs;
             std::vector<uint64_t> word_off(1, 0);
             std::vector<CompactJob> region_jobs;  // region-mode meshes' levels 1-2
-            std::vector<uint32_t> region_counts;
+            std::vector<std::pair<uint32_t, uint32_t>> region_range;  // first region, regions
             std::vector<KeyJob> kjobs;
             std::vector<uint64_t> blk_off(1, 0);
             std::vector<EmitParams> ep(n);
@@ -842,7 +846,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                     // level 3 words of unflagged regions are empty, not read
                     job.rflag = b->rflag + mh.cta0;
                     region_jobs.push_back(job);
-                    region_counts.push_back(mh.py.ctas);
+                    region_range.push_back({mh.cta0, mh.py.ctas});
                 }
                 if (want_keys && (mh.T < 3 || mh.py.words[0] <= kDirectKeyWords)) {
                     job.l0 = 0;
@@ -930,7 +934,9 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                                  word_off.back(), st),
                   "compact");
             for (size_t i = 0; i < region_jobs.size(); ++i)
-                check(launch_compact_regions(region_jobs[i], region_counts[i], ctx->num_sms, st), "compact");
+                check(launch_compact_regions(region_jobs[i], b->rlist, b->rcount, region_range[i].first,
+                                             region_range[i].second, ctx->num_sms, st),
+                      "compact");
             if (!kjobs.empty())
                 check(launch_compact_keys(KeyBatch{d_kjobs, (int)kjobs.size(), d_blk_off}, blk_off.back(), st), "keys");
             tm.mark(StageTimer::kCompact, st);

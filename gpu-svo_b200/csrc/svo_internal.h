@@ -93,6 +93,11 @@ struct BatchDev {
     const uint32_t *cta_off;   // first pyramid CTA of each mesh
     const uint32_t *bbox_off;  // first bbox-reduction block of each mesh
     uint8_t *rflag = nullptr;  // per pyramid CTA (a 2048-word region of level 0): a triangle reaches it
+    // Batches with a region-mode mesh: the regions that are read (all of the
+    // other meshes', the flagged ones of region-mode meshes) in no order, and
+    // their number, zeroed.
+    uint32_t *rlist = nullptr;
+    uint32_t *rcount = nullptr;
 };
 
 // Level-0 regions (2048 words: 64 x 64 x 32 voxels) are tracked from this
@@ -204,9 +209,12 @@ cudaError_t launch_voxelize(const BatchDev &b, int64_t total_tris, bool strict, 
                             uint4 *big, uint32_t big_cap, uint32_t *counters, int num_sms, cudaStream_t st);
 // Builds levels 1.. of every mesh's pyramid, the block ranks and the level
 // totals; max_ctas: the most regions of any mesh (py.ctas).  done must be zero.
+// With b.rlist set only the listed regions are visited.
 cudaError_t launch_pyramid(const BatchDev &b, uint32_t total_ctas, uint32_t max_ctas, int num_sms, cudaStream_t st);
 // For batches with a region-mode mesh: flags the level-0 regions that its
-// triangles reach (rflag zeroed by launch_front), then zeroes those.
+// triangles reach (rflag zeroed by launch_front), zeroes those and lists the
+// regions to read; the unflagged regions get their words of levels 1..4 and
+// their region sums here (zeros), and the pyramid only visits the list.
 cudaError_t launch_regions(const BatchDev &b, int64_t total_tris, uint32_t total_ctas, int num_sms, cudaStream_t st);
 // Exclusive scan of n u32 values; out has n + 1 entries (out[n] = total).
 // scratch: >= scan_scratch_words(n) u64 words, zeroed by the call.
@@ -229,8 +237,10 @@ cudaError_t pool_malloc(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t
 // one: the job of a one-job batch (host copy, passed by value), or null.
 cudaError_t launch_compact(const CompactBatch &c, const CompactJob *one, uint64_t total_words, cudaStream_t st);
 cudaError_t launch_compact_keys(const KeyBatch &k, uint64_t total_blocks, cudaStream_t st);
-// Levels 1 and 2 of a region-mode job (job.rflag set), one block per level-0 region.
-cudaError_t launch_compact_regions(const CompactJob &job, uint32_t regions, int num_sms, cudaStream_t st);
+// Levels 1 and 2 of a region-mode job (job.rflag set): its regions are those of
+// the batch's list (BatchDev) from cta0 on.
+cudaError_t launch_compact_regions(const CompactJob &job, const uint32_t *rlist, const uint32_t *rcount, uint32_t cta0,
+                                   uint32_t regions, int num_sms, cudaStream_t st);
 // one: the EmitParams of a one-mesh batch (host copy, passed by value to the
 // kernel), or null for a batch of several meshes.
 cudaError_t launch_emit(const EmitBatch &b, const EmitParams *one, uint64_t total_nodes, uint32_t flags,

@@ -215,9 +215,9 @@ __device__ __forceinline__ void finish_top(const MeshDev &md, uint64_t (*s_top)[
 // set bits of levels 0..3 (md.base), whose prefix over the regions completes
 // the rank -- there is no scan over the blocks (19.2M of them at res 2048:
 // that scan and the memset before it took 60 us, this scan of 4 x 65,536
-// region sums takes 7).  A region-mode mesh's region that no triangle reaches
-// is empty and is not read (its level-0 words are not zeroed in memory): its
-// words of levels 1..4 and its sums are written as zeros.
+// region sums takes 7).  With a region-mode mesh in the batch only the listed
+// regions are visited: the others are empty, not zeroed in memory at level 0
+// and dealt with by k_region_prepare.
 //
 // FUSE: the CTA that finishes a mesh's last region scans the sums and builds
 // the levels above 4 as well, which saves a launch (about 5 us of the 213 us
@@ -238,20 +238,16 @@ __global__ void __launch_bounds__(256, FUSE ? 4 : 8) k_pyramid(BatchDev bd, uint
     __shared__ uint32_t s_last;
     __shared__ __align__(16) uint64_t s_top[FUSE ? 2 : 1][kTopWords];
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    for (uint32_t g = blockIdx.x; g < total; g += gridDim.x) {
+    const uint32_t count = !FUSE && bd.rlist ? *bd.rcount : total;
+    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+        const uint32_t g = !FUSE && bd.rlist ? bd.rlist[i] : i;
         const int m = find_segment(bd.cta_off, bd.n, g);
         const MeshDev &md = bd.mesh[m];
         const Pyramid &py = md.py;
         uint64_t *__restrict__ bits = md.bits;
         uint32_t *__restrict__ pre = md.pre;
         const uint32_t b = g - bd.cta_off[m];
-        if (md.regions && !bd.rflag[g]) {  // the same for the whole CTA
-            bits[py.woff[1] + (uint64_t)b * 256 + t] = 0;
-            if (t < 32) bits[py.woff[2] + (uint64_t)b * 32 + t] = 0;
-            if (t < 4) bits[py.woff[3] + (uint64_t)b * 4 + t] = 0;
-            if (t < 4) md.base[(uint64_t)t * md.bstride + b] = 0;
-            if (t == 0) reinterpret_cast<uint32_t *>(bits + py.woff[4])[b] = 0;
-        } else {
+        {
             const uint4 *src = reinterpret_cast<const uint4 *>(bits + py.woff[0] + (uint64_t)b * 2048 + t * 8);
             uint64_t w1 = 0;
             uint32_t c0 = 0, first = 0;  // first: bit of the block
@@ -656,13 +652,18 @@ __global__ void __launch_bounds__(256) k_compact(CompactBatch cb, const __grid_c
     compact_word(ONE ? one : cb.job[j], l, w, v);
 }
 
-// Levels 1 and 2 of a region-mode mesh, region by region (a block takes
-// level-0 regions in turn): the 256 level-1 and 32 level-2 words above a
-// region lie inside it, so an unflagged region (most of them at res 2048)
-// costs one flag read.
-__global__ void __launch_bounds__(256) k_compact_regions(const __grid_constant__ CompactJob job, uint32_t regions) {
-    for (uint32_t rg = blockIdx.x; rg < regions; rg += gridDim.x) {
-        if (!job.rflag[rg]) continue;
+// Levels 1 and 2 of a region-mode mesh, listed region by listed region (a
+// block takes them in turn): the 256 level-1 and 32 level-2 words above a
+// region lie inside it, and the unflagged ones (most of them at res 2048) hold
+// none.  The list is the batch's: the mesh's own regions are cta0 on.
+__global__ void __launch_bounds__(256) k_compact_regions(const __grid_constant__ CompactJob job,
+                                                         const uint32_t *__restrict__ rlist,
+                                                         const uint32_t *__restrict__ rcount, uint32_t cta0,
+                                                         uint32_t regions) {
+    const uint32_t count = *rcount;
+    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+        const uint32_t rg = rlist[i] - cta0;  // wraps for the meshes before
+        if (rg >= regions) continue;
         const uint64_t w1 = (uint64_t)rg * 256 + threadIdx.x;
         compact_word(job, 1, w1, job.bits[job.py.woff[1] + w1]);
         if (threadIdx.x < 32 && job.l1 > 2) {  // a two-voxel octree's top is level 1
@@ -1294,9 +1295,11 @@ cudaError_t launch_compact(const CompactBatch &c, const CompactJob *one, uint64_
     return cudaGetLastError();
 }
 
-cudaError_t launch_compact_regions(const CompactJob &job, uint32_t regions, int num_sms, cudaStream_t st) {
+cudaError_t launch_compact_regions(const CompactJob &job, const uint32_t *rlist, const uint32_t *rcount, uint32_t cta0,
+                                   uint32_t regions, int num_sms, cudaStream_t st) {
     if (regions == 0) return cudaSuccess;
-    k_compact_regions<<<std::min<uint32_t>(regions, (uint32_t)num_sms * 8), 256, 0, st>>>(job, regions);
+    k_compact_regions<<<std::min<uint32_t>(regions, (uint32_t)num_sms * 8), 256, 0, st>>>(job, rlist, rcount, cta0,
+                                                                                         regions);
     count_launches(1);
     return cudaGetLastError();
 }

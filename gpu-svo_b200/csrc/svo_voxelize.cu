@@ -189,17 +189,26 @@ __global__ void __launch_bounds__(256) k_front(BatchDev bd, const __grid_constan
         return;
     }
     const uint32_t zb = blockIdx.x - bbox_blocks, nz = gridDim.x - bbox_blocks;
-    for (uint32_t i = zb * blockDim.x + threadIdx.x; i < flag_words; i += nz * blockDim.x)
-        reinterpret_cast<uint32_t *>(bd.rflag)[i] = 0;
+    if (flag_words) {  // some mesh is in region mode: its level 0 is not cleared here
+        for (uint32_t i = zb * blockDim.x + threadIdx.x; i < flag_words; i += nz * blockDim.x)
+            reinterpret_cast<uint32_t *>(bd.rflag)[i] = 0;
+        for (int m = 0; m < bd.n; ++m) {
+            const MeshDev &md = by_value ? one : bd.mesh[m];
+            if (!md.regions) continue;
+            const uint64_t end = md.py.total_words, step = (uint64_t)nz * blockDim.x;
+            for (uint64_t i = md.py.woff[3] + 4ull * md.py.ctas + zb * blockDim.x + threadIdx.x; i < end; i += step)
+                md.bits[i] = 0;
+        }
+        if (by_value) return;  // (65,536 regions at res 2048: looking through them took 25 us)
+    }
     for (uint32_t g = zb; g < regions; g += nz) {
         const int m = by_value ? 0 : find_segment(bd.cta_off, bd.n, g);
         const MeshDev &md = by_value ? one : bd.mesh[m];
+        if (md.regions) continue;
         const uint32_t r = by_value ? g : g - bd.cta_off[m];
-        if (!md.regions) {
-            uint4 *w = reinterpret_cast<uint4 *>(md.bits + md.py.woff[0] + (uint64_t)r * 2048);
+        uint4 *w = reinterpret_cast<uint4 *>(md.bits + md.py.woff[0] + (uint64_t)r * 2048);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) w[threadIdx.x + 256 * q] = make_uint4(0, 0, 0, 0);
-        }
+        for (int q = 0; q < 4; ++q) w[threadIdx.x + 256 * q] = make_uint4(0, 0, 0, 0);
         const uint64_t z0 = md.py.woff[3] + 4ull * md.py.ctas;
         for (uint64_t i = z0 + (uint64_t)r * 256 + threadIdx.x; i < md.py.total_words; i += (uint64_t)md.py.ctas * 256)
             md.bits[i] = 0;
@@ -1022,16 +1031,60 @@ __global__ void __launch_bounds__(256) k_region_mark(BatchDev bd, int64_t total)
     }
 }
 
-// Zeroes the flagged level-0 regions of the region-mode meshes, a persistent
-// grid taking the regions in turn.
-__global__ void __launch_bounds__(256) k_region_zero(BatchDev bd, uint32_t total) {
-    for (uint32_t g = blockIdx.x; g < total; g += gridDim.x) {
-        if (!bd.rflag[g]) continue;
-        const int m = find_segment(bd.cta_off, bd.n, g);
-        const MeshDev &md = bd.mesh[m];
-        uint4 *w = reinterpret_cast<uint4 *>(md.bits + md.py.woff[0] + (uint64_t)(g - bd.cta_off[m]) * 2048);
+// The level-0 regions of a batch with a region-mode mesh, 8 at a time per
+// block: the regions to read are listed (one append per 8), a region-mode
+// mesh's flagged ones zeroed at level 0, and its unflagged ones zeroed at levels
+// 1..4 and in the region sums, which the pyramid then need not visit.  At res
+// 2048 the heightfield reaches 3,170 of 65,536 regions; a block that looked at
+// every region in turn waited for one flag after another (clearing, region
+// pass, pyramid and compaction together 217 us, 127 with the list).
+constexpr uint32_t kRegionChunk = 8;
+
+__global__ void __launch_bounds__(256) k_region_prepare(BatchDev bd, uint32_t total) {
+    __shared__ uint32_t s_live, s_zero;  // bits of the chunk: listed; region mode and unflagged
+    const uint32_t t = threadIdx.x;
+    for (uint32_t g0 = blockIdx.x * kRegionChunk; g0 < total; g0 += gridDim.x * kRegionChunk) {
+        if (t < 32) {
+            const uint32_t g = g0 + t;
+            bool live = false, zero = false;
+            if (t < kRegionChunk && g < total) {
+                const bool flagged = bd.rflag[g] != 0;
+                zero = bd.mesh[find_segment(bd.cta_off, bd.n, g)].regions && !flagged;
+                live = !zero;
+            }
+            const uint32_t lm = __ballot_sync(0xFFFFFFFFu, live), zm = __ballot_sync(0xFFFFFFFFu, zero);
+            uint32_t at = 0;
+            if (t == 0 && lm) at = atomicAdd(bd.rcount, (uint32_t)__popc(lm));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            if (live) bd.rlist[at + __popc(lm & ((1u << t) - 1u))] = g;
+            if (t == 0) {
+                s_live = lm;
+                s_zero = zm;
+            }
+        }
+        __syncthreads();
+        const uint32_t lm = s_live, zm = s_zero;
+        for (uint32_t k = 0; k < kRegionChunk; ++k) {
+            if (!(((lm | zm) >> k) & 1u)) continue;
+            const uint32_t g = g0 + k;
+            const int m = find_segment(bd.cta_off, bd.n, g);
+            const MeshDev &md = bd.mesh[m];
+            const uint32_t b = g - bd.cta_off[m];
+            if ((lm >> k) & 1u) {
+                if (!md.regions) continue;  // cleared by k_front
+                uint4 *w = reinterpret_cast<uint4 *>(md.bits + md.py.woff[0] + (uint64_t)b * 2048);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) w[threadIdx.x + 256 * q] = make_uint4(0, 0, 0, 0);
+                for (int q = 0; q < 4; ++q) w[t + 256 * q] = make_uint4(0, 0, 0, 0);
+            } else {
+                uint64_t *bits = md.bits;
+                bits[md.py.woff[1] + (uint64_t)b * 256 + t] = 0;
+                if (t < 32) bits[md.py.woff[2] + (uint64_t)b * 32 + t] = 0;
+                else if (t < 36) bits[md.py.woff[3] + (uint64_t)b * 4 + (t - 32)] = 0;
+                else if (t < 40) md.base[(uint64_t)(t - 36) * md.bstride + b] = 0;
+                else if (t == 40) reinterpret_cast<uint32_t *>(bits + md.py.woff[4])[b] = 0;
+            }
+        }
+        __syncthreads();  // s_live, s_zero are rewritten by the next chunk
     }
 }
 
@@ -1044,7 +1097,8 @@ cudaError_t launch_regions(const BatchDev &b, int64_t total_tris, uint32_t total
         k_region_mark<<<blocks, 256, 0, st>>>(b, total_tris);
         count_launches(1);
     }
-    k_region_zero<<<std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 8), 256, 0, st>>>(b, total_ctas);
+    k_region_prepare<<<std::min<uint32_t>((total_ctas + kRegionChunk - 1) / kRegionChunk, (uint32_t)num_sms * 16), 256, 0, st>>>(
+        b, total_ctas);
     count_launches(1);
     return cudaGetLastError();
 }
