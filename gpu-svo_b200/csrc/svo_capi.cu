@@ -732,12 +732,16 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 }
                 tm.mark(StageTimer::kDedup0, ds);
                 // early starts hold their candidate bitmaps (R^3 / 8 bytes each) until their
-                // finish: up to 4 GiB of them; the other meshes start just before they finish
+                // finish: up to 4 GiB of them; the other meshes start just before they
+                // finish, and so do grids above 1024: their candidate pass (110 us at res
+                // 2048) holds the compaction up (60 us beside it, 7 without), while their
+                // dedup ends long before the emission
                 uint64_t early = 0;
                 for (int j = 0; j < n; ++j) {
                     const MeshHost &mh = b->m[wave[j]];
                     const uint64_t R = 1ull << (mh.py.grid_levels - 1);
-                    if (j > 0 && early + R * R * R / 8 > (4ull << 30)) break;
+                    if (R > 1024) continue;
+                    if (early + R * R * R / 8 > (4ull << 30)) break;
                     early += R * R * R / 8;
                     dedup_start(j);
                 }
@@ -913,10 +917,11 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
             }
             // the wave's tables: one block, one upload; what one kernel takes by
             // value (a lone mesh's compaction job and emission) needs none
-            const bool lone_job = jobs.size() == 1;
+            const bool lone_job = jobs.size() == 1, lone_keys = kjobs.size() == 1;
             HostPack wt;
             const size_t p_jobs = lone_job ? 0 : wt.add(jobs), p_woff = lone_job ? 0 : wt.add(word_off),
-                         p_kjobs = wt.add(kjobs), p_boff = kjobs.empty() ? 0 : wt.add(blk_off),
+                         p_kjobs = lone_keys ? 0 : wt.add(kjobs),
+                         p_boff = kjobs.empty() || lone_keys ? 0 : wt.add(blk_off),
                          p_eps = wt.add(ep_small), p_offs = ep_small.empty() ? 0 : wt.add(off_small);
             unsigned char *dwt = wt.buf.empty() ? nullptr : S.get<unsigned char>(wt.buf.size());
             if (S.err != cudaSuccess) {
@@ -933,12 +938,24 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
             check(launch_compact(CompactBatch{d_jobs, (int)jobs.size(), d_word_off}, lone_job ? &jobs[0] : nullptr,
                                  word_off.back(), st),
                   "compact");
+            // The keys need the level-3 lists and nothing needs the keys: they run on
+            // a stream of their own beside the remaining lists and the emission (320
+            // triangles at res 512 420 us before, 414 this way; heightfield at res
+            // 2048, with the later dedup start above, 4,076 and 4,046).
+            AuxStreams *kset = kjobs.empty() ? nullptr : aux_acquire(ctx);
+            const cudaStream_t ks = kset ? kset->s[0] : st;
+            if (kset) {
+                check(cudaEventRecord(kset->fork, st), "fork");
+                check(cudaStreamWaitEvent(ks, kset->fork, 0), "fork");
+            }
+            if (!kjobs.empty())
+                check(launch_compact_keys(KeyBatch{d_kjobs, (int)kjobs.size(), d_blk_off}, lone_keys ? &kjobs[0] : nullptr,
+                                          blk_off.back(), ks),
+                      "keys");
             for (size_t i = 0; i < region_jobs.size(); ++i)
                 check(launch_compact_regions(region_jobs[i], b->rlist, b->rcount, region_range[i].first,
                                              region_range[i].second, ctx->num_sms, st),
                       "compact");
-            if (!kjobs.empty())
-                check(launch_compact_keys(KeyBatch{d_kjobs, (int)kjobs.size(), d_blk_off}, blk_off.back(), st), "keys");
             tm.mark(StageTimer::kCompact, st);
             // The dedup keys read only the bitmaps and code lists: they run on
             // a stream of their own, forked here, while the emission writes.
@@ -991,6 +1008,11 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 tm.mark(StageTimer::kDedup, ds);
             }
             join_dedup();
+            if (kset) {
+                check(cudaEventRecord(kset->join[0], ks), "join");
+                check(cudaStreamWaitEvent(st, kset->join[0], 0), "join");
+                aux_release(ctx, kset);
+            }
             check(cudaStreamSynchronize(st), "emit phase");
             bool more = false;  // work launched after this wait
             for (int j = 0; j < n && rc == SVO_OK; ++j) {

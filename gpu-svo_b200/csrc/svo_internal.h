@@ -236,7 +236,8 @@ cudaError_t launch_scan_stalled(const uint32_t *in, uint32_t *out, uint64_t n, u
 cudaError_t pool_malloc(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t st);
 // one: the job of a one-job batch (host copy, passed by value), or null.
 cudaError_t launch_compact(const CompactBatch &c, const CompactJob *one, uint64_t total_words, cudaStream_t st);
-cudaError_t launch_compact_keys(const KeyBatch &k, uint64_t total_blocks, cudaStream_t st);
+// one: the job of a one-job batch (host copy, passed by value), or null.
+cudaError_t launch_compact_keys(const KeyBatch &k, const KeyJob *one, uint64_t total_blocks, cudaStream_t st);
 // Levels 1 and 2 of a region-mode job (job.rflag set): its regions are those of
 // the batch's list (BatchDev) from cta0 on.
 cudaError_t launch_compact_regions(const CompactJob &job, const uint32_t *rlist, const uint32_t *rcount, uint32_t cta0,

@@ -676,7 +676,10 @@ __global__ void __launch_bounds__(256) k_compact_regions(const __grid_constant__
 // Level-0 set bits (the surface-voxel keys) from the non-empty 512-bit blocks
 // only: a mesh's level-3 code list is exactly its non-empty level-0 blocks,
 // in order.  8 lanes per block, one word each.
-__global__ void __launch_bounds__(256) k_compact_keys(KeyBatch kb, uint64_t total_blocks) {
+// ONE: a single job, passed by value.
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_compact_keys(KeyBatch kb, const __grid_constant__ KeyJob one,
+                                                      uint64_t total_blocks) {
     __shared__ uint16_t stage[8][2048];  // a warp's 4 blocks x 512 bits
     const uint64_t gi = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const uint64_t item = gi >> 3;
@@ -686,9 +689,9 @@ __global__ void __launch_bounds__(256) k_compact_keys(KeyBatch kb, uint64_t tota
     uint32_t r = 0;
     int j = 0;
     if (item < total_blocks) {
-        j = find_segment(kb.blk_off, kb.n, item);
-        const KeyJob &job = kb.job[j];
-        blk = job.blocks[item - kb.blk_off[j]];
+        if (!ONE) j = find_segment(kb.blk_off, kb.n, item);
+        const KeyJob &job = ONE ? one : kb.job[j];
+        blk = job.blocks[ONE ? item : item - kb.blk_off[j]];
         v = job.bits[blk * 8 + sub];
         r = job.rank.base[blk >> 8] + job.rank.pre[blk];
     }
@@ -702,8 +705,8 @@ __global__ void __launch_bounds__(256) k_compact_keys(KeyBatch kb, uint64_t tota
     // the warp's blocks are consecutive non-empty blocks of one mesh (its
     // outputs one range) unless it straddles two meshes
     const int j0 = __shfl_sync(0xFFFFFFFFu, j, 0);
-    if (__all_sync(0xFFFFFFFFu, item >= total_blocks || j == j0)) {
-        warp_codes(kb.job[j0].out, item < total_blocks ? r + x - pc : 0xFFFFFFFFu, pc, v, (blk * 8 + sub) * 64,
+    if (ONE || __all_sync(0xFFFFFFFFu, item >= total_blocks || j == j0)) {
+        warp_codes((ONE ? one : kb.job[j0]).out, item < total_blocks ? r + x - pc : 0xFFFFFFFFu, pc, v, (blk * 8 + sub) * 64,
                    stage[threadIdx.x >> 5], threadIdx.x & 31);
         return;
     }
@@ -1304,9 +1307,11 @@ cudaError_t launch_compact_regions(const CompactJob &job, const uint32_t *rlist,
     return cudaGetLastError();
 }
 
-cudaError_t launch_compact_keys(const KeyBatch &k, uint64_t total_blocks, cudaStream_t st) {
+cudaError_t launch_compact_keys(const KeyBatch &k, const KeyJob *one, uint64_t total_blocks, cudaStream_t st) {
     if (total_blocks == 0) return cudaSuccess;
-    k_compact_keys<<<(unsigned)((total_blocks * 8 + 255) / 256), 256, 0, st>>>(k, total_blocks);
+    const unsigned blocks = (unsigned)((total_blocks * 8 + 255) / 256);
+    if (one) k_compact_keys<true><<<blocks, 256, 0, st>>>(k, *one, total_blocks);
+    else k_compact_keys<false><<<blocks, 256, 0, st>>>(k, KeyJob{}, total_blocks);
     count_launches(1);
     return cudaGetLastError();
 }
