@@ -492,16 +492,16 @@ int batch_phase_a(svo_batch *b) {
     const uint64_t *d_tri_off = reinterpret_cast<const uint64_t *>(dt + p_tri);
     const uint32_t *d_cta_off = reinterpret_cast<const uint32_t *>(dt + p_cta);
     const uint32_t *d_bbox_off = reinterpret_cast<const uint32_t *>(dt + p_bbox);
-    if (n > 1)  // a lone mesh's table goes with the first kernel
+    if (n > 1)  // a lone mesh's table is passed to the kernels by value
         SVO_TRY(cudaMemcpyAsync(dt, tables.buf.data(), tables.buf.size(), cudaMemcpyHostToDevice, st), "upload meshes");
-    const BatchDev bd{b->d_mesh, n, d_tri_off, d_cta_off, d_bbox_off, rflag, any_regions ? b->rlist : nullptr, b->rcount};
+    const BatchDev bd{b->d_mesh, n, d_tri_off, d_cta_off, d_bbox_off, rflag, any_regions ? b->rlist : nullptr, b->rcount,
+                      n == 1 ? &b->h_mesh[0] : nullptr};
     const bool strict = (b->flags & SVO_FLAG_STRICT_FP) != 0;
     StageTimer tm((b->flags & SVO_FLAG_TIMINGS) != 0);
     for (int attempt = 0; attempt < 2; ++attempt) {
         tm.mark(StageTimer::kStart, st);
         SVO_TRY(cudaMemsetAsync(meta, 0, ml.bytes, st), "memset meta");
-        SVO_TRY(launch_front(bd, n == 1 ? &b->h_mesh[0] : nullptr, bblocks, ctas, any_regions, ctx->num_sms, st),
-                "bounding cube");
+        SVO_TRY(launch_front(bd, bblocks, ctas, any_regions, ctx->num_sms, st), "bounding cube");
         tm.mark(StageTimer::kBbox, st);
         if (any_regions) SVO_TRY(launch_regions(bd, (int64_t)tris, ctas, ctx->num_sms, st), "zero regions");
         SVO_TRY(launch_voxelize(bd, (int64_t)tris, strict, b->tune, big, big_cap, counters, ctx->num_sms, st),

@@ -125,9 +125,6 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
     MeshOut *report = c.take<MeshOut>(1);
     uint32_t *counters = c.take<uint32_t>(4);
     uint32_t *done = c.take<uint32_t>(1);
-    MeshDev *d_mesh = c.take<MeshDev>(1);
-    uint64_t *d_tri_off = c.take<uint64_t>(2);
-    uint32_t *d_cta_off = c.take<uint32_t>(2);
     uint64_t *bits = c.take<uint64_t>(py.total_words);
     uint32_t *pre = c.take<uint32_t>(py.total_blocks);
     const uint32_t bstride = (py.ctas + 3) & ~3u;
@@ -144,7 +141,7 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
         if ((rc = cuda(cudaStreamSynchronize(st)))) return rc;
         if (h[0] < 0 || h[1] >= n_points) return noalloc_fail(SVO_ERR_INVALID_ARGUMENT, "triangle index out of range");
     }
-    // the one-mesh table, passed by value to the first kernel
+    // the one-mesh table, passed to the kernels by value
     MeshDev md{};
     md.pts = points;
     md.tris = tris;
@@ -166,8 +163,10 @@ extern "C" int svo_voxelize_keys_noalloc(const float *points, int64_t n_points, 
     md.py = py;
     // everything that must start at zero (the array keeps the last call's data)
     if ((rc = cuda(cudaMemsetAsync(base, 0, c.used, st)))) return rc;
-    const BatchDev bd{d_mesh, 1, d_tri_off, d_cta_off, nullptr};
-    if ((rc = cuda(launch_front(bd, &md, bbox_blocks(n_points), 0, false, num_sms, st)))) return rc;
+    BatchDev bd{};
+    bd.n = 1;
+    bd.one = &md;
+    if ((rc = cuda(launch_front(bd, bbox_blocks(n_points), 0, false, num_sms, st)))) return rc;
     VoxTuning tune;
     tune.warp_max = 0xFFFFFFFFu;  // no big-triangle queue: warps take every large triangle
     if ((rc = cuda(launch_voxelize(bd, nt, (flags & SVO_FLAG_STRICT_FP) != 0, tune, nullptr, 0, counters,

@@ -229,8 +229,10 @@ __device__ __forceinline__ void finish_top(const MeshDev &md, uint64_t (*s_top)[
 // instead of 8) cost the streaming pass more than the launch saves.
 constexpr uint32_t kFuseRegions = 1024;
 
-template <bool FUSE>
-__global__ void __launch_bounds__(256, FUSE ? 4 : 8) k_pyramid(BatchDev bd, uint32_t total) {
+template <bool FUSE, bool ONE>
+__global__ void __launch_bounds__(256, FUSE ? 4 : 8) k_pyramid(const __grid_constant__ BatchDev bd,
+                                                               const __grid_constant__ MeshDev one, uint32_t total) {
+    const Meshes<ONE> mesh{bd, one};
     __shared__ uint64_t s1[256];
     __shared__ uint64_t s2[32];
     __shared__ uint64_t s3[4];
@@ -241,12 +243,12 @@ __global__ void __launch_bounds__(256, FUSE ? 4 : 8) k_pyramid(BatchDev bd, uint
     const uint32_t count = !FUSE && bd.rlist ? *bd.rcount : total;
     for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
         const uint32_t g = !FUSE && bd.rlist ? bd.rlist[i] : i;
-        const int m = find_segment(bd.cta_off, bd.n, g);
-        const MeshDev &md = bd.mesh[m];
+        const int m = mesh.of_region(g);
+        const MeshDev &md = mesh[m];
         const Pyramid &py = md.py;
         uint64_t *__restrict__ bits = md.bits;
         uint32_t *__restrict__ pre = md.pre;
-        const uint32_t b = g - bd.cta_off[m];
+        const uint32_t b = g - mesh.first_region(m);
         {
             const uint4 *src = reinterpret_cast<const uint4 *>(bits + py.woff[0] + (uint64_t)b * 2048 + t * 8);
             uint64_t w1 = 0;
@@ -343,10 +345,13 @@ __global__ void __launch_bounds__(256, FUSE ? 4 : 8) k_pyramid(BatchDev bd, uint
 
 // The region sums' prefixes (CTAs 0..3 of a mesh, one level each) and levels
 // 5.. (CTA 4) of every mesh.
-__global__ void __launch_bounds__(1024) k_pyramid_finish(BatchDev bd) {
+template <bool ONE>
+__global__ void __launch_bounds__(1024) k_pyramid_finish(const __grid_constant__ BatchDev bd,
+                                                         const __grid_constant__ MeshDev one) {
     __shared__ __align__(16) uint64_t s_top[2][kTopWords];
     __shared__ uint32_t s_warp[32];
-    const MeshDev &md = bd.mesh[blockIdx.y];
+    const Meshes<ONE> mesh{bd, one};
+    const MeshDev &md = mesh[blockIdx.y];
     if (blockIdx.x < 4) scan_regions<1024, 16>(md, (int)blockIdx.x, s_warp);
     else finish_top<1024>(md, s_top, s_warp);
 }
@@ -1238,13 +1243,22 @@ cudaError_t unique_impl(const T *in, uint64_t n, T *out, uint32_t *tile_counts, 
 
 cudaError_t launch_pyramid(const BatchDev &b, uint32_t total_ctas, uint32_t max_ctas, int num_sms, cudaStream_t st) {
     if (total_ctas == 0) return cudaSuccess;
+    const MeshDev one = b.one ? *b.one : MeshDev{};
     if (max_ctas <= kFuseRegions && total_ctas <= (uint32_t)num_sms * 8) {
-        k_pyramid<true><<<std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 4), 256, 0, st>>>(b, total_ctas);
+        const uint32_t blocks = std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 4);
+        if (b.one) k_pyramid<true, true><<<blocks, 256, 0, st>>>(b, one, total_ctas);
+        else k_pyramid<true, false><<<blocks, 256, 0, st>>>(b, one, total_ctas);
         count_launches(1);
         return cudaGetLastError();
     }
-    k_pyramid<false><<<std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 8), 256, 0, st>>>(b, total_ctas);
-    k_pyramid_finish<<<dim3(5, b.n), 1024, 0, st>>>(b);
+    const uint32_t blocks = std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 8);
+    if (b.one) {
+        k_pyramid<false, true><<<blocks, 256, 0, st>>>(b, one, total_ctas);
+        k_pyramid_finish<true><<<dim3(5, b.n), 1024, 0, st>>>(b, one);
+    } else {
+        k_pyramid<false, false><<<blocks, 256, 0, st>>>(b, one, total_ctas);
+        k_pyramid_finish<false><<<dim3(5, b.n), 1024, 0, st>>>(b, one);
+    }
     count_launches(2);
     return cudaGetLastError();
 }

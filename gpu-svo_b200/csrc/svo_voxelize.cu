@@ -160,32 +160,16 @@ __device__ __forceinline__ void grid_setup(const MeshDev &md) {
 //     in region mode (those clear their flagged regions later), the level-0
 //     region flags, and the words the pyramid does not write whole (level-3
 //     padding, level 4, which it writes as 32-bit halves, and levels >= 5).
-// A lone mesh's table travels by value (`one`) and is stored for the later
-// kernels here, which saves its upload.  (One kernel instead of the five
-// launches it replaces: a launch costs about 4 us in a small build, where the
-// host's launches are the critical path.)
-__global__ void __launch_bounds__(256) k_front(BatchDev bd, const __grid_constant__ MeshDev one, int by_value,
+// (One kernel instead of the five launches it replaces: a launch costs about
+// 4 us in a small build, where the host's launches are the critical path.)
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_front(const __grid_constant__ BatchDev bd, const __grid_constant__ MeshDev one,
                                                uint32_t bbox_blocks, uint32_t regions, uint32_t flag_words) {
+    const Meshes<ONE> mesh{bd, one};
     if (blockIdx.x < bbox_blocks) {
-        const int m = by_value ? 0 : find_segment(bd.bbox_off, bd.n, (uint32_t)blockIdx.x);
-        if (by_value && blockIdx.x == 0 && threadIdx.x == 0) {
-            *const_cast<MeshDev *>(bd.mesh) = one;
-            auto *tri = const_cast<uint64_t *>(bd.tri_off);
-            auto *cta = const_cast<uint32_t *>(bd.cta_off);
-            tri[0] = 0;
-            tri[1] = (uint64_t)one.n_tris;
-            cta[0] = 0;
-            cta[1] = one.py.ctas;
-        }
-        const uint32_t b0 = by_value ? 0u : bd.bbox_off[m];
-        const uint32_t nb = by_value ? bbox_blocks : bd.bbox_off[m + 1] - b0;
-        // (two calls: the by-value table is read from the constant bank)
-        if (by_value) {
-            if (bbox_block(one, blockIdx.x - b0, nb) && threadIdx.x == 0) grid_setup(one);
-        } else {
-            const MeshDev &md = bd.mesh[m];
-            if (bbox_block(md, blockIdx.x - b0, nb) && threadIdx.x == 0) grid_setup(md);
-        }
+        const int m = ONE ? 0 : find_segment(bd.bbox_off, bd.n, (uint32_t)blockIdx.x);
+        const uint32_t b0 = ONE ? 0u : bd.bbox_off[m], nb = ONE ? bbox_blocks : bd.bbox_off[m + 1] - b0;
+        if (bbox_block(mesh[m], blockIdx.x - b0, nb) && threadIdx.x == 0) grid_setup(mesh[m]);
         return;
     }
     const uint32_t zb = blockIdx.x - bbox_blocks, nz = gridDim.x - bbox_blocks;
@@ -193,19 +177,19 @@ __global__ void __launch_bounds__(256) k_front(BatchDev bd, const __grid_constan
         for (uint32_t i = zb * blockDim.x + threadIdx.x; i < flag_words; i += nz * blockDim.x)
             reinterpret_cast<uint32_t *>(bd.rflag)[i] = 0;
         for (int m = 0; m < bd.n; ++m) {
-            const MeshDev &md = by_value ? one : bd.mesh[m];
+            const MeshDev &md = mesh[m];
             if (!md.regions) continue;
             const uint64_t end = md.py.total_words, step = (uint64_t)nz * blockDim.x;
             for (uint64_t i = md.py.woff[3] + 4ull * md.py.ctas + zb * blockDim.x + threadIdx.x; i < end; i += step)
                 md.bits[i] = 0;
         }
-        if (by_value) return;  // (65,536 regions at res 2048: looking through them took 25 us)
+        if (ONE) return;  // (65,536 regions at res 2048: looking through them took 25 us)
     }
     for (uint32_t g = zb; g < regions; g += nz) {
-        const int m = by_value ? 0 : find_segment(bd.cta_off, bd.n, g);
-        const MeshDev &md = by_value ? one : bd.mesh[m];
+        const int m = mesh.of_region(g);
+        const MeshDev &md = mesh[m];
         if (md.regions) continue;
-        const uint32_t r = by_value ? g : g - bd.cta_off[m];
+        const uint32_t r = g - mesh.first_region(m);
         uint4 *w = reinterpret_cast<uint4 *>(md.bits + md.py.woff[0] + (uint64_t)r * 2048);
 #pragma unroll
         for (int q = 0; q < 4; ++q) w[threadIdx.x + 256 * q] = make_uint4(0, 0, 0, 0);
@@ -649,8 +633,8 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t v, int lane) {
 // q (degenerate or subnormal normals: |q| < 1e-15, where products of two such
 // distances could underflow) the whole column is taken.
 // Tri's 39-word stride is odd: distinct triangles fall in distinct banks.
-template <bool S>
-__device__ __forceinline__ void warp_columns(const BatchDev &bd, const Tri *st, const int *sm, uint32_t *pend, uint32_t c0,
+template <bool S, bool ONE>
+__device__ __forceinline__ void warp_columns(const Meshes<ONE> &mesh, const Tri *st, const int *sm, uint32_t *pend, uint32_t c0,
                                              uint32_t cnt, int lane) {
     const uint32_t incl = warp_inclusive(cnt, lane);
     const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
@@ -660,7 +644,7 @@ __device__ __forceinline__ void warp_columns(const BatchDev &bd, const Tri *st, 
         const bool on = (uint32_t)lane < n;
         const uint32_t bw = on ? pend[lane] : pend[0];
         const Tri &t = st[bw >> 27];
-        const MeshDev &md = bd.mesh[sm[bw >> 27]];
+        const MeshDev &md = mesh[sm[bw >> 27]];
         const float unit[3] = {md.gp->unit[0], md.gp->unit[1], md.gp->unit[2]};
         brick_lanes<S>(t, unit, reinterpret_cast<uint32_t *>(md.bits), (int)(bw & 511u), (int)((bw >> 9) & 511u),
                        (int)((bw >> 18) & 511u), on);
@@ -676,7 +660,7 @@ __device__ __forceinline__ void warp_columns(const BatchDev &bd, const Tri *st, 
         int k0 = 0;
         if (item < total) {
             const Tri &t = st[src];
-            const GridParams *gp = bd.mesh[sm[src]].gp;
+            const GridParams *gp = mesh[sm[src]].gp;
             const float u[3] = {gp->unit[0], gp->unit[1], gp->unit[2]};
             const int d = column_axis(t, u), i = d == 2 ? 0 : d + 1, j = d == 0 ? 2 : d - 1;
             const int p = i;  // the projection along d: XY (0), YZ (1), ZX (2)
@@ -736,7 +720,7 @@ __device__ __forceinline__ void warp_columns(const BatchDev &bd, const Tri *st, 
                           bz = d == 0 ? bj : d == 1 ? bi : kz;
                 const int lo[3] = {max(4 * bx, t.lo[0]), max(4 * by, t.lo[1]), max(4 * bz, t.lo[2])};
                 const int hi[3] = {min(4 * bx + 3, t.hi[0]), min(4 * by + 3, t.hi[1]), min(4 * bz + 3, t.hi[2])};
-                live = !t.cull || !brick_reject<S>(t, bd.mesh[sm[ts]].gp->unit, lo, hi);
+                live = !t.cull || !brick_reject<S>(t, mesh[sm[ts]].gp->unit, lo, hi);
                 brick = (uint32_t)bx | (uint32_t)by << 9 | (uint32_t)bz << 18 | (uint32_t)ts << 27;
             }
             // ---- round 3: the survivors' voxels ----
@@ -764,10 +748,11 @@ __device__ __forceinline__ void warp_columns(const BatchDev &bd, const Tri *st, 
 //   tier 1 (larger): queue entries of at most `cols` brick columns for
 //     k_voxelize_columns, which balances them across the GPU; INPLACE (no
 //     queue), its columns are walked by this warp right away.
-template <bool S, bool INPLACE>
+template <bool S, bool INPLACE, bool ONE>
 __global__ void __launch_bounds__(256, INPLACE ? 2 : 3)
-    k_voxelize(BatchDev bd, int64_t total, uint32_t serial_max, uint32_t cols, uint4 *__restrict__ big, uint32_t big_cap,
+    k_voxelize(const __grid_constant__ BatchDev bd, const __grid_constant__ MeshDev one, int64_t total, uint32_t serial_max, uint32_t cols, uint4 *__restrict__ big, uint32_t big_cap,
                uint32_t *__restrict__ big_count) {
+    const Meshes<ONE> mesh{bd, one};
     __shared__ Tri s_tri[INPLACE ? 8 : 1][32];  // the warp's tier-1 triangles
     __shared__ int s_mesh[INPLACE ? 8 : 1][32];  // their meshes
     __shared__ uint32_t s_pend[INPLACE ? 8 : 1][64];
@@ -780,11 +765,11 @@ __global__ void __launch_bounds__(256, INPLACE ? 2 : 3)
         uint32_t ncol = 0;
         int tier = -1, m = 0;
         if (gid < total) {
-            m = find_segment(bd.tri_off, bd.n, (uint64_t)gid);
-            const MeshDev &md = bd.mesh[m];
+            m = mesh.of_tri((uint64_t)gid);
+            const MeshDev &md = mesh[m];
             const GridParams g = *md.gp;
             float p[3][3];
-            if (load_tri_checked(md.pts, md.tris, md.n_pts, gid - (int64_t)bd.tri_off[m], p)) {
+            if (load_tri_checked(md.pts, md.tris, md.n_pts, gid - (int64_t)mesh.first_tri(m), p)) {
                 tri_setup<S>(g, md.res, p[0], p[1], p[2], t);
                 const int nx = t.hi[0] - t.lo[0] + 1, ny = t.hi[1] - t.lo[1] + 1, nz = t.hi[2] - t.lo[2] + 1;
                 tier = nx <= 4 && ny <= 4 && nz <= kSerialDepth && (uint32_t)(nx * ny * nz) <= serial_max ? 0 : 1;
@@ -794,7 +779,7 @@ __global__ void __launch_bounds__(256, INPLACE ? 2 : 3)
             }
         }
         if (__any_sync(0xFFFFFFFFu, tier == 0)) {
-            const MeshDev &md = bd.mesh[m];
+            const MeshDev &md = mesh[m];
             const float unit[3] = {md.gp->unit[0], md.gp->unit[1], md.gp->unit[2]};
             serial_tile<S>(t, unit, reinterpret_cast<uint32_t *>(md.bits), tier == 0);
         }
@@ -807,7 +792,7 @@ __global__ void __launch_bounds__(256, INPLACE ? 2 : 3)
                 sm[lane] = m;
             }
             __syncwarp();
-            warp_columns<S>(bd, st, sm, s_pend[threadIdx.x >> 5], 0, ncol, lane);
+            warp_columns<S, ONE>(mesh, st, sm, s_pend[threadIdx.x >> 5], 0, ncol, lane);
             __syncwarp();  // st is rewritten by the next round
         } else {
             // one append per warp; entries past the queue's end are counted, not
@@ -829,10 +814,13 @@ __global__ void __launch_bounds__(256, INPLACE ? 2 : 3)
 // triangles on a 300 x 200 x 100 grid: 31 us, with a quarter of it 68); 16
 // columns per entry by default, since with 64 the last warps of a batch of 15
 // meshes work alone (140 us against 124 with 24 already).
-template <bool S>
-__global__ void __launch_bounds__(256, 2) k_voxelize_columns(BatchDev bd, const uint4 *__restrict__ big,
+template <bool S, bool ONE>
+__global__ void __launch_bounds__(256, 2) k_voxelize_columns(const __grid_constant__ BatchDev bd,
+                                                             const __grid_constant__ MeshDev one,
+                                                             const uint4 *__restrict__ big,
                                                              const uint32_t *__restrict__ big_count, uint32_t big_cap,
                                                              uint32_t *__restrict__ cursor) {
+    const Meshes<ONE> mesh{bd, one};
     __shared__ Tri s_tri[8][32];
     __shared__ int s_mesh[8][32];
     __shared__ uint32_t s_pend[8][64];
@@ -852,11 +840,11 @@ __global__ void __launch_bounds__(256, 2) k_voxelize_columns(BatchDev bd, const 
         if ((uint32_t)lane < chunk && e0 + lane < n) {
             const uint4 ent = big[e0 + lane];
             const int64_t gid = (int64_t)ent.x | ((int64_t)ent.w << 32);
-            const int m = find_segment(bd.tri_off, bd.n, (uint64_t)gid);
-            const MeshDev &md = bd.mesh[m];
+            const int m = mesh.of_tri((uint64_t)gid);
+            const MeshDev &md = mesh[m];
             const GridParams g = *md.gp;
             float p[3][3];
-            load_tri(md.pts, md.tris, gid - (int64_t)bd.tri_off[m], p);
+            load_tri(md.pts, md.tris, gid - (int64_t)mesh.first_tri(m), p);
             Tri t;
             tri_setup<S>(g, md.res, p[0], p[1], p[2], t);
             st[lane] = t;
@@ -865,7 +853,7 @@ __global__ void __launch_bounds__(256, 2) k_voxelize_columns(BatchDev bd, const 
             cnt = ent.z - ent.y;
         }
         __syncwarp();
-        warp_columns<S>(bd, st, sm, s_pend[threadIdx.x >> 5], c0, cnt, lane);
+        warp_columns<S, ONE>(mesh, st, sm, s_pend[threadIdx.x >> 5], c0, cnt, lane);
         __syncwarp();  // st is rewritten by the next chunk
     }
 }
@@ -941,11 +929,12 @@ cudaError_t launch_index_ranges(const IndexJob *jobs, int n, const uint32_t *blo
     return cudaGetLastError();
 }
 
-cudaError_t launch_front(const BatchDev &b, const MeshDev *one, uint32_t bbox_blocks, uint32_t total_ctas,
-                         bool any_regions, int num_sms, cudaStream_t st) {
-    const uint32_t zblocks = std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 8);
-    k_front<<<bbox_blocks + zblocks, 256, 0, st>>>(b, one ? *one : MeshDev{}, one ? 1 : 0, bbox_blocks, total_ctas,
-                                                   any_regions ? (total_ctas + 3) / 4 : 0);
+cudaError_t launch_front(const BatchDev &b, uint32_t bbox_blocks, uint32_t total_ctas, bool any_regions, int num_sms,
+                         cudaStream_t st) {
+    const uint32_t blocks = bbox_blocks + std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 8);
+    const uint32_t flag_words = any_regions ? (total_ctas + 3) / 4 : 0;
+    if (b.one) k_front<true><<<blocks, 256, 0, st>>>(b, *b.one, bbox_blocks, total_ctas, flag_words);
+    else k_front<false><<<blocks, 256, 0, st>>>(b, MeshDev{}, bbox_blocks, total_ctas, flag_words);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -966,7 +955,10 @@ namespace {
 // the same.
 constexpr int kMarkBatch = 3;
 
-__global__ void __launch_bounds__(256) k_region_mark(BatchDev bd, int64_t total) {
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_region_mark(const __grid_constant__ BatchDev bd, const __grid_constant__ MeshDev one,
+                                                     int64_t total) {
+    const Meshes<ONE> mesh{bd, one};
     int cur = -1;
     float org[3] = {0, 0, 0}, inv[3] = {0, 0, 0};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -978,17 +970,17 @@ __global__ void __launch_bounds__(256) k_region_mark(BatchDev bd, int64_t total)
         for (int k = 0; k < kMarkBatch; ++k) {
             const int64_t gid = g0 + k * stride;
             live[k] = gid < total;
-            mk[k] = live[k] ? find_segment(bd.tri_off, bd.n, (uint64_t)gid) : 0;
-            const MeshDev &md = bd.mesh[mk[k]];
+            mk[k] = live[k] ? mesh.of_tri((uint64_t)gid) : 0;
+            const MeshDev &md = mesh[mk[k]];
             live[k] = live[k] && md.regions != 0;
-            const int64_t t = gid - (int64_t)bd.tri_off[mk[k]];
+            const int64_t t = gid - (int64_t)mesh.first_tri(mk[k]);
 #pragma unroll
             for (int j = 0; j < 3; ++j) vi[k][j] = live[k] ? (md.tris ? (int64_t)__ldg(md.tris + 3 * t + j) : 3 * t + j) : 0;
         }
         float p[kMarkBatch][3][3];
 #pragma unroll
         for (int k = 0; k < kMarkBatch; ++k) {
-            const MeshDev &md = bd.mesh[mk[k]];
+            const MeshDev &md = mesh[mk[k]];
             // an index outside the mesh: skipped here, k_voxelize reports it
             live[k] = live[k] && (uint64_t)vi[k][0] < (uint64_t)md.n_pts && (uint64_t)vi[k][1] < (uint64_t)md.n_pts &&
                       (uint64_t)vi[k][2] < (uint64_t)md.n_pts;
@@ -1000,7 +992,7 @@ __global__ void __launch_bounds__(256) k_region_mark(BatchDev bd, int64_t total)
 #pragma unroll
         for (int k = 0; k < kMarkBatch; ++k) {
             if (!live[k]) continue;
-            const MeshDev &md = bd.mesh[mk[k]];
+            const MeshDev &md = mesh[mk[k]];
             if (mk[k] != cur) {
                 cur = mk[k];
                 // the one-voxel margin absorbs an approximate reciprocal (2 ulp)
@@ -1019,7 +1011,7 @@ __global__ void __launch_bounds__(256) k_region_mark(BatchDev bd, int64_t total)
                 lo[a] = clampi(f2i_rz(__fsub_rn(__fmul_rn(cminf(v0, cminf(v1, v2)), inv[a]), 1.0f)), 0, md.res[a] - 1);
                 hi[a] = clampi(f2i_rz(__fadd_rn(__fmul_rn(cmaxf(v0, cmaxf(v1, v2)), inv[a]), 1.0f)), 0, md.res[a] - 1);
             }
-            uint8_t *flag = bd.rflag + bd.cta_off[mk[k]];
+            uint8_t *flag = bd.rflag + mesh.first_region(mk[k]);
             // region bits: z at 3i, x at 3i + 1, y at 3i + 2 (z in 32-voxel, x and y in 64-voxel steps)
             for (uint32_t rz = (uint32_t)lo[2] >> 5; rz <= (uint32_t)hi[2] >> 5; ++rz)
                 for (uint32_t ry = (uint32_t)lo[1] >> 6; ry <= (uint32_t)hi[1] >> 6; ++ry)
@@ -1040,7 +1032,10 @@ __global__ void __launch_bounds__(256) k_region_mark(BatchDev bd, int64_t total)
 // pass, pyramid and compaction together 217 us, 127 with the list).
 constexpr uint32_t kRegionChunk = 8;
 
-__global__ void __launch_bounds__(256) k_region_prepare(BatchDev bd, uint32_t total) {
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_region_prepare(const __grid_constant__ BatchDev bd,
+                                                        const __grid_constant__ MeshDev one, uint32_t total) {
+    const Meshes<ONE> mesh{bd, one};
     __shared__ uint32_t s_live, s_zero;  // bits of the chunk: listed; region mode and unflagged
     const uint32_t t = threadIdx.x;
     for (uint32_t g0 = blockIdx.x * kRegionChunk; g0 < total; g0 += gridDim.x * kRegionChunk) {
@@ -1049,7 +1044,7 @@ __global__ void __launch_bounds__(256) k_region_prepare(BatchDev bd, uint32_t to
             bool live = false, zero = false;
             if (t < kRegionChunk && g < total) {
                 const bool flagged = bd.rflag[g] != 0;
-                zero = bd.mesh[find_segment(bd.cta_off, bd.n, g)].regions && !flagged;
+                zero = mesh[mesh.of_region(g)].regions && !flagged;
                 live = !zero;
             }
             const uint32_t lm = __ballot_sync(0xFFFFFFFFu, live), zm = __ballot_sync(0xFFFFFFFFu, zero);
@@ -1067,9 +1062,9 @@ __global__ void __launch_bounds__(256) k_region_prepare(BatchDev bd, uint32_t to
         for (uint32_t k = 0; k < kRegionChunk; ++k) {
             if (!(((lm | zm) >> k) & 1u)) continue;
             const uint32_t g = g0 + k;
-            const int m = find_segment(bd.cta_off, bd.n, g);
-            const MeshDev &md = bd.mesh[m];
-            const uint32_t b = g - bd.cta_off[m];
+            const int m = mesh.of_region(g);
+            const MeshDev &md = mesh[m];
+            const uint32_t b = g - mesh.first_region(m);
             if ((lm >> k) & 1u) {
                 if (!md.regions) continue;  // cleared by k_front
                 uint4 *w = reinterpret_cast<uint4 *>(md.bits + md.py.woff[0] + (uint64_t)b * 2048);
@@ -1094,11 +1089,13 @@ cudaError_t launch_regions(const BatchDev &b, int64_t total_tris, uint32_t total
                            cudaStream_t st) {
     if (total_tris > 0) {
         const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((total_tris + 255) / 256, (int64_t)num_sms * 8));
-        k_region_mark<<<blocks, 256, 0, st>>>(b, total_tris);
+        if (b.one) k_region_mark<true><<<blocks, 256, 0, st>>>(b, *b.one, total_tris);
+        else k_region_mark<false><<<blocks, 256, 0, st>>>(b, MeshDev{}, total_tris);
         count_launches(1);
     }
-    k_region_prepare<<<std::min<uint32_t>((total_ctas + kRegionChunk - 1) / kRegionChunk, (uint32_t)num_sms * 16), 256, 0, st>>>(
-        b, total_ctas);
+    const uint32_t blocks = std::min<uint32_t>((total_ctas + kRegionChunk - 1) / kRegionChunk, (uint32_t)num_sms * 16);
+    if (b.one) k_region_prepare<true><<<blocks, 256, 0, st>>>(b, *b.one, total_ctas);
+    else k_region_prepare<false><<<blocks, 256, 0, st>>>(b, MeshDev{}, total_ctas);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -1111,19 +1108,30 @@ cudaError_t launch_voxelize(const BatchDev &b, int64_t total, bool strict, const
         const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)num_sms * 16));
         const bool inplace = big == nullptr || big_cap == 0;
         const uint32_t cols = std::max<uint32_t>(1, tune.warp_max / 16);
-        if (strict) {
-            if (inplace) k_voxelize<true, true><<<blocks, 256, 0, st>>>(b, total, tune.serial_max, cols, big, big_cap, counters);
-            else k_voxelize<true, false><<<blocks, 256, 0, st>>>(b, total, tune.serial_max, cols, big, big_cap, counters);
+        const MeshDev one = b.one ? *b.one : MeshDev{};
+#define SVO_VOX(S_, I_, O_) \
+    k_voxelize<S_, I_, O_><<<blocks, 256, 0, st>>>(b, one, total, tune.serial_max, cols, big, big_cap, counters)
+#define SVO_COLS(S_, O_) \
+    k_voxelize_columns<S_, O_><<<num_sms * 2, 256, 0, st>>>(b, one, big, counters, big_cap, counters + 1)
+        if (inplace) {  // the allocation-free entry point: one mesh
+            if (!b.one) return cudaErrorInvalidValue;
+            if (strict) SVO_VOX(true, true, true); else SVO_VOX(false, true, true);
+        } else if (strict) {
+            if (b.one) SVO_VOX(true, false, true); else SVO_VOX(true, false, false);
         } else {
-            if (inplace) k_voxelize<false, true><<<blocks, 256, 0, st>>>(b, total, tune.serial_max, cols, big, big_cap, counters);
-            else k_voxelize<false, false><<<blocks, 256, 0, st>>>(b, total, tune.serial_max, cols, big, big_cap, counters);
+            if (b.one) SVO_VOX(false, false, true); else SVO_VOX(false, false, false);
         }
         count_launches(1);
         if (!inplace) {
-            if (strict) k_voxelize_columns<true><<<num_sms * 2, 256, 0, st>>>(b, big, counters, big_cap, counters + 1);
-            else k_voxelize_columns<false><<<num_sms * 2, 256, 0, st>>>(b, big, counters, big_cap, counters + 1);
+            if (strict) {
+                if (b.one) SVO_COLS(true, true); else SVO_COLS(true, false);
+            } else {
+                if (b.one) SVO_COLS(false, true); else SVO_COLS(false, false);
+            }
             count_launches(1);
         }
+#undef SVO_COLS
+#undef SVO_VOX
     }
     return cudaGetLastError();
 }
