@@ -104,6 +104,35 @@ struct BatchDev {
 };
 
 #if defined(__CUDACC__)
+// Chained launches.  A kernel launched by launch_chained may have its blocks
+// placed while the last blocks of the kernel before it on the stream are still
+// running; chain_begin(), the first thing every block of such a kernel does,
+// lets the next chained kernel in and then waits until everything before its
+// own kernel is complete and visible.  Since every block waits, a kernel that
+// is complete implies that all earlier ones are.  Used where a short kernel
+// follows another on the same stream: two plain launches are about 2 us apart.
+// With 320 triangles at 32^3 a build took 92.8 us and takes 83.6 this way, with
+// 20k at 128^3 120.8 and 108.9, with 5M at 2048^3 4,037 and 4,020.
+__device__ __forceinline__ void chain_begin() {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+}
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t shmem, cudaStream_t st,
+                                  const A &...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = shmem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // The meshes of a batch as a kernel sees them: the tables in device memory, or
 // (ONE) a lone mesh's table in the kernel's parameters, whose fields come from
 // the constant bank instead of a chain of loads at the start of every kernel

@@ -232,6 +232,7 @@ constexpr uint32_t kFuseRegions = 1024;
 template <bool FUSE, bool ONE>
 __global__ void __launch_bounds__(256, FUSE ? 4 : 8) k_pyramid(const __grid_constant__ BatchDev bd,
                                                                const __grid_constant__ MeshDev one, uint32_t total) {
+    chain_begin();
     const Meshes<ONE> mesh{bd, one};
     __shared__ uint64_t s1[256];
     __shared__ uint64_t s2[32];
@@ -350,6 +351,7 @@ __global__ void __launch_bounds__(1024) k_pyramid_finish(const __grid_constant__
                                                          const __grid_constant__ MeshDev one) {
     __shared__ __align__(16) uint64_t s_top[2][kTopWords];
     __shared__ uint32_t s_warp[32];
+    chain_begin();
     const Meshes<ONE> mesh{bd, one};
     const MeshDev &md = mesh[blockIdx.y];
     if (blockIdx.x < 4) scan_regions<1024, 16>(md, (int)blockIdx.x, s_warp);
@@ -640,6 +642,7 @@ __device__ __forceinline__ void compact_word(const CompactJob &job, int l, uint6
 template <bool ONE>
 __global__ void __launch_bounds__(256) k_compact(CompactBatch cb, const __grid_constant__ CompactJob one,
                                                  uint64_t total) {
+    chain_begin();
     const uint64_t gi = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (gi >= ((total + 31) & ~31ull)) return;  // whole warps stay for the shuffles
     uint64_t v = 0, w = 0;
@@ -665,6 +668,7 @@ __global__ void __launch_bounds__(256) k_compact_regions(const __grid_constant__
                                                          const uint32_t *__restrict__ rlist,
                                                          const uint32_t *__restrict__ rcount, uint32_t cta0,
                                                          uint32_t regions) {
+    chain_begin();
     const uint32_t count = *rcount;
     for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
         const uint32_t rg = rlist[i] - cta0;  // wraps for the meshes before
@@ -975,6 +979,7 @@ constexpr int kOwnBytes = 32 * 9 * 4;    // vertex owners (full neighbour tables
 template <bool S, bool FULL, bool VE, bool ONE>
 __global__ void __launch_bounds__(kEmitWarps * 32, FULL || VE ? 6 : 8)
     k_emit(EmitBatch eb, const __grid_constant__ EmitParams one, uint64_t total) {
+    chain_begin();
     extern __shared__ __align__(128) uint4 smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int kWarpBytes = kEmitBufBytes + (VE && FULL ? kOwnBytes : 0);
@@ -1246,18 +1251,18 @@ cudaError_t launch_pyramid(const BatchDev &b, uint32_t total_ctas, uint32_t max_
     const MeshDev one = b.one ? *b.one : MeshDev{};
     if (max_ctas <= kFuseRegions && total_ctas <= (uint32_t)num_sms * 8) {
         const uint32_t blocks = std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 4);
-        if (b.one) k_pyramid<true, true><<<blocks, 256, 0, st>>>(b, one, total_ctas);
-        else k_pyramid<true, false><<<blocks, 256, 0, st>>>(b, one, total_ctas);
+        if (b.one) launch_chained(k_pyramid<true, true>, blocks, 256, 0, st, b, one, total_ctas);
+        else launch_chained(k_pyramid<true, false>, blocks, 256, 0, st, b, one, total_ctas);
         count_launches(1);
         return cudaGetLastError();
     }
     const uint32_t blocks = std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 8);
     if (b.one) {
-        k_pyramid<false, true><<<blocks, 256, 0, st>>>(b, one, total_ctas);
-        k_pyramid_finish<true><<<dim3(5, b.n), 1024, 0, st>>>(b, one);
+        launch_chained(k_pyramid<false, true>, blocks, 256, 0, st, b, one, total_ctas);
+        launch_chained(k_pyramid_finish<true>, dim3(5, b.n), 1024, 0, st, b, one);
     } else {
-        k_pyramid<false, false><<<blocks, 256, 0, st>>>(b, one, total_ctas);
-        k_pyramid_finish<false><<<dim3(5, b.n), 1024, 0, st>>>(b, one);
+        launch_chained(k_pyramid<false, false>, blocks, 256, 0, st, b, one, total_ctas);
+        launch_chained(k_pyramid_finish<false>, dim3(5, b.n), 1024, 0, st, b, one);
     }
     count_launches(2);
     return cudaGetLastError();
@@ -1315,8 +1320,8 @@ cudaError_t launch_compact(const CompactBatch &c, const CompactJob *one, uint64_
 cudaError_t launch_compact_regions(const CompactJob &job, const uint32_t *rlist, const uint32_t *rcount, uint32_t cta0,
                                    uint32_t regions, int num_sms, cudaStream_t st) {
     if (regions == 0) return cudaSuccess;
-    k_compact_regions<<<std::min<uint32_t>(regions, (uint32_t)num_sms * 8), 256, 0, st>>>(job, rlist, rcount, cta0,
-                                                                                         regions);
+    launch_chained(k_compact_regions, std::min<uint32_t>(regions, (uint32_t)num_sms * 8), 256, 0, st, job, rlist, rcount,
+                   cta0, regions);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -1342,8 +1347,8 @@ cudaError_t launch_emit(const EmitBatch &b, const EmitParams *one, uint64_t tota
     const EmitParams p1 = one ? *one : EmitParams{};
 #define SVO_EMIT1(S_, F_, V_)                                                                       \
     do {                                                                                             \
-        if (one) k_emit<S_, F_, V_, true><<<blocks, kEmitWarps * 32, shmem, st>>>(b, p1, total);      \
-        else k_emit<S_, F_, V_, false><<<blocks, kEmitWarps * 32, shmem, st>>>(b, p1, total);        \
+        if (one) launch_chained(k_emit<S_, F_, V_, true>, blocks, kEmitWarps * 32, shmem, st, b, p1, total);   \
+        else launch_chained(k_emit<S_, F_, V_, false>, blocks, kEmitWarps * 32, shmem, st, b, p1, total);     \
     } while (0)
 #define SVO_EMIT(S_, F_, V_) SVO_EMIT1(S_, F_, V_)
     if (s) {

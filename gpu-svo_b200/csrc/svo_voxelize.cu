@@ -165,6 +165,7 @@ __device__ __forceinline__ void grid_setup(const MeshDev &md) {
 template <bool ONE>
 __global__ void __launch_bounds__(256) k_front(const __grid_constant__ BatchDev bd, const __grid_constant__ MeshDev one,
                                                uint32_t bbox_blocks, uint32_t regions, uint32_t flag_words) {
+    chain_begin();
     const Meshes<ONE> mesh{bd, one};
     if (blockIdx.x < bbox_blocks) {
         const int m = ONE ? 0 : find_segment(bd.bbox_off, bd.n, (uint32_t)blockIdx.x);
@@ -752,6 +753,7 @@ template <bool S, bool INPLACE, bool ONE>
 __global__ void __launch_bounds__(256, INPLACE ? 2 : 3)
     k_voxelize(const __grid_constant__ BatchDev bd, const __grid_constant__ MeshDev one, int64_t total, uint32_t serial_max, uint32_t cols, uint4 *__restrict__ big, uint32_t big_cap,
                uint32_t *__restrict__ big_count) {
+    chain_begin();
     const Meshes<ONE> mesh{bd, one};
     __shared__ Tri s_tri[INPLACE ? 8 : 1][32];  // the warp's tier-1 triangles
     __shared__ int s_mesh[INPLACE ? 8 : 1][32];  // their meshes
@@ -820,6 +822,7 @@ __global__ void __launch_bounds__(256, 2) k_voxelize_columns(const __grid_consta
                                                              const uint4 *__restrict__ big,
                                                              const uint32_t *__restrict__ big_count, uint32_t big_cap,
                                                              uint32_t *__restrict__ cursor) {
+    chain_begin();
     const Meshes<ONE> mesh{bd, one};
     __shared__ Tri s_tri[8][32];
     __shared__ int s_mesh[8][32];
@@ -958,6 +961,7 @@ constexpr int kMarkBatch = 3;
 template <bool ONE>
 __global__ void __launch_bounds__(256) k_region_mark(const __grid_constant__ BatchDev bd, const __grid_constant__ MeshDev one,
                                                      int64_t total) {
+    chain_begin();
     const Meshes<ONE> mesh{bd, one};
     int cur = -1;
     float org[3] = {0, 0, 0}, inv[3] = {0, 0, 0};
@@ -1035,6 +1039,7 @@ constexpr uint32_t kRegionChunk = 8;
 template <bool ONE>
 __global__ void __launch_bounds__(256) k_region_prepare(const __grid_constant__ BatchDev bd,
                                                         const __grid_constant__ MeshDev one, uint32_t total) {
+    chain_begin();
     const Meshes<ONE> mesh{bd, one};
     __shared__ uint32_t s_live, s_zero;  // bits of the chunk: listed; region mode and unflagged
     const uint32_t t = threadIdx.x;
@@ -1089,13 +1094,13 @@ cudaError_t launch_regions(const BatchDev &b, int64_t total_tris, uint32_t total
                            cudaStream_t st) {
     if (total_tris > 0) {
         const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((total_tris + 255) / 256, (int64_t)num_sms * 8));
-        if (b.one) k_region_mark<true><<<blocks, 256, 0, st>>>(b, *b.one, total_tris);
-        else k_region_mark<false><<<blocks, 256, 0, st>>>(b, MeshDev{}, total_tris);
+        if (b.one) launch_chained(k_region_mark<true>, blocks, 256, 0, st, b, *b.one, total_tris);
+        else launch_chained(k_region_mark<false>, blocks, 256, 0, st, b, MeshDev{}, total_tris);
         count_launches(1);
     }
     const uint32_t blocks = std::min<uint32_t>((total_ctas + kRegionChunk - 1) / kRegionChunk, (uint32_t)num_sms * 16);
-    if (b.one) k_region_prepare<true><<<blocks, 256, 0, st>>>(b, *b.one, total_ctas);
-    else k_region_prepare<false><<<blocks, 256, 0, st>>>(b, MeshDev{}, total_ctas);
+    if (b.one) launch_chained(k_region_prepare<true>, blocks, 256, 0, st, b, *b.one, total_ctas);
+    else launch_chained(k_region_prepare<false>, blocks, 256, 0, st, b, MeshDev{}, total_ctas);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -1110,9 +1115,10 @@ cudaError_t launch_voxelize(const BatchDev &b, int64_t total, bool strict, const
         const uint32_t cols = std::max<uint32_t>(1, tune.warp_max / 16);
         const MeshDev one = b.one ? *b.one : MeshDev{};
 #define SVO_VOX(S_, I_, O_) \
-    k_voxelize<S_, I_, O_><<<blocks, 256, 0, st>>>(b, one, total, tune.serial_max, cols, big, big_cap, counters)
+    launch_chained(k_voxelize<S_, I_, O_>, blocks, 256, 0, st, b, one, total, tune.serial_max, cols, big, big_cap, \
+                   counters)
 #define SVO_COLS(S_, O_) \
-    k_voxelize_columns<S_, O_><<<num_sms * 2, 256, 0, st>>>(b, one, big, counters, big_cap, counters + 1)
+    launch_chained(k_voxelize_columns<S_, O_>, num_sms * 2, 256, 0, st, b, one, big, counters, big_cap, counters + 1)
         if (inplace) {  // the allocation-free entry point: one mesh
             if (!b.one) return cudaErrorInvalidValue;
             if (strict) SVO_VOX(true, true, true); else SVO_VOX(false, true, true);
