@@ -214,8 +214,8 @@ __device__ __forceinline__ void finish_top(const MeshDev &md, uint64_t (*s_top)[
 // gets the set bits before it in its region (md.pre), and every region its
 // set bits of levels 0..3 (md.base), whose prefix over the regions completes
 // the rank -- there is no scan over the blocks (19.2M of them at res 2048:
-// that scan and the memset before it took 60 us, this scan of 4 x 65,536
-// region sums takes 7).  With a region-mode mesh in the batch only the listed
+// that scan and the memset before it took 60 us; the scan of 4 x 65,536 region
+// sums is part of k_pyramid_finish, 24 us in all).  With a region-mode mesh in the batch only the listed
 // regions are visited: the others are empty, not zeroed in memory at level 0
 // and dealt with by k_region_prepare.
 //

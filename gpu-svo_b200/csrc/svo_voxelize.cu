@@ -160,8 +160,12 @@ __device__ __forceinline__ void grid_setup(const MeshDev &md) {
 //     in region mode (those clear their flagged regions later), the level-0
 //     region flags, and the words the pyramid does not write whole (level-3
 //     padding, level 4, which it writes as 32-bit halves, and levels >= 5).
-// (One kernel instead of the five launches it replaces: a launch costs about
-// 4 us in a small build, where the host's launches are the critical path.)
+// (One kernel instead of the five launches it replaces: in a small build the
+// host's launches are the critical path.  The meta words are cleared by a memset
+// before it: cleared here, by one block up to 2,048 points and by a cluster of
+// eight up to 32,768, 320 triangles at 32^3 take 83.2 us against 83.1 and 30k
+// at 300 x 200 x 100 143.0 against 137.9, for eight blocks read the points
+// slower than the memset costs.)
 template <bool ONE>
 __global__ void __launch_bounds__(256) k_front(const __grid_constant__ BatchDev bd, const __grid_constant__ MeshDev one,
                                                uint32_t bbox_blocks, uint32_t regions, uint32_t flag_words) {
@@ -358,7 +362,7 @@ __device__ __forceinline__ uint32_t edge_fail_row(const float *cf, const float *
 // The hits of a slice pair (a bitmap word holds 4 x 4 x 2 voxels, and the walk
 // begins at an even z in every lane) are collected for the 2 x 2 bricks an
 // unaligned box can reach and written with at most four atomicOr.
-// Bound by issue (68% of the slots; setup 480 of 1,600 instructions a warp).
+// Bound by issue (68% of the slots).
 // One loop per lane over its own rows and voxels, with their early exits, costs
 // the warp its largest triangle's loops: 407 us for the 5M triangles (2-3
 // voxels across) of the heightfield at res 2048 against 336 us this way, 90
@@ -484,8 +488,8 @@ __device__ __forceinline__ bool brick_reject(const Tri &t, const float *unit, co
 
 // The bricks of 32 lanes at once, one per lane (on: the lane has one): the
 // serial tier's slices over an aligned 4x4x4 box, clipped to the triangle's
-// bbox.  About 1,100 instructions per 32 bricks; a brick per half-warp, a row
-// of it per lane, takes 130 per two (whole voxelizer of a batch of 15 meshes
+// bbox.  Bound by issue.  The form before, a brick per half-warp and a row of
+// it per lane, took more instructions a brick (whole voxelizer of a batch of 15 meshes
 // 177 us, 124 this way; torus soup 281 and 220).
 template <bool S>
 __device__ __forceinline__ void brick_lanes(const Tri &t, const float unit[3], uint32_t *__restrict__ bm, int sx, int sy,
@@ -751,7 +755,8 @@ __device__ __forceinline__ void warp_columns(const Meshes<ONE> &mesh, const Tri 
 //     queue), its columns are walked by this warp right away.
 template <bool S, bool INPLACE, bool ONE>
 __global__ void __launch_bounds__(256, INPLACE ? 2 : 3)
-    k_voxelize(const __grid_constant__ BatchDev bd, const __grid_constant__ MeshDev one, int64_t total, uint32_t serial_max, uint32_t cols, uint4 *__restrict__ big, uint32_t big_cap,
+    k_voxelize(const __grid_constant__ BatchDev bd, const __grid_constant__ MeshDev one, int64_t total,
+               uint32_t serial_max, uint32_t cols, uint4 *__restrict__ big, uint32_t big_cap,
                uint32_t *__restrict__ big_count) {
     chain_begin();
     const Meshes<ONE> mesh{bd, one};
@@ -815,7 +820,11 @@ __global__ void __launch_bounds__(256, INPLACE ? 2 : 3)
 // columns together (warp_columns).  A share at once keeps its lanes busy (30k
 // triangles on a 300 x 200 x 100 grid: 31 us, with a quarter of it 68); 16
 // columns per entry by default, since with 64 the last warps of a batch of 15
-// meshes work alone (140 us against 124 with 24 already).
+// meshes work alone (140 us against 124 with 24 already).  Its end is uneven (a
+// batch of 15 meshes: 11 of 16 warps per SM busy on average), but smaller
+// shares, the same from the start (6, 8, 16 entries) or falling towards the end
+// of the queue, cost as much in setups and half-full rounds: batch 1,709-1,787
+// us against 1,709-1,719, torus soup 1,882-1,942 against 1,872-1,882.
 template <bool S, bool ONE>
 __global__ void __launch_bounds__(256, 2) k_voxelize_columns(const __grid_constant__ BatchDev bd,
                                                              const __grid_constant__ MeshDev one,
