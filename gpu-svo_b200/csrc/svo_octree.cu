@@ -345,7 +345,8 @@ __global__ void __launch_bounds__(256, FUSE ? 4 : 8) k_pyramid(const __grid_cons
 }
 
 // The region sums' prefixes (CTAs 0..3 of a mesh, one level each) and levels
-// 5.. (CTA 4) of every mesh.
+// 5.. (CTA 4) of every mesh.  The mesh is the grid's x: y ends at 65,535, and a
+// batch may hold more meshes than that.
 template <bool ONE>
 __global__ void __launch_bounds__(1024) k_pyramid_finish(const __grid_constant__ BatchDev bd,
                                                          const __grid_constant__ MeshDev one) {
@@ -353,8 +354,8 @@ __global__ void __launch_bounds__(1024) k_pyramid_finish(const __grid_constant__
     __shared__ uint32_t s_warp[32];
     chain_begin();
     const Meshes<ONE> mesh{bd, one};
-    const MeshDev &md = mesh[blockIdx.y];
-    if (blockIdx.x < 4) scan_regions<1024, 16>(md, (int)blockIdx.x, s_warp);
+    const MeshDev &md = mesh[blockIdx.x];
+    if (blockIdx.y < 4) scan_regions<1024, 16>(md, (int)blockIdx.y, s_warp);
     else finish_top<1024>(md, s_top, s_warp);
 }
 
@@ -1259,10 +1260,10 @@ cudaError_t launch_pyramid(const BatchDev &b, uint32_t total_ctas, uint32_t max_
     const uint32_t blocks = std::min<uint32_t>(total_ctas, (uint32_t)num_sms * 8);
     if (b.one) {
         launch_chained(k_pyramid<false, true>, blocks, 256, 0, st, b, one, total_ctas);
-        launch_chained(k_pyramid_finish<true>, dim3(5, b.n), 1024, 0, st, b, one);
+        launch_chained(k_pyramid_finish<true>, dim3(b.n, 5), 1024, 0, st, b, one);
     } else {
         launch_chained(k_pyramid<false, false>, blocks, 256, 0, st, b, one, total_ctas);
-        launch_chained(k_pyramid_finish<false>, dim3(5, b.n), 1024, 0, st, b, one);
+        launch_chained(k_pyramid_finish<false>, dim3(b.n, 5), 1024, 0, st, b, one);
     }
     count_launches(2);
     return cudaGetLastError();
