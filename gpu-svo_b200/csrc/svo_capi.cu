@@ -264,20 +264,29 @@ T *batch_alloc(svo_batch *b, size_t count, cudaError_t &err) {
     return p;
 }
 
-// A pinned host block of at least `bytes` (kept blocks first); p is null when
-// there is none to be had.  Blocks of up to 1 MiB are kept for later batches,
-// at most 16 of them; the context frees them.
+// A pinned host block of at least `bytes` (the smallest kept one that holds
+// them first); p is null when there is none to be had.  Sizes are powers of two,
+// so that batches of about the same number of meshes take each other's blocks.
+// Kept for later batches: at most 16 blocks and kPinnedKept bytes (the reports
+// of 80,000 meshes), the largest ones; the context frees them.  A block that is
+// not kept costs its batch a cudaHostAlloc and a cudaFreeHost, and the latter
+// waits for all work on the device, other streams' too.
+constexpr size_t kPinnedKept = 16u << 20;
+
 svo_ctx::Pinned pinned_acquire(svo_ctx *ctx, size_t bytes) {
     {
         std::lock_guard<std::mutex> lk(ctx->pinned_mu);
-        for (size_t i = 0; i < ctx->pinned_free.size(); ++i)
-            if (ctx->pinned_free[i].bytes >= bytes) {
-                const svo_ctx::Pinned b = ctx->pinned_free[i];
-                ctx->pinned_free.erase(ctx->pinned_free.begin() + (long)i);
-                return b;
-            }
+        auto best = ctx->pinned_free.end();
+        for (auto it = ctx->pinned_free.begin(); it != ctx->pinned_free.end(); ++it)
+            if (it->bytes >= bytes && (best == ctx->pinned_free.end() || it->bytes < best->bytes)) best = it;
+        if (best != ctx->pinned_free.end()) {
+            const svo_ctx::Pinned b = *best;
+            ctx->pinned_free.erase(best);
+            return b;
+        }
     }
-    svo_ctx::Pinned b{nullptr, std::max<size_t>(bytes, 1 << 14)};
+    svo_ctx::Pinned b{nullptr, 1u << 14};
+    while (b.bytes < bytes) b.bytes *= 2;
     if (cudaHostAlloc(&b.p, b.bytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
         cudaGetLastError();
         b.p = nullptr;
@@ -287,14 +296,22 @@ svo_ctx::Pinned pinned_acquire(svo_ctx *ctx, size_t bytes) {
 
 void pinned_release(svo_ctx *ctx, svo_ctx::Pinned b) {
     if (!b.p) return;
+    std::vector<svo_ctx::Pinned> drop;
     {
         std::lock_guard<std::mutex> lk(ctx->pinned_mu);
-        if (b.bytes <= (1u << 20) && ctx->pinned_free.size() < 16) {
-            ctx->pinned_free.push_back(b);
-            return;
+        std::vector<svo_ctx::Pinned> &kept = ctx->pinned_free;
+        kept.push_back(b);
+        size_t total = 0;
+        for (const svo_ctx::Pinned &k : kept) total += k.bytes;
+        auto smaller = [](const svo_ctx::Pinned &x, const svo_ctx::Pinned &y) { return x.bytes < y.bytes; };
+        while (kept.size() > 16 || total > kPinnedKept) {
+            auto it = b.bytes > kPinnedKept ? kept.end() - 1 : std::min_element(kept.begin(), kept.end(), smaller);
+            total -= it->bytes;
+            drop.push_back(*it);
+            kept.erase(it);
         }
     }
-    cudaFreeHost(b.p);
+    for (svo_ctx::Pinned &d : drop) cudaFreeHost(d.p);
 }
 
 // The batch's stream must have finished (its kernels write to the report).
