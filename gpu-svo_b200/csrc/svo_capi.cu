@@ -14,6 +14,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -231,6 +232,27 @@ struct MetaLayout {
     }
 };
 
+// Host tables laid out in one buffer, filled in place and uploaded with one
+// copy: add() every table, then make(), then fill at().  No growing and no second
+// copy, since a table of thousands of meshes is megabytes, whose fresh pages cost
+// more than their contents: with vectors of jobs and emission parameters that were
+// appended to a growing buffer (13.8 KB of fresh pages a mesh, 4.0 this way) a
+// batch of 1,000 small meshes at res 8 took 2.8 ms instead of 0.97, one of 300
+// 1.12 instead of 0.31, one of 6,000 37 instead of 14.
+struct HostPack {
+    size_t bytes = 0;
+    std::unique_ptr<unsigned char[]> buf;
+    template <class T>
+    size_t add(size_t count) {
+        const size_t off = (bytes + 15) / 16 * 16;
+        if (count) bytes = off + count * sizeof(T);
+        return off;
+    }
+    void make() { buf.reset(bytes ? new unsigned char[bytes] : nullptr); }
+    template <class T>
+    T *at(size_t off) const { return reinterpret_cast<T *>(buf.get() + off); }
+};
+
 }  // namespace
 
 struct svo_batch {
@@ -249,7 +271,8 @@ struct svo_batch {
     svo_ctx::Pinned box{nullptr, 0};        // pinned host memory: a MeshOut per live mesh
     MeshOut *out = nullptr;
     MeshDev *d_mesh = nullptr;
-    std::vector<MeshDev> h_mesh;
+    HostPack tables;                        // the host copy of the mesh tables
+    MeshDev *h_mesh = nullptr;              // in tables, one per live mesh
     bool pending = false;                   // the stream may still hold work of this batch
     float timings_a[5] = {};                // total, bbox, voxelize, pyramid, scan
     bool timed = false;
@@ -340,20 +363,6 @@ struct Layout {
     }
 };
 
-// Small host tables packed into one buffer, uploaded with one copy.
-struct HostPack {
-    std::vector<unsigned char> buf;
-    template <class T>
-    size_t add(const T *src, size_t count) {
-        const size_t at = (buf.size() + 15) / 16 * 16;
-        buf.resize(at + count * sizeof(T));
-        if (count) std::memcpy(buf.data() + at, src, count * sizeof(T));
-        return at;
-    }
-    template <class T>
-    size_t add(const std::vector<T> &v) { return add(v.data(), v.size()); }
-};
-
 template <class T>
 cudaError_t upload(T *dst, const std::vector<T> &src, cudaStream_t st) {
     if (src.empty()) return cudaSuccess;
@@ -428,8 +437,13 @@ int batch_phase_a(svo_batch *b) {
     uint64_t words = 0, blocks = 0, bases = 0, tris = 0;
     uint32_t ctas = 0, max_ctas = 0, bblocks = 0;
     bool any_regions = false;
-    std::vector<uint64_t> tri_off(n + 1);
-    std::vector<uint32_t> cta_off(n + 1), bbox_off(n + 1);
+    HostPack &tables = b->tables;  // mesh table, triangle / CTA / bbox-block offsets
+    const size_t p_mesh = tables.add<MeshDev>(n), p_tri = tables.add<uint64_t>(n + 1),
+                 p_cta = tables.add<uint32_t>(n + 1), p_bbox = tables.add<uint32_t>(n + 1);
+    tables.make();
+    b->h_mesh = tables.at<MeshDev>(p_mesh);
+    uint64_t *tri_off = tables.at<uint64_t>(p_tri);
+    uint32_t *cta_off = tables.at<uint32_t>(p_cta), *bbox_off = tables.at<uint32_t>(p_bbox);
     for (int k = 0; k < n; ++k) {
         MeshHost &mh = b->m[b->live[k]];
         mh.py = make_pyramid(mh.res[0], mh.res[1], mh.res[2]);
@@ -454,16 +468,13 @@ int batch_phase_a(svo_batch *b) {
     bbox_off[n] = bblocks;
     // the batch's scratch arrays and its mesh tables: one block, one upload
     uint32_t big_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(2 * tris, 1 << 16), 0x7FFFFFFFu);
-    HostPack tables;  // mesh table, triangle / CTA / bbox-block offsets (filled below)
-    auto a16 = [](size_t x) { return (x + 15) / 16 * 16; };
-    const size_t t_bytes = a16(sizeof(MeshDev) * n) + a16(8 * (size_t)(n + 1)) + a16(4 * (size_t)(n + 1)) + 4 * (size_t)(n + 1);
     Layout lay;
     const size_t o_meta = lay.add<unsigned char>(ml.bytes);
     const size_t o_bits = lay.add<uint64_t>(words), o_pre = lay.add<uint32_t>(blocks), o_base = lay.add<uint32_t>(bases),
                  o_big = lay.add<uint4>(big_cap),
                  o_rflag = lay.add<uint8_t>(std::max<uint32_t>(ctas, 1)),
                  o_rlist = lay.add<uint32_t>(any_regions ? ctas : 0);
-    const size_t o_tables = lay.add<unsigned char>(t_bytes);
+    const size_t o_tables = lay.add<unsigned char>(tables.bytes);
     unsigned char *blk = batch_alloc<unsigned char>(b, lay.bytes, err);
     if (err != cudaSuccess || !blk) return cuda_fail(err, "batch scratch");
     b->bits = reinterpret_cast<uint64_t *>(blk + o_bits);
@@ -480,10 +491,9 @@ int batch_phase_a(svo_batch *b) {
     uint32_t *counters = reinterpret_cast<uint32_t *>(meta + ml.counters);
     b->rcount = counters + 2;
     b->dups = reinterpret_cast<unsigned long long *>(meta + ml.dups);
-    b->h_mesh.assign(n, MeshDev{});
     for (int k = 0; k < n; ++k) {
         const MeshHost &mh = b->m[b->live[k]];
-        MeshDev &d = b->h_mesh[k];
+        MeshDev &d = *new (b->h_mesh + k) MeshDev{};
         d.pts = mh.d_pts;
         d.tris = mh.d_tris;
         d.n_pts = mh.n_pts;
@@ -502,15 +512,13 @@ int batch_phase_a(svo_batch *b) {
         d.py = mh.py;
         d.regions = mh.py.words[0] >= kRegionWords ? 1 : 0;
     }
-    const size_t p_mesh = tables.add(b->h_mesh), p_tri = tables.add(tri_off), p_cta = tables.add(cta_off),
-                 p_bbox = tables.add(bbox_off);
     unsigned char *dt = blk + o_tables;
     b->d_mesh = reinterpret_cast<MeshDev *>(dt + p_mesh);
     const uint64_t *d_tri_off = reinterpret_cast<const uint64_t *>(dt + p_tri);
     const uint32_t *d_cta_off = reinterpret_cast<const uint32_t *>(dt + p_cta);
     const uint32_t *d_bbox_off = reinterpret_cast<const uint32_t *>(dt + p_bbox);
     if (n > 1)  // a lone mesh's table is passed to the kernels by value
-        SVO_TRY(cudaMemcpyAsync(dt, tables.buf.data(), tables.buf.size(), cudaMemcpyHostToDevice, st), "upload meshes");
+        SVO_TRY(cudaMemcpyAsync(dt, tables.buf.get(), tables.bytes, cudaMemcpyHostToDevice, st), "upload meshes");
     const BatchDev bd{b->d_mesh, n, d_tri_off, d_cta_off, d_bbox_off, rflag, any_regions ? b->rlist : nullptr, b->rcount,
                       n == 1 ? &b->h_mesh[0] : nullptr};
     const bool strict = (b->flags & SVO_FLAG_STRICT_FP) != 0;
@@ -765,13 +773,37 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 }
             }
             // outputs, code lists, job tables
-            std::vector<CompactJob> jobs;
-            std::vector<uint64_t> word_off(1, 0);
             std::vector<CompactJob> region_jobs;  // region-mode meshes' levels 1-2
             std::vector<std::pair<uint32_t, uint32_t>> region_range;  // first region, regions
-            std::vector<KeyJob> kjobs;
-            std::vector<uint64_t> blk_off(1, 0);
-            std::vector<EmitParams> ep(n);
+            auto regions = [](const MeshHost &mh) { return mh.py.words[0] >= kRegionWords; };
+            auto direct_keys = [&](const MeshHost &mh) {
+                return want_keys && (mh.T < 3 || mh.py.words[0] <= kDirectKeyWords);
+            };
+            auto own_emit = [&](const MeshHost &mh) { return n == 1 || mh.N >= kOwnEmitNodes; };
+            int n_jobs = 0, n_kjobs = 0, n_own = 0;
+            for (int j = 0; j < n; ++j) {
+                const MeshHost &mh = b->m[wave[j]];
+                n_jobs += regions(mh) ? (direct_keys(mh) ? 1 : 0) + (mh.T >= 3 ? 1 : 0) : 1;
+                n_kjobs += want_keys && !direct_keys(mh) ? 1 : 0;
+                n_own += own_emit(mh) ? 1 : 0;
+            }
+            const int n_small = n - n_own;
+            // the tables of the wave's kernels: compaction jobs, key jobs, emission
+            // parameters of the meshes that share one emission launch
+            HostPack wt;
+            const size_t p_jobs = wt.add<CompactJob>(n_jobs), p_woff = wt.add<uint64_t>(n_jobs + 1),
+                         p_kjobs = wt.add<KeyJob>(n_kjobs), p_boff = wt.add<uint64_t>(n_kjobs + 1),
+                         p_eps = wt.add<EmitParams>(n_small), p_offs = wt.add<uint64_t>(n_small + 1);
+            wt.make();
+            CompactJob *jobs = wt.at<CompactJob>(p_jobs);
+            uint64_t *word_off = wt.at<uint64_t>(p_woff);
+            KeyJob *kjobs = wt.at<KeyJob>(p_kjobs);
+            uint64_t *blk_off = wt.at<uint64_t>(p_boff);
+            EmitParams *ep_small = wt.at<EmitParams>(p_eps);
+            uint64_t *off_small = wt.at<uint64_t>(p_offs);
+            word_off[0] = blk_off[0] = off_small[0] = 0;
+            std::vector<EmitParams> ep_own(n_own);  // large meshes' launches of their own take them by value
+            std::vector<EmitParams *> ep(n);        // in one of the two
             uint64_t ktot = 0;
             std::vector<uint64_t> kbase(n);
             for (int j = 0; j < n; ++j) {
@@ -817,7 +849,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 }
                 arena = nullptr;
             };
-            for (int j = 0; j < n; ++j) {
+            for (int j = 0, at_job = 0, at_kjob = 0, at_own = 0, at_small = 0; j < n; ++j) {
                 const MeshHost &mh = b->m[wave[j]];
                 const MeshDev &md = b->h_mesh[dev_k[j]];
                 svo_result *r = new svo_result();
@@ -863,27 +895,29 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                     job.koff[l] = ko;
                     ko += mh.totals[l];
                 }
-                if (mh.py.words[0] >= kRegionWords) {
+                if (regions(mh)) {
                     // region mode: levels 1-2 region by region (k_compact_regions);
                     // level 3 words of unflagged regions are empty, not read
                     job.rflag = b->rflag + mh.cta0;
                     region_jobs.push_back(job);
                     region_range.push_back({mh.cta0, mh.py.ctas});
                 }
-                if (want_keys && (mh.T < 3 || mh.py.words[0] <= kDirectKeyWords)) {
+                if (direct_keys(mh)) {
                     job.l0 = 0;
                     job.keys = r->keys;
                 } else if (want_keys) {
                     // the level-3 code list is the list of non-empty level-0 blocks
-                    kjobs.push_back(KeyJob{md.bits, job.rank, job.out + job.koff[3], r->keys});
-                    blk_off.push_back(blk_off.back() + mh.totals[3]);
+                    new (kjobs + at_kjob) KeyJob{md.bits, job.rank, job.out + job.koff[3], r->keys};
+                    blk_off[at_kjob + 1] = blk_off[at_kjob] + mh.totals[3];
+                    ++at_kjob;
                 }
                 auto add_job = [&](int l0, int l1) {
                     if (l0 >= l1) return;
                     job.l0 = l0;
                     job.l1 = l1;
-                    jobs.push_back(job);
-                    word_off.push_back(word_off.back() + mh.py.woff[l1 - 1] + mh.py.words[l1 - 1] - mh.py.woff[l0]);
+                    new (jobs + at_job) CompactJob(job);
+                    word_off[at_job + 1] = word_off[at_job] + mh.py.woff[l1 - 1] + mh.py.words[l1 - 1] - mh.py.woff[l0];
+                    ++at_job;
                 };
                 if (job.rflag) {  // levels 1-2 have a launch of their own (region_jobs)
                     if (job.l0 == 0) add_job(0, 1);
@@ -892,7 +926,13 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                     add_job(job.l0, mh.T + 1);
                 }
                 // emission parameters
-                EmitParams &P = ep[j];
+                const bool own = own_emit(mh);
+                ep[j] = own ? &ep_own[at_own++] : new (ep_small + at_small) EmitParams{};
+                if (!own) {
+                    off_small[at_small + 1] = off_small[at_small] + (mh.N + 31) / 32 * 32;
+                    ++at_small;
+                }
+                EmitParams &P = *ep[j];
                 P.T = mh.T;
                 P.N = (uint32_t)mh.N;
                 P.flags = flags;
@@ -920,28 +960,10 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 drop_arena();
                 return cuda_fail(err, "output allocation");
             }
-            // Large meshes' emission launches of their own (parameters in the kernel's
-            // constant space); the rest share one launch over the mesh table.
-            std::vector<EmitParams> ep_small;
-            std::vector<uint64_t> off_small(1, 0);
-            int n_own = 0;
-            for (int j = 0; j < n; ++j) {
-                if (n == 1 || ep[j].N >= kOwnEmitNodes) {
-                    ++n_own;
-                } else {
-                    ep_small.push_back(ep[j]);
-                    off_small.push_back(off_small.back() + (ep[j].N + 31) / 32 * 32);
-                }
-            }
-            // the wave's tables: one block, one upload; what one kernel takes by
-            // value (a lone mesh's compaction job and emission) needs none
-            const bool lone_job = jobs.size() == 1, lone_keys = kjobs.size() == 1;
-            HostPack wt;
-            const size_t p_jobs = lone_job ? 0 : wt.add(jobs), p_woff = lone_job ? 0 : wt.add(word_off),
-                         p_kjobs = lone_keys ? 0 : wt.add(kjobs),
-                         p_boff = kjobs.empty() || lone_keys ? 0 : wt.add(blk_off),
-                         p_eps = wt.add(ep_small), p_offs = ep_small.empty() ? 0 : wt.add(off_small);
-            unsigned char *dwt = wt.buf.empty() ? nullptr : S.get<unsigned char>(wt.buf.size());
+            // one upload of the tables; what one kernel takes by value (a lone mesh's
+            // jobs and emission) needs none
+            const bool lone_job = n_jobs == 1, lone_keys = n_kjobs == 1;
+            unsigned char *dwt = n_jobs > 1 || n_kjobs > 1 || n_small > 0 ? S.get<unsigned char>(wt.bytes) : nullptr;
             if (S.err != cudaSuccess) {
                 free_results();
                 drop_arena();
@@ -951,24 +973,23 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
             const uint64_t *d_word_off = reinterpret_cast<const uint64_t *>(dwt + p_woff);
             const KeyJob *d_kjobs = reinterpret_cast<const KeyJob *>(dwt + p_kjobs);
             const uint64_t *d_blk_off = reinterpret_cast<const uint64_t *>(dwt + p_boff);
-            if (dwt) check(cudaMemcpyAsync(dwt, wt.buf.data(), wt.buf.size(), cudaMemcpyHostToDevice, st), "upload");
+            if (dwt) check(cudaMemcpyAsync(dwt, wt.buf.get(), wt.bytes, cudaMemcpyHostToDevice, st), "upload");
             tm.mark(StageTimer::kCompact0, st);
-            check(launch_compact(CompactBatch{d_jobs, (int)jobs.size(), d_word_off}, lone_job ? &jobs[0] : nullptr,
-                                 word_off.back(), st),
+            check(launch_compact(CompactBatch{d_jobs, n_jobs, d_word_off}, lone_job ? jobs : nullptr, word_off[n_jobs], st),
                   "compact");
             // The keys need the level-3 lists and nothing needs the keys: they run on
             // a stream of their own beside the remaining lists and the emission (320
             // triangles at res 512 420 us before, 414 this way; heightfield at res
             // 2048, with the later dedup start above, 4,076 and 4,046).
-            AuxStreams *kset = kjobs.empty() ? nullptr : aux_acquire(ctx);
+            AuxStreams *kset = n_kjobs == 0 ? nullptr : aux_acquire(ctx);
             const cudaStream_t ks = kset ? kset->s[0] : st;
             if (kset) {
                 check(cudaEventRecord(kset->fork, st), "fork");
                 check(cudaStreamWaitEvent(ks, kset->fork, 0), "fork");
             }
-            if (!kjobs.empty())
-                check(launch_compact_keys(KeyBatch{d_kjobs, (int)kjobs.size(), d_blk_off}, lone_keys ? &kjobs[0] : nullptr,
-                                          blk_off.back(), ks),
+            if (n_kjobs > 0)
+                check(launch_compact_keys(KeyBatch{d_kjobs, n_kjobs, d_blk_off}, lone_keys ? kjobs : nullptr, blk_off[n_kjobs],
+                                          ks),
                       "keys");
             for (size_t i = 0; i < region_jobs.size(); ++i)
                 check(launch_compact_regions(region_jobs[i], b->rlist, b->rcount, region_range[i].first,
@@ -991,11 +1012,11 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
             }
             int k_own = 0;
             for (int j = 0; j < n; ++j) {
-                if (n == 1 || ep[j].N >= kOwnEmitNodes) {
+                if (own_emit(b->m[wave[j]])) {
                     const int lane = aux ? k_own % (AuxStreams::kCount + 1) : 0;
                     cudaStream_t es = lane == 0 ? st : aux->s[lane - 1];
                     ++k_own;
-                    check(launch_emit(EmitBatch{nullptr, 1, nullptr}, &ep[j], ep[j].N, flags, ctx->num_sms, es), "emit");
+                    check(launch_emit(EmitBatch{nullptr, 1, nullptr}, ep[j], ep[j]->N, flags, ctx->num_sms, es), "emit");
                 }
             }
             if (aux) {
@@ -1005,10 +1026,10 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 }
                 aux_release(ctx, aux);
             }
-            if (!ep_small.empty())
-                check(launch_emit(EmitBatch{reinterpret_cast<const EmitParams *>(dwt + p_eps), (int)ep_small.size(),
+            if (n_small > 0)
+                check(launch_emit(EmitBatch{reinterpret_cast<const EmitParams *>(dwt + p_eps), n_small,
                                             reinterpret_cast<const uint64_t *>(dwt + p_offs)},
-                                  nullptr, off_small.back(), flags, ctx->num_sms, st),
+                                  nullptr, off_small[n_small], flags, ctx->num_sms, st),
                       "emit");
             tm.mark(StageTimer::kEmit, st);
             // Dedup of every mesh on the forked stream (its host-side waits
@@ -1019,7 +1040,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                     if (b->m[wave[j]].status != SVO_OK) continue;
                     if (!dstarted[j]) dedup_start(j);
                     if (!druns[j]) continue;
-                    drc[j] = dedup_finish(druns[j], ctx->out_pool, ep[j], res[j]->n_dedup, res[j]->dedup);
+                    drc[j] = dedup_finish(druns[j], ctx->out_pool, *ep[j], res[j]->n_dedup, res[j]->dedup);
                     druns[j] = nullptr;
                     if (drc[j] != SVO_OK) dmsg[j] = svo_last_error();
                 }

@@ -1,9 +1,12 @@
 """Batches of very many small meshes (an asset import): every mesh gets the
 octree of its own build, whatever their number."""
-import numpy as np
+import os
+import subprocess
+import sys
+
 import pytest
 
-from conftest import random_mesh
+from conftest import ROOT, random_mesh
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +55,35 @@ def test_many_meshes_do_not_wait_for_other_streams(gpu_ctx, svo_mod):
     running = not done.query()
     torch.cuda.synchronize()
     assert rc == 0 and running
+
+
+FRESH_PAGES = """
+import sys, resource
+sys.path[:0] = [sys.argv[1] + "/gpu-svo_b200", sys.argv[1] + "/tests"]
+import ctypes as C
+import torch, svo_b200
+from conftest import random_mesh
+v, f = random_mesh(41, 2)
+mesh = (torch.from_numpy(v).cuda(), torch.from_numpy(f).cuda(), 4)
+ctx, n = svo_b200.Context(0), 4000
+descs, keep = svo_b200._descs([mesh] * n, svo_b200.FLAG_NO_VERT_EDGE)
+outs, st = (C.c_void_p * n)(), (C.c_int * n)()
+for _ in range(4):
+    before = resource.getrusage(resource.RUSAGE_SELF).ru_minflt
+    assert svo_b200.lib().svo_build_batch(ctx.handle, descs, n, None, outs, st) == 0
+    faults = resource.getrusage(resource.RUSAGE_SELF).ru_minflt - before
+    for o in outs:
+        svo_b200.lib().svo_result_free(o)
+print(faults * resource.getpagesize() / n)
+"""
+
+
+def test_tables_of_many_meshes_are_made_once(svo_mod):
+    """Fresh host memory of a batch, by the pages it faults in (every block of
+    128 KiB and more its own mapping).  The per-mesh records (two of the mesh,
+    its compaction job and its emission parameters, 24 levels each) are 4.0 KB
+    together; made once they stay below one and a half times that."""
+    env = dict(os.environ, MALLOC_MMAP_THRESHOLD_="131072")
+    p = subprocess.run([sys.executable, "-c", FRESH_PAGES, ROOT], env=env, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]
+    assert float(p.stdout) < 6000
