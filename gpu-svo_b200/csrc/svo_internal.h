@@ -113,6 +113,11 @@ struct BatchDev {
 // follows another on the same stream: two plain launches are about 2 us apart.
 // With 320 triangles at 32^3 a build took 92.8 us and takes 83.6 this way, with
 // 20k at 128^3 120.8 and 108.9, with 5M at 2048^3 4,037 and 4,020.
+//
+// Such a kernel may be resident while the kernels before it still write.  So it
+// reads nothing of theirs as data that is constant over the whole kernel (const
+// T *__restrict__, __ldg): the compiler could then use read-only loads, and move
+// them before the wait.  Mesh inputs are constant.
 __device__ __forceinline__ void chain_begin() {
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();

@@ -666,9 +666,8 @@ __global__ void __launch_bounds__(256) k_compact(CompactBatch cb, const __grid_c
 // region lie inside it, and the unflagged ones (most of them at res 2048) hold
 // none.  The list is the batch's: the mesh's own regions are cta0 on.
 __global__ void __launch_bounds__(256) k_compact_regions(const __grid_constant__ CompactJob job,
-                                                         const uint32_t *__restrict__ rlist,
-                                                         const uint32_t *__restrict__ rcount, uint32_t cta0,
-                                                         uint32_t regions) {
+                                                         const uint32_t *rlist, const uint32_t *rcount,
+                                                         uint32_t cta0, uint32_t regions) {
     chain_begin();
     const uint32_t count = *rcount;
     for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
@@ -817,8 +816,8 @@ __device__ __forceinline__ void full_neighbors(const EmitParams &P, const NodeIn
             ok |= ((m[a] != 0 ? 1u : 0u) | 2u | (up[a] < lim[a] && up[a] != 0 ? 4u : 0u)) << (3 * a);
         }
         const bool top = l1 >= P.T;  // the root level: rank 0
-        const uint64_t *__restrict__ bits = P.lv[l1].bits;
-        const uint32_t *__restrict__ wpre = P.lv[l1].wpre;
+        const uint64_t *bits = P.lv[l1].bits;
+        const uint32_t *wpre = P.lv[l1].wpre;
         uint64_t wd[4];
         uint32_t wp[4], sh[4];
 #pragma unroll

@@ -828,9 +828,8 @@ __global__ void __launch_bounds__(256, INPLACE ? 2 : 3)
 template <bool S, bool ONE>
 __global__ void __launch_bounds__(256, 2) k_voxelize_columns(const __grid_constant__ BatchDev bd,
                                                              const __grid_constant__ MeshDev one,
-                                                             const uint4 *__restrict__ big,
-                                                             const uint32_t *__restrict__ big_count, uint32_t big_cap,
-                                                             uint32_t *__restrict__ cursor) {
+                                                             const uint4 *big, const uint32_t *big_count,
+                                                             uint32_t big_cap, uint32_t *cursor) {
     chain_begin();
     const Meshes<ONE> mesh{bd, one};
     __shared__ Tri s_tri[8][32];
