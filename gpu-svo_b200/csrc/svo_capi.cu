@@ -160,7 +160,7 @@ T *pool_alloc(cudaMemPool_t pool, cudaStream_t st, size_t count, cudaError_t &er
 
 // CUDA events at stage boundaries (SVO_FLAG_TIMINGS).
 struct StageTimer {
-    enum { kStart, kBbox, kVox, kPyr, kScan, kCompact0, kCompact, kEmit, kUnique, kDedup0, kDedup, kEnd, kN };
+    enum { kStart, kBbox, kVox, kPyr, kCompact0, kCompact, kEmit, kUnique, kDedup0, kDedup, kEnd, kN };
     bool on = false;
     cudaEvent_t ev[kN] = {};
     bool rec[kN] = {};
@@ -274,7 +274,7 @@ struct svo_batch {
     HostPack tables;                        // the host copy of the mesh tables
     MeshDev *h_mesh = nullptr;              // in tables, one per live mesh
     bool pending = false;                   // the stream may still hold work of this batch
-    float timings_a[5] = {};                // total, bbox, voxelize, pyramid, scan
+    float timings_a[4] = {};                // total, bbox, voxelize, pyramid
     bool timed = false;
 };
 
@@ -534,7 +534,6 @@ int batch_phase_a(svo_batch *b) {
         tm.mark(StageTimer::kVox, st);
         SVO_TRY(launch_pyramid(bd, ctas, max_ctas, ctx->num_sms, st), "pyramid");
         tm.mark(StageTimer::kPyr, st);
-        tm.mark(StageTimer::kScan, st);
         SVO_TRY(cudaStreamSynchronize(st), "count phase");
         b->pending = false;
         if (b->out[0].queue > big_cap) {  // more big-triangle entries than the queue holds: grow it, redo
@@ -554,11 +553,10 @@ int batch_phase_a(svo_batch *b) {
     }
     if (tm.on) {
         b->timed = true;
-        b->timings_a[0] = tm.span(StageTimer::kStart, StageTimer::kScan);
+        b->timings_a[0] = tm.span(StageTimer::kStart, StageTimer::kPyr);
         b->timings_a[1] = tm.span(StageTimer::kStart, StageTimer::kBbox);
         b->timings_a[2] = tm.span(StageTimer::kBbox, StageTimer::kVox);
         b->timings_a[3] = tm.span(StageTimer::kVox, StageTimer::kPyr);
-        b->timings_a[4] = tm.span(StageTimer::kPyr, StageTimer::kScan);
     }
     // ---- level structure per mesh (src/SVO.cu:383-495) ----
     for (int k = 0; k < n; ++k) {
@@ -1138,7 +1136,6 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 r->timings[1] = b->timings_a[1];
                 r->timings[2] = b->timings_a[2];
                 r->timings[3] = b->timings_a[3];
-                r->timings[4] = b->timings_a[4];
                 r->timings[5] = tm.span(StageTimer::kCompact0, StageTimer::kCompact);
                 r->timings[6] = tm.span(StageTimer::kCompact, StageTimer::kEmit);
                 r->timings[7] = tm.span(StageTimer::kEmit, StageTimer::kUnique);
