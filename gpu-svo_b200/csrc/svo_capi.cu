@@ -160,7 +160,7 @@ T *pool_alloc(cudaMemPool_t pool, cudaStream_t st, size_t count, cudaError_t &er
 
 // CUDA events at stage boundaries (SVO_FLAG_TIMINGS).
 struct StageTimer {
-    enum { kStart, kBbox, kVox, kPyr, kCompact0, kCompact, kEmit, kUnique, kDedup0, kDedup, kEnd, kN };
+    enum { kStart, kBbox, kVox, kPyr, kCompact0, kCompact, kKeys, kEmit, kUnique, kDedup0, kDedup, kEnd, kN };
     bool on = false;
     cudaEvent_t ev[kN] = {};
     bool rec[kN] = {};
@@ -989,6 +989,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 check(launch_compact_keys(KeyBatch{d_kjobs, n_kjobs, d_blk_off}, lone_keys ? kjobs : nullptr, blk_off[n_kjobs],
                                           ks),
                       "keys");
+            if (n_kjobs > 0) tm.mark(StageTimer::kKeys, ks);
             for (size_t i = 0; i < region_jobs.size(); ++i)
                 check(launch_compact_regions(region_jobs[i], b->rlist, b->rcount, region_range[i].first,
                                              region_range[i].second, ctx->num_sms, st),
@@ -1136,7 +1137,8 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 r->timings[1] = b->timings_a[1];
                 r->timings[2] = b->timings_a[2];
                 r->timings[3] = b->timings_a[3];
-                r->timings[5] = tm.span(StageTimer::kCompact0, StageTimer::kCompact);
+                r->timings[5] = std::max(tm.span(StageTimer::kCompact0, StageTimer::kCompact),
+                                         tm.span(StageTimer::kCompact0, StageTimer::kKeys));
                 r->timings[6] = tm.span(StageTimer::kCompact, StageTimer::kEmit);
                 r->timings[7] = tm.span(StageTimer::kEmit, StageTimer::kUnique);
                 r->timings[8] = tm.span(StageTimer::kDedup0, StageTimer::kDedup);

@@ -340,7 +340,8 @@ int svo_result_copy_keys(const svo_result *r, uint64_t *dst, int64_t cap);
  * host round trip that sizes the outputs), [1] bounding cube and clearing of
  * the bitmaps, [2] voxelize,
  * [3] bitmap pyramid with its block ranks, [4] 0 (a rank scan of its own in
- * earlier versions), [5] level code lists,
+ * earlier versions), [5] level code lists and surface-voxel keys (the keys of
+ * grids above 256 on a stream of their own, concurrent with [6]),
  * [6] node/vertex/edge emission, [7] duplicate removal, [8] dedup keys (on a
  * stream of its own, concurrent with [6] and [7], so the stages need not add
  * up to [0]).  Returns the number of entries (9), or 0 without timings.  No

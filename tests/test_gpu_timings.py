@@ -5,6 +5,11 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+def _best(ctx, mesh, res, flags, stage, n=5):
+    """The stage's least time over some builds, in ms (device times plus the odd host hiccup)."""
+    return min(ctx.build(*mesh, res, flags).timings()[stage] for _ in range(n + 2))
+
+
 def _mesh(n, size, seed=9):
     import torch
 
@@ -19,3 +24,16 @@ def test_no_scan_stage(gpu_ctx, svo_mod):
     assert t["scan"] == 0.0
     assert all(t[k] > 0.0 for k in ("total", "bbox", "voxelize", "pyramid", "compact", "emit"))
     assert t["total"] >= t["bbox"] + t["voxelize"] + t["pyramid"]
+
+
+def test_compact_stage_has_the_keys(gpu_ctx, svo_mod):
+    """Above res 256 the keys have a launch and a stream of their own.  Writing
+    them takes at least their bytes over the path from the SMs to L2 (32 bytes a
+    clock and SM, 148 SMs, 1.965 GHz)."""
+    mesh = _mesh(300, 0.4)
+    flags = svo_mod.FLAG_TIMINGS | svo_mod.FLAG_NO_VERT_EDGE
+    n_keys = gpu_ctx.build(*mesh, 512, flags).num_keys
+    assert n_keys > 8_000_000
+    with_keys = _best(gpu_ctx, mesh, 512, flags, "compact")
+    without = _best(gpu_ctx, mesh, 512, flags | svo_mod.FLAG_NO_KEYS, "compact")
+    assert with_keys - without > n_keys * 8 / (148 * 32 * 1.965e9) * 1e3
