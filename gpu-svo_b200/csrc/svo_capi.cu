@@ -160,7 +160,7 @@ T *pool_alloc(cudaMemPool_t pool, cudaStream_t st, size_t count, cudaError_t &er
 
 // CUDA events at stage boundaries (SVO_FLAG_TIMINGS).
 struct StageTimer {
-    enum { kStart, kBbox, kVox, kPyr, kCompact0, kCompact, kKeys, kEmit, kUnique, kDedup0, kDedup, kEnd, kN };
+    enum { kStart, kBbox, kVox, kPyr, kCompact0, kCompact, kKeys, kEmit, kUnique0, kUnique, kDedup0, kDedup, kEnd, kN };
     bool on = false;
     cudaEvent_t ev[kN] = {};
     bool rec[kN] = {};
@@ -1052,6 +1052,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 aux_release(ctx, kset);
             }
             check(cudaStreamSynchronize(st), "emit phase");
+            tm.mark(StageTimer::kUnique0, st);  // (the wait above is for the dedup and the keys as well)
             bool more = false;  // work launched after this wait
             for (int j = 0; j < n && rc == SVO_OK; ++j) {
                 MeshHost &mh = b->m[wave[j]];
@@ -1140,7 +1141,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 r->timings[5] = std::max(tm.span(StageTimer::kCompact0, StageTimer::kCompact),
                                          tm.span(StageTimer::kCompact0, StageTimer::kKeys));
                 r->timings[6] = tm.span(StageTimer::kCompact, StageTimer::kEmit);
-                r->timings[7] = tm.span(StageTimer::kEmit, StageTimer::kUnique);
+                r->timings[7] = tm.span(StageTimer::kUnique0, StageTimer::kUnique);
                 r->timings[8] = tm.span(StageTimer::kDedup0, StageTimer::kDedup);
                 r->timings[0] = b->timings_a[0] + tm.span(StageTimer::kCompact0, StageTimer::kEnd);
             }

@@ -343,8 +343,8 @@ int svo_result_copy_keys(const svo_result *r, uint64_t *dst, int64_t cap);
  * earlier versions), [5] level code lists and surface-voxel keys (the keys of
  * grids above 256 on a stream of their own, concurrent with [6]),
  * [6] node/vertex/edge emission, [7] duplicate removal, [8] dedup keys (on a
- * stream of its own, concurrent with [6] and [7], so the stages need not add
- * up to [0]).  Returns the number of entries (9), or 0 without timings.  No
+ * stream of its own, concurrent with [6], so the stages need not add up to
+ * [0]).  Returns the number of entries (9), or 0 without timings.  No
  * counterpart in the reference (it has no instrumentation). */
 int svo_result_timings(const svo_result *r, float *ms, int cap);
 

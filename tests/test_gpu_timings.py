@@ -37,3 +37,11 @@ def test_compact_stage_has_the_keys(gpu_ctx, svo_mod):
     with_keys = _best(gpu_ctx, mesh, 512, flags, "compact")
     without = _best(gpu_ctx, mesh, 512, flags | svo_mod.FLAG_NO_KEYS, "compact")
     assert with_keys - without > n_keys * 8 / (148 * 32 * 1.965e9) * 1e3
+
+
+def test_unique_stage_is_not_the_wait_for_the_dedup(gpu_ctx, svo_mod):
+    """No duplicates: nothing to remove, however long the dedup's stream runs on."""
+    mesh = _mesh(20000, 0.01)
+    flags = svo_mod.FLAG_TIMINGS | svo_mod.FLAG_NO_VERT_EDGE | svo_mod.FLAG_DEDUP
+    t = [gpu_ctx.build(*mesh, 256, flags).timings() for _ in range(7)]
+    assert min(x["unique"] for x in t) < 0.25 * min(x["dedup"] for x in t)
