@@ -14,6 +14,7 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -39,9 +40,10 @@ struct CopyPool {
 
     bool init() {
         if (tried) return !w.empty();
-        tried = true;
         const unsigned cores = std::thread::hardware_concurrency();
         const int n = std::max(1, std::min<int>(kWorkers, (int)cores / 2));
+        w.reserve((size_t)n);  // (the only step here that throws: nothing is held yet)
+        tried = true;
         bool ok = cudaEventCreateWithFlags(&start, cudaEventDisableTiming) == cudaSuccess;
         for (int i = 0; i < n && ok; ++i) {
             Worker k;
@@ -85,7 +87,16 @@ std::shared_ptr<CopyPool> copy_pool_create(int device) {
 bool copy_to_pageable(CopyPool &pool, void *dst, const void *src, size_t bytes, cudaStream_t st, cudaError_t *err) {
     if (bytes < 4 * kChunk) return false;
     std::unique_lock<std::mutex> lk(pool.mu, std::try_to_lock);
-    if (!lk.owns_lock() || !pool.init()) return false;
+    if (!lk.owns_lock()) return false;
+    std::vector<std::thread> threads;
+    std::vector<size_t> here;  // the shares copied by this thread
+    try {
+        if (!pool.init()) return false;
+        threads.reserve(pool.w.size());  // nothing below allocates beside a thread's start
+        here.reserve(pool.w.size());
+    } catch (const std::bad_alloc &) {
+        return false;
+    }
     if ((*err = cudaEventRecord(pool.start, st)) != cudaSuccess) return true;
     // Spans end at multiples of kSpan in the destination's addresses, so that no
     // two threads fault the same huge page in.
@@ -125,8 +136,7 @@ bool copy_to_pageable(CopyPool &pool, void *dst, const void *src, size_t bytes, 
             first_error.compare_exchange_strong(none, (int)e);
         }
     };
-    std::vector<std::thread> threads;
-    std::vector<size_t> here(1, 0);
+    here.push_back(0);
     for (size_t i = 1; i < nw; ++i) {
         try {
             threads.emplace_back(work, i);
