@@ -98,6 +98,11 @@ bool copy_to_pageable(CopyPool &pool, void *dst, const void *src, size_t bytes, 
         return false;
     }
     if ((*err = cudaEventRecord(pool.start, st)) != cudaSuccess) return true;
+    // The caller's capture mode holds for the threads that copy for it.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if ((*err = cudaThreadExchangeStreamCaptureMode(&mode)) != cudaSuccess) return true;
+    cudaStreamCaptureMode relaxed = mode;
+    cudaThreadExchangeStreamCaptureMode(&relaxed);
     // Spans end at multiples of kSpan in the destination's addresses, so that no
     // two threads fault the same huge page in.
     const size_t skew = (size_t)(reinterpret_cast<uintptr_t>(dst) % kSpan);
@@ -106,7 +111,9 @@ bool copy_to_pageable(CopyPool &pool, void *dst, const void *src, size_t bytes, 
     std::atomic<int> first_error{cudaSuccess};
     auto work = [&](size_t i) {
         CopyPool::Worker &k = pool.w[i];
-        cudaError_t e = cudaSetDevice(pool.device);
+        cudaStreamCaptureMode own = mode;
+        cudaError_t e = cudaThreadExchangeStreamCaptureMode(&own);
+        if (e == cudaSuccess) e = cudaSetDevice(pool.device);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(k.stream, pool.start, 0);
         size_t at[2] = {0, 0}, len[2] = {0, 0};  // what the slots hold (len 0: nothing)
         auto drain = [&](int j) {
