@@ -33,11 +33,28 @@ struct AuxStreams {
     cudaEvent_t join[kCount] = {};
 };
 
+// The pool of the result arrays.  A context and its results share it and the last
+// of them destroys it, after every free has completed: later copies of the
+// process crashed in the driver once a pool had been destroyed with allocations
+// outstanding.
+struct OutPool {
+    int device;
+    cudaMemPool_t pool;
+    std::atomic<bool> outlived{false};  // results were left when the context went
+    OutPool(int d, cudaMemPool_t p) : device(d), pool(p) {}
+    ~OutPool() {
+        cudaSetDevice(device);
+        if (outlived) cudaDeviceSynchronize();  // the frees may be on several streams
+        cudaMemPoolDestroy(pool);
+    }
+};
+
 struct svo_ctx {
     int device = 0;
     int num_sms = 148;
     cudaMemPool_t pool = nullptr;      // per-build scratch
     cudaMemPool_t out_pool = nullptr;  // result arrays, kept apart so scratch never splits their blocks
+    std::shared_ptr<OutPool> out_keep;  // holds out_pool
     VoxTuning tune;                    // read and written under tune_mu
     std::mutex tune_mu;
     std::mutex aux_mu;                 // builds on other threads take sets of their own
@@ -62,7 +79,7 @@ struct svo_arena {
 struct svo_result {
     int device = 0;
     cudaStream_t stream = nullptr;
-    cudaMemPool_t pool = nullptr;
+    std::shared_ptr<OutPool> out_keep;  // the pool of its arrays
     int depth = 0;
     std::vector<int64_t> level_counts;
     svo_aabb bbox{};
@@ -854,7 +871,7 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 res[j] = r;
                 r->device = ctx->device;
                 r->stream = st;
-                r->pool = ctx->pool;
+                r->out_keep = ctx->out_keep;
                 r->copies = ctx->copies;
                 r->depth = mh.T + 1;
                 for (int l = 0; l <= mh.T; ++l) r->level_counts.push_back((int64_t)mh.n_l[l]);
@@ -1242,6 +1259,7 @@ int svo_ctx_create(int device, svo_ctx **out) {
             return fail(SVO_ERR_CUDA, "memory pool");
         }
     }
+    c->out_keep = std::make_shared<OutPool>(device, c->out_pool);
     *out = c;
     return SVO_OK;
 }
@@ -1270,8 +1288,7 @@ int svo_ctx_device(const svo_ctx *ctx, int *device) {
     return SVO_OK;
 }
 
-// Results may outlive the context: a pool destroyed with allocations
-// outstanding is released once they are freed.
+// Results may outlive the context: they hold the pool of their arrays (OutPool).
 void svo_ctx_destroy(svo_ctx *ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
@@ -1285,7 +1302,11 @@ void svo_ctx_destroy(svo_ctx *ctx) {
     }
     for (svo_ctx::Pinned &b : ctx->pinned_free) cudaFreeHost(b.p);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
-    if (ctx->out_pool) cudaMemPoolDestroy(ctx->out_pool);
+    if (ctx->out_keep) {
+        if (ctx->out_keep.use_count() > 1) ctx->out_keep->outlived = true;
+    } else if (ctx->out_pool) {
+        cudaMemPoolDestroy(ctx->out_pool);
+    }
     delete ctx;
 }
 
