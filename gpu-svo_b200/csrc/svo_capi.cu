@@ -380,12 +380,6 @@ struct Layout {
     }
 };
 
-template <class T>
-cudaError_t upload(T *dst, const std::vector<T> &src, cudaStream_t st) {
-    if (src.empty()) return cudaSuccess;
-    return cudaMemcpyAsync(dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice, st);
-}
-
 // Phase A.  Returns SVO_OK when the batch itself works (individual meshes
 // may still carry an error status).
 int batch_phase_a(svo_batch *b) {

@@ -116,7 +116,6 @@ struct GridParams {
 // Status word bits reported back to the host.
 enum : uint32_t {
     kStatusNonFinite = 1u,
-    kStatusBigOverflow = 2u,
     kStatusScanTimeout = 4u,
     kStatusBadIndex = 8u,  // a triangle names a vertex outside the mesh (that triangle is skipped)
 };

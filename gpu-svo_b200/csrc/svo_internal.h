@@ -255,16 +255,6 @@ cudaError_t launch_front(const BatchDev &b, uint32_t bbox_blocks, uint32_t total
                          bool any_regions, int num_sms, cudaStream_t st);
 // mm[0] = min, mm[1] = max of n int32 indices.
 cudaError_t launch_index_range(const int32_t *idx, int64_t n, int32_t *mm, cudaStream_t st);
-// The same for a table of n index arrays in one launch: job k gets
-// index_blocks(jobs[k].n) blocks, block_off their prefix (n + 1 entries);
-// mm[2k], mm[2k+1] = min, max of job k.
-struct IndexJob {
-    const int32_t *idx;
-    int64_t n;
-};
-uint32_t index_blocks(int64_t n);
-cudaError_t launch_index_ranges(const IndexJob *jobs, int n, const uint32_t *block_off, uint32_t total_blocks,
-                                int32_t *mm, cudaStream_t st);
 // counters: 2 zeroed u32 (queue entries, queue cursor); big: the queue of
 // large triangles, or null: every large triangle is walked by the warp that
 // set it up.

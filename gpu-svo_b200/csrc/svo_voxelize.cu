@@ -889,35 +889,6 @@ __global__ void k_index_range(const int32_t *__restrict__ idx, int64_t n, int32_
     }
 }
 
-// Min/max index of each job of a table (jobs whose blocks follow block_off).
-__global__ void k_index_ranges_init(int32_t *mm, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        mm[2 * i] = 0x7FFFFFFF;
-        mm[2 * i + 1] = (int32_t)0x80000000;
-    }
-}
-
-__global__ void k_index_ranges(const IndexJob *__restrict__ jobs, int n, const uint32_t *__restrict__ block_off,
-                               int32_t *__restrict__ mm) {
-    const int k = find_segment(block_off, n, (uint32_t)blockIdx.x);
-    const IndexJob jb = jobs[k];
-    const int64_t nb = block_off[k + 1] - block_off[k];
-    int32_t lo = 0x7FFFFFFF, hi = (int32_t)0x80000000;
-    for (int64_t i = (blockIdx.x - block_off[k]) * (int64_t)blockDim.x + threadIdx.x; i < jb.n;
-         i += nb * blockDim.x) {
-        const int32_t v = __ldg(jb.idx + i);
-        lo = min(lo, v);
-        hi = max(hi, v);
-    }
-    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
-    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(mm + 2 * k, lo);
-        atomicMax(mm + 2 * k + 1, hi);
-    }
-}
-
 }  // namespace
 
 cudaError_t launch_index_range(const int32_t *idx, int64_t n, int32_t *mm, cudaStream_t st) {
@@ -926,17 +897,6 @@ cudaError_t launch_index_range(const int32_t *idx, int64_t n, int32_t *mm, cudaS
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 8));
     k_index_range<<<blocks, 256, 0, st>>>(idx, n, mm);
     count_launches(1);
-    return cudaGetLastError();
-}
-
-uint32_t index_blocks(int64_t n) { return (uint32_t)std::max<int64_t>(1, std::min<int64_t>((n + 2047) / 2048, 2048)); }
-
-cudaError_t launch_index_ranges(const IndexJob *jobs, int n, const uint32_t *block_off, uint32_t total_blocks,
-                                int32_t *mm, cudaStream_t st) {
-    if (n == 0) return cudaSuccess;
-    k_index_ranges_init<<<(n + 127) / 128, 128, 0, st>>>(mm, n);
-    k_index_ranges<<<total_blocks, 256, 0, st>>>(jobs, n, block_off, mm);
-    count_launches(2);
     return cudaGetLastError();
 }
 
