@@ -203,8 +203,8 @@ struct StageTimer {
 
 // ---------------------------------------------------------------------------
 // Batches.  Phase A (svo_batch_create) runs for every mesh at once: bounding
-// cube, voxelization, bitmap pyramid, one scan over all block counts, level
-// totals, then one small device->host read.  Phase B (svo_batch_emit) writes
+// cube, voxelization, a bitmap pyramid that ranks its own blocks, and a report
+// with the level totals that the last kernel writes to pinned host memory.  Phase B (svo_batch_emit) writes
 // the octrees of any subset of the meshes in one compaction launch and one
 // emission launch.  svo_build is a batch of one.
 // ---------------------------------------------------------------------------
@@ -383,7 +383,7 @@ struct Layout {
 // Phase A.  Returns SVO_OK when the batch itself works (individual meshes
 // may still carry an error status).
 int batch_phase_a(svo_batch *b) {
-    svo::host::TraceRange trace("svo: counting phase (voxelize, pyramid, scan)");
+    svo::host::TraceRange trace("svo: counting phase (voxelize, pyramid)");
     svo_ctx *ctx = b->ctx;
     cudaStream_t st = b->st;
     SVO_TRY(cudaSetDevice(ctx->device), "cudaSetDevice");
@@ -672,9 +672,11 @@ constexpr uint64_t kOwnEmitNodes = SVO_OWN_EMIT_NODES;
 
 // Meshes of up to this many level-0 words (res 256) have their surface-voxel
 // keys listed by the launch that lists the other levels; above, a launch of its
-// own visits the non-empty level-0 blocks only (k_compact_keys).  At res 512
-// level 0 is 2.1M words, 16 MB that hold few bits, and the launch of its own
-// runs beside the emission; up to res 256 level 0 is 2 MB and a launch saved.
+// own visits the non-empty level-0 blocks only (k_compact_keys).  Up to res 256
+// level 0 is 2 MB and a launch is saved; at res 512 it is 16 MB that hold few
+// bits.  Builds of an icosphere, both ways (us, listed with the levels / a launch
+// of its own): res 64 70 / 70, res 128 89 / 93 (without vertices and edges 73 /
+// 81), res 256 148 / 149 (94 / 95), res 512 394 / 387 (179 / 174).
 constexpr uint64_t kDirectKeyWords = 1ull << 18;
 
 // Phase B for meshes [first, first + count).
@@ -717,10 +719,11 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
         const int wave_rc = [&]() -> int {
             cudaError_t err = cudaSuccess;
             // The dedup keys read only the bitmaps and code lists: they run on
-            // a stream of their own, forked here, where their first step (the
-            // level-1 candidate bitmap, from the bitmaps alone) runs while the
-            // host prepares the wave; the rest follows the code lists and runs
-            // beside the emission.  The wave joins it before returning.
+            // a stream of their own.  Of grids up to 1024 the first step (the
+            // level-1 candidate bitmap, from the bitmaps alone) is forked here and
+            // runs while the host prepares the wave; the rest, and the whole dedup
+            // of larger grids, follows the code lists and runs beside the
+            // emission.  The wave joins the stream before returning.
             const bool dd = (flags & SVO_FLAG_DEDUP) != 0;
             AuxStreams *dset = dd ? aux_acquire(ctx) : nullptr;
             const cudaStream_t ds = dset ? dset->s[0] : st;
@@ -770,7 +773,10 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                 // finish: up to 4 GiB of them; the other meshes start just before they
                 // finish, and so do grids above 1024: their candidate pass (110 us at res
                 // 2048) holds the compaction up (60 us beside it, 7 without), while their
-                // dedup ends long before the emission
+                // dedup ends long before the emission.  Whole builds, started early / late
+                // (us): heightfield at res 2048 4,035 / 4,010; at res 1024 and below both
+                // the same (heightfield at res 1024 980 / 985, icosphere 2,477 / 2,476, at
+                // res 512 692 / 693), and the early start spares the emission's memory path
                 uint64_t early = 0;
                 for (int j = 0; j < n; ++j) {
                     const MeshHost &mh = b->m[wave[j]];
@@ -987,9 +993,11 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
             check(launch_compact(CompactBatch{d_jobs, n_jobs, d_word_off}, lone_job ? jobs : nullptr, word_off[n_jobs], st),
                   "compact");
             // The keys need the level-3 lists and nothing needs the keys: they run on
-            // a stream of their own beside the remaining lists and the emission (320
-            // triangles at res 512 420 us before, 414 this way; heightfield at res
-            // 2048, with the later dedup start above, 4,076 and 4,046).
+            // a stream of their own beside the remaining lists (320 triangles at res 512
+            // 420 us before, 414 this way; heightfield at res 2048, with the later dedup
+            // start above, 4,076 and 4,046).  The auxiliary streams have the highest
+            // priority, so the keys go before the emission rather than beside it: at res
+            // 2048 they take 54 us, and the emission starts 28 us after the last list.
             AuxStreams *kset = n_kjobs == 0 ? nullptr : aux_acquire(ctx);
             const cudaStream_t ks = kset ? kset->s[0] : st;
             if (kset) {
@@ -1006,8 +1014,6 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                                              region_range[i].second, ctx->num_sms, st),
                       "compact");
             tm.mark(StageTimer::kCompact, st);
-            // The dedup keys read only the bitmaps and code lists: they run on
-            // a stream of their own, forked here, while the emission writes.
             // the dedup's coarse marks, states and keys need the code lists
             if (dset) {
                 check(cudaEventRecord(dset->fork, st), "fork");

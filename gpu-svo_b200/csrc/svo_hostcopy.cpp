@@ -6,7 +6,9 @@
 // previous one is copied out: 20 MB of node records 700 us (1,030 by the
 // driver), 748 MB of edges 20 ms (35), bound by the threads' copies and the
 // link.  4 threads take 10% longer, chunks of 512 KiB 25% (more events and
-// hand-overs per byte).
+// hand-overs per byte).  From 4 MiB on, where it begins to pay for the threads'
+// start: 3.1 MB into memory in use 206-215 us staged and 183-202 by the driver,
+// 4.0 MB 218-226 and 228-262, 5.2 MB 265-294 and 296-312.
 #include "svo_hostcopy.h"
 
 #include <algorithm>

@@ -225,8 +225,8 @@ __device__ __forceinline__ void finish_top(const MeshDev &md, uint64_t (*s_top)[
 // sums per thread and level in one step up to kFuseRegions; meshes with more
 // regions (res 1024 and up) are finished by k_pyramid_finish, whose five
 // 1024-thread CTAs per mesh work side by side, and so are batches with more
-// than 8 regions per SM, where the fused variant's 56 registers (4 CTAs per SM
-// instead of 8) cost the streaming pass more than the launch saves.
+// than 8 regions per SM, where the fused variant's 62 to 64 registers (4 CTAs per
+// SM instead of 8) cost the streaming pass more than the launch saves.
 constexpr uint32_t kFuseRegions = 1024;
 
 template <bool FUSE, bool ONE>
@@ -582,16 +582,6 @@ __device__ __forceinline__ uint32_t block_rank(const RankDev &r, const Pyramid &
     return r.base[(uint64_t)l * r.bstride + (blk >> (8 - 3 * l))] + r.pre[py.coff[l] + blk];
 }
 
-// One thread per 64-bit word of every job's levels: its first rank is the
-// block prefix plus the popcounts of the preceding words of its block.
-// One thread per bitmap word; the 8 lanes of a 512-bit block are 8 aligned
-// lanes of a warp (every level and job starts on a block boundary), so a
-// word's rank in its level is the block's scanned base plus an 8-lane prefix
-// of popcounts.  Writes the sorted set-bit positions and, for levels >= 1,
-// the rank at each non-empty word (rank_of's table).
-// In a region-mode mesh a word of levels 0-3 lies inside one level-0 region
-// (level-l word w covers level-0 words w * 8^l ..): an unflagged one is
-// empty and is not read.
 // The set-bit codes of the warp's 32 words, whose outputs are one contiguous
 // range in lane order (lane i's codes at o, o + 1, ...; lanes without bits
 // hold pc = 0): staged in shared memory as (lane, bit) entries, then read in
@@ -639,6 +629,14 @@ __device__ __forceinline__ void compact_word(const CompactJob &job, int l, uint6
     }
 }
 
+// One thread per 64-bit word of every job's levels; the 8 lanes of a 512-bit
+// block are 8 aligned lanes of a warp (every level and job starts on a block
+// boundary), so a word's rank in its level is the block's rank plus an 8-lane
+// prefix of popcounts.  Writes the sorted set-bit positions and, for levels >= 1,
+// the rank at each non-empty word (rank_of's table).
+// In a region-mode mesh a word of levels 0-3 lies inside one level-0 region
+// (level-l word w covers level-0 words w * 8^l ..): an unflagged one is
+// empty and is not read.
 // ONE: a single job, passed by value (no upload of its table).
 template <bool ONE>
 __global__ void __launch_bounds__(256) k_compact(CompactBatch cb, const __grid_constant__ CompactJob one,
@@ -969,11 +967,14 @@ constexpr int kOwnBytes = 32 * 9 * 4;    // vertex owners (full neighbour tables
 // 78%.  633 bytes a node: 27.4M nodes in 2,380 us (7.3 TB/s), with full
 // neighbour tables, whose look-ups cost the same memory pipe, in 2,540 to 2,580
 // (2,680 with 7 look-ups per node, plain stores and the whole edge stage at 5
-// CTAs per SM).  6 CTAs per SM: with full tables that spills a few registers
-// that 5 would not, but the dedup's kernels fit beside it (heightfield at res
-// 2048 with dedup 4,150 us for the build, 4,255 with 5, 4,240 before); the
-// vertex and edge arrays alone gain 1% from 6 instead of 8 (torus soup
-// 1,900 us, 1,912), node records alone need 8 (121 us for 3.7M nodes, 139).
+// CTAs per SM).  6 CTAs per SM, 80 registers a thread: with full tables a lone
+// mesh's variant spills 72 bytes of stores and 108 of loads a thread and the one
+// over a mesh table 92 and 232, the others none.  Beside the dedup that still
+// gains (heightfield at res 2048 with dedup 4,150 us for the build, 4,255 with 5,
+// 4,240 before): six leave 4,096 registers of an SM, a dedup CTA takes 11,264 or
+// 12,288, so each one displaces an emission CTA, and five stay where four did
+// with 5.  The vertex and edge arrays alone gain 1% from 6 instead of 8 (torus
+// soup 1,900 us, 1,912), node records alone need 8 (121 us for 3.7M nodes, 139).
 // Without the eviction mark the outputs crowd out the bitmaps (heightfield at
 // res 1024 864 us, 840 with it).
 template <bool S, bool FULL, bool VE, bool ONE>

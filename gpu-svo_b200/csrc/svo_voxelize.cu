@@ -912,18 +912,15 @@ cudaError_t launch_front(const BatchDev &b, uint32_t bbox_blocks, uint32_t total
 
 namespace {
 
-// Flags the level-0 regions (Morton code >> 17: x >> 6, y >> 6, z >> 5) that
-// each triangle's voxel bbox overlaps, for region-mode meshes.  The bbox is
-// tri_box's widened by one voxel on each side, with a product by the
-// reciprocal voxel size in place of the division: the two differ by a few
-// ulps at coordinates <= 2048, far less than the margin, so the flagged
-// regions cover every voxel the voxel test can set.
-// The flags of the level-0 regions (64 x 64 x 32 voxels, region index =
-// morton3(x, y, z) >> 17) each triangle's voxel box (with a one-voxel margin)
-// reaches.  The kernel waits on gathers (indices, then vertices), so each
-// thread takes 3 triangles at a time and issues all their loads before using
-// them; the mesh's grid and reciprocal units are kept while the mesh stays
-// the same.
+// Flags the level-0 regions (64 x 64 x 32 voxels, region index =
+// morton3(x, y, z) >> 17) that each triangle's voxel bbox overlaps, for
+// region-mode meshes.  The bbox is tri_box's widened by one voxel on each side,
+// with a product by the reciprocal voxel size in place of the division: the two
+// differ by a few ulps at coordinates <= 2048, far less than the margin, so the
+// flagged regions cover every voxel the voxel test can set.
+// The kernel waits on gathers (indices, then vertices), so each thread takes 3
+// triangles at a time and issues all their loads before using them; the mesh's
+// grid and reciprocal units are kept while the mesh stays the same.
 constexpr int kMarkBatch = 3;
 
 template <bool ONE>
