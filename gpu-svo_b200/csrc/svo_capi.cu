@@ -1071,6 +1071,17 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
             check(cudaStreamSynchronize(st), "emit phase");
             tm.mark(StageTimer::kUnique0, st);  // (the wait above is for the dedup and the keys as well)
             bool more = false;  // work launched after this wait
+            // the counters of all meshes at once, when some mesh has duplicates (a read
+            // and a wait for each mesh: 100 meshes far from the origin at res 64 9.5 ms,
+            // 8.15 this way)
+            std::vector<unsigned long long> h_dups;
+            if (ve && std::any_of(dev_k.begin(), dev_k.end(), [&](int k) { return b->out[k].dup != 0; })) {
+                h_dups.resize(2 * b->live.size());
+                check(cudaMemcpyAsync(h_dups.data(), b->dups, h_dups.size() * sizeof(h_dups[0]), cudaMemcpyDeviceToHost, st),
+                      "read dups");
+                check(cudaStreamSynchronize(st), "read dups");
+                more = true;
+            }
             for (int j = 0; j < n && rc == SVO_OK; ++j) {
                 MeshHost &mh = b->m[wave[j]];
                 svo_result *r = res[j];
@@ -1079,14 +1090,9 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                                "single top-level node with a non-zero octant: undefined in the reference");
                     continue;
                 }
-                unsigned long long h_dups[2] = {0, 0};
-                if (ve && b->out[dev_k[j]].dup) {
-                    check(cudaMemcpyAsync(h_dups, b->dups + 2 * dev_k[j], sizeof(h_dups), cudaMemcpyDeviceToHost, st),
-                          "read dups");
-                    check(cudaStreamSynchronize(st), "read dups");
-                    more = true;
-                }
-                if (h_dups[0] || h_dups[1]) {
+                const unsigned long long vdup = h_dups.empty() ? 0 : h_dups[2 * dev_k[j]],
+                                         edup = h_dups.empty() ? 0 : h_dups[2 * dev_k[j] + 1];
+                if (vdup || edup) {
                     // consecutive duplicates (degenerate widths or absorbed
                     // coordinates): compact both arrays as thrust::unique does
                     const uint64_t nv = mh.N * 8, ne = mh.N * 12;
@@ -1095,8 +1101,8 @@ int batch_phase_b(svo_batch *b, int first, int count, svo_result **out, int *sta
                     uint32_t *tc = U.get<uint32_t>(tiles), *tp = U.get<uint32_t>(tiles + 1);
                     unsigned long long *ss = U.get<unsigned long long>(scan_scratch_words(tiles));
                     uint32_t *ustat = U.get<uint32_t>(1);
-                    svo_vertex *v2 = h_dups[0] ? pool_alloc<svo_vertex>(ctx->out_pool, st, nv, err) : nullptr;
-                    svo_edge *e2 = h_dups[1] ? pool_alloc<svo_edge>(ctx->out_pool, st, ne, err) : nullptr;
+                    svo_vertex *v2 = vdup ? pool_alloc<svo_vertex>(ctx->out_pool, st, nv, err) : nullptr;
+                    svo_edge *e2 = edup ? pool_alloc<svo_edge>(ctx->out_pool, st, ne, err) : nullptr;
                     if (U.err != cudaSuccess || err != cudaSuccess) {
                         rc = cuda_fail(U.err != cudaSuccess ? U.err : err, "unique scratch");
                         break;
