@@ -963,15 +963,16 @@ constexpr int kOwnBytes = 32 * 9 * 4;    // vertex owners (full neighbour tables
 // Node records and edges are staged per warp and leave as bulk copies (the
 // edges 16 nodes at a time, which halves the stage), vertices straight from
 // registers, everything marked to leave L2 first.  The kernel is bound by
-// writes: the SMs' path to L2 is 80% busy (32 bytes per clock and SM) and DRAM
-// 78%.  633 bytes a node: 27.4M nodes in 2,380 us (7.3 TB/s), with full
-// neighbour tables, whose look-ups cost the same memory pipe, in 2,540 to 2,580
-// (2,680 with 7 look-ups per node, plain stores and the whole edge stage at 5
-// CTAs per SM).  6 CTAs per SM, 80 registers a thread: with full tables a lone
-// mesh's variant spills 72 bytes of stores and 108 of loads a thread and the one
-// over a mesh table 92 and 232, the others none.  Beside the dedup that still
-// gains (heightfield at res 2048 with dedup 4,150 us for the build, 4,255 with 5,
-// 4,240 before): six leave 4,096 registers of an SM, a dedup CTA takes 11,264 or
+// writes: the SMs' path to L2 is 77% busy (32 bytes per clock and SM; 84% with
+// full tables) and DRAM 85% (83%).  633 bytes a node: 27.4M nodes in 2,380 us
+// (7.3 TB/s), with full neighbour tables, whose look-ups cost the same memory
+// pipe, in 2,540 to 2,580 (2,680 with 7 look-ups per node, plain stores and the
+// whole edge stage at 5 CTAs per SM).
+// 6 CTAs per SM, 80 registers a thread: with full tables a lone mesh's variant
+// spills 72 bytes of stores and 108 of loads a thread and the one over a mesh
+// table 92 and 232, the others none.  Beside the dedup that still gains
+// (heightfield at res 2048 with dedup 4,150 us for the build, 4,255 with 5, 4,240
+// before): six leave 4,096 registers of an SM, a dedup CTA takes 11,264 or
 // 12,288, so each one displaces an emission CTA, and five stay where four did
 // with 5.  The vertex and edge arrays alone gain 1% from 6 instead of 8 (torus
 // soup 1,900 us, 1,912), node records alone need 8 (121 us for 3.7M nodes, 139).

@@ -90,6 +90,7 @@ typedef struct svo_result svo_result;
  * reference's process-global launch state (src/SVO.cu:15-18) and its
  * per-call cudaMalloc/thrust allocations (src/SVO.cu:353-376). */
 int svo_ctx_create(int device, svo_ctx **out);
+/* Results may outlive their context; batches, servers and fleets may not. */
 void svo_ctx_destroy(svo_ctx *ctx);
 int svo_ctx_device(const svo_ctx *ctx, int *device);
 /* Maps device memory into the context's pools up front (result arrays,
